@@ -397,7 +397,7 @@ void Batch::build_pairs() {
     PF_CUDA(cudaMemcpyAsync(d_perm, perm.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
     PF_CUDA(cudaMemcpyAsync(d_ps, new_ps.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
     launch_gather_pairs(pd.npair, d_perm, d_ps, tmp.info0, tmp.info1, tmp.info2, tmp.geom, tmp.prim, d_q, cut,
-                        pd.info0, pd.info1, pd.info2, pd.geom, pd.prim, pd.primf, stream);
+                        pd.info0, pd.info1, pd.info2, pd.geom, pd.prim, pd.primf, nullptr, KetTables(), stream);
   }
   PF_CUDA(cudaStreamSynchronize(stream));
   tp[6] = wall_ms();

@@ -403,12 +403,24 @@ void System::build_pairs() {
   }
   pd.npair = (int)perm.size();
   pd.nprim = nprim_new;
+  // slots of the transposed records (s/p classes)
+  size_t nslots = 0;
+  for (int c = 0; c < NCLASS; ++c) {
+    pd.kt.slot[c] = (int)nslots;
+    pd.kt.class_off[c] = pd.class_off[c];
+    pd.kt.maxprim[c] = pd.class_maxprim[c];
+    nslots += (size_t)(pd.class_off[c + 1] - pd.class_off[c]) * (pd.class_maxprim[c] + 1);
+  }
+  pd.kt.class_off[NCLASS] = pd.class_off[NCLASS];
+  nslots = (nslots + 64) / 64 * 64;
   // final records
   o = 0;
   const size_t f_i0 = carve(pd.npair * sizeof(int4)), f_i1 = carve(pd.npair * sizeof(int4)),
                f_i2 = carve(pd.npair * sizeof(int4)), f_g = carve(pd.npair * sizeof(double4)),
                f_pr = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(double4)),
-               f_prf = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(float4));
+               f_prf = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(float4)),
+               f_test = carve(pd.npair * 2 * sizeof(float4)),
+               f_kt = carve(nslots * KetTables::SLOT_BYTES);
   pd.buf.ensure(std::max<size_t>(o, 256));
   char* pb = pd.buf.as<char>();
   pd.info0 = reinterpret_cast<int4*>(pb + f_i0);
@@ -417,11 +429,13 @@ void System::build_pairs() {
   pd.geom = reinterpret_cast<double4*>(pb + f_g);
   pd.prim = reinterpret_cast<double4*>(pb + f_pr);
   pd.primf = reinterpret_cast<float4*>(pb + f_prf);
+  pd.kt.carve(pb + f_kt, nslots);
+  pd.test = reinterpret_cast<float4*>(pb + f_test);
   if (pd.npair > 0) {
     PF_CUDA(cudaMemcpyAsync(d_perm, perm.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
     PF_CUDA(cudaMemcpyAsync(d_ps, new_ps.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
     launch_gather_pairs(pd.npair, d_perm, d_ps, tmp.info0, tmp.info1, tmp.info2, tmp.geom, tmp.prim, d_q, cut,
-                        pd.info0, pd.info1, pd.info2, pd.geom, pd.prim, pd.primf, stream);
+                        pd.info0, pd.info1, pd.info2, pd.geom, pd.prim, pd.primf, pd.test, pd.kt, stream);
   }
   PF_CUDA(cudaStreamSynchronize(stream));
   tq[4] = clk::now();
@@ -457,11 +471,20 @@ void partition_costs(int n, const double* cost, int parts, int* bounds) {
 // classes only kets up to the bra itself are canonical.
 void System::build_tasks() {
   std::vector<int> hostbuf;
-  struct Pending { int bc, kc, prec; size_t off; int nbra; };
+  struct Pending { int bc, kc, prec; size_t off, off_c; int nbra; };
   std::vector<Pending> pend;
   const double thr = std::max(opt.schwarz_thresh, 0.0);
   const double t32 = opt.fp32_thresh;
   quartets_total = 0;
+  any_split = false;
+  // share of atom pairs beyond FAR_DISTANCE, for the choice of the split kernels
+  long long far_pairs = 0;
+  for (int i = 0; i < natoms; ++i)
+    for (int j = 0; j < i; ++j) {
+      const double dx = xyz[3 * i] - xyz[3 * j], dy = xyz[3 * i + 1] - xyz[3 * j + 1], dz = xyz[3 * i + 2] - xyz[3 * j + 2];
+      far_pairs += dx * dx + dy * dy + dz * dz > FAR_DISTANCE * FAR_DISTANCE;
+    }
+  const double far_share = natoms > 1 ? far_pairs / (0.5 * natoms * (natoms - 1)) : 0.0;
   for (int bc = 0; bc < NPAIRCLASS; ++bc)
     for (int kc = 0; kc <= bc; ++kc) {
       const int nb = pd.class_off[bc + 1] - pd.class_off[bc];
@@ -484,7 +507,7 @@ void System::build_tasks() {
         m64v[i] = std::min(p64, m);
       }
       for (int prec = 0; prec < 3; ++prec) {
-        Pending p{bc, kc, prec, hostbuf.size(), nb};
+        Pending p{bc, kc, prec, hostbuf.size(), 0, nb};
         std::vector<int> toff(nb + 1), lo(nb), hi(nb);
         long long quart = 0;
         int ntask = 0;
@@ -501,6 +524,7 @@ void System::build_tasks() {
         }
         toff[nb] = ntask;
         if (prec == 0) quartets_total += quart;
+        const int chunk = bc >= NCLASS ? 0 : split_chunk(quart, far_share, pd.class_maxprim[bc] * pd.class_maxprim[kc], num_sms);
         TaskList& tl = tasks[bc][kc][prec];
         tl.width = task_width;
         tl.nbra = nb;
@@ -509,6 +533,18 @@ void System::build_tasks() {
         hostbuf.insert(hostbuf.end(), toff.begin(), toff.end());
         hostbuf.insert(hostbuf.end(), lo.begin(), lo.end());
         hostbuf.insert(hostbuf.end(), hi.begin(), hi.end());
+        tl.chunk = chunk;
+        any_split = any_split || chunk > 0;
+        if (chunk) {
+          p.off_c = hostbuf.size();
+          int nt = 0;
+          for (int i = 0; i < nb; ++i) {
+            hostbuf.push_back(nt);
+            nt += (hi[i] - lo[i] + chunk - 1) / chunk;
+          }
+          hostbuf.push_back(nt);
+          tl.ntasks_c = nt;
+        }
         pend.push_back(p);
       }
     }
@@ -532,7 +568,10 @@ void System::build_tasks() {
         tl.width = task_width;
         tl.nbra = nb;
         tl.ntasks = std::max(1, tasks[bc][kc][0].ntasks);
-        tl.task_off = dd;
+        tl.chunk = part == 1 ? tasks[bc][kc][0].chunk : 0;
+        tl.nquartets = tasks[bc][kc][0].nquartets;  // a bound
+        tl.ntasks_c = std::max(1, tasks[bc][kc][0].ntasks_c);
+        tl.task_off = tl.off_c = dd;
         tl.ket_lo = dd + nb + 1;
         tl.ket_hi = dd + 2 * nb + 1;
         tl.ntasks_dev = dyn.ntasks_dev + 2 * qc + part;
@@ -546,6 +585,8 @@ void System::build_tasks() {
     tl.task_off = d + p.off;
     tl.ket_lo = d + p.off + p.nbra + 1;
     tl.ket_hi = d + p.off + 2 * p.nbra + 1;
+    tl.off_c = tl.chunk ? d + p.off_c : nullptr;
+    tl.bra_offset = tl.task_begin = tl.task_begin_c = 0;
     if (nsh > 1) {
       // this shard's bra range of the list, balanced by task counts
       const int* toff = hostbuf.data() + p.off;
@@ -565,6 +606,12 @@ void System::build_tasks() {
       tl.ket_hi += b0;
       tl.task_begin = toff[b0];
       tl.ntasks = toff[b1] - toff[b0];
+      if (tl.chunk) {
+        const int* toc = hostbuf.data() + p.off_c;
+        tl.off_c += b0;
+        tl.task_begin_c = toc[b0];
+        tl.ntasks_c = toc[b1] - toc[b0];
+      }
       tl.nquartets = q;
     }
   }
@@ -594,7 +641,8 @@ void System::alloc_matrices() {
   dmax = reinterpret_cast<float*>(m);
   const size_t red_bytes = (size_t)RED_BLOCKS * (nd + 3) * sizeof(double);
   small_buf.ensure(2 * nbf * sizeof(double) + 256 + sizeof(JkStats) + 256 + 64 * sizeof(double*) + 256 +
-                   3 * natoms * sizeof(double) + 256 + 256 + red_bytes + 256 + nbf * sizeof(double) + 256 + 256);
+                   3 * natoms * sizeof(double) + 256 + 256 + red_bytes + 256 + nbf * sizeof(double) + 256 + 256 +
+                   SPLIT_COUNTERS * sizeof(int) + 256);
   {
     char* b = small_buf.as<char>();
     size_t o = 0;
@@ -607,6 +655,7 @@ void System::alloc_matrices() {
     red_part = reinterpret_cast<double*>(take(red_bytes));
     occ_dev = reinterpret_cast<double*>(take(nbf * sizeof(double)));
     pmin_dev = reinterpret_cast<double*>(take(sizeof(double)));
+    jk_next = reinterpret_cast<int*>(take(SPLIT_COUNTERS * sizeof(int)));
   }
   {
     const std::vector<double> occ = atomic_occupations();
@@ -629,6 +678,7 @@ void System::release_extra() {
   red_part = nullptr;
   occ_dev = nullptr;
   pmin_dev = nullptr;
+  jk_next = nullptr;
 }
 
 }  // namespace pyfacc

@@ -9,9 +9,11 @@
 //                 info2 = {matrix offset (lo, hi), ld, molecule},
 //                 geom = {A-B, Q_ab}
 //  * prim pairs   3 x double4 per primitive pair:
-//                 {p, 1/(2p), K, alpha}, {P, 0}, {P-A, 0} with
+//                 {p, 1/(2p), K, alpha}, {P, k}, {P-A, 1/(2p)} with
 //                 K = c_a c_b N_a N_b exp(-alpha beta/p |AB|^2) sqrt(2) pi^(5/4) / p
-//                 so that a primitive quartet prefactor is K_ab K_cd / sqrt(p+q);
+//                 so that a primitive quartet prefactor is K_ab K_cd / sqrt(p+q),
+//                 and k = K sqrt(sqrt(pi)/2) / sqrt(p), so that a far one's
+//                 (ss|ss) is k_ab k_cd / |PQ|;
 //                 primitive pairs with |K| < 1e-16 max|K| are left out.
 //  * tasks        per (bra class, ket class, precision): for bra pair i the
 //                 ket range [ket_lo[i], ket_hi[i]) in chunks of 32 (one warp,
@@ -151,6 +153,42 @@ struct TaskList {
   int bra_offset = 0;   // first bra of this (shard of the) list within its class
   int task_begin = 0;   // global index of the first task (task_off values are global)
   int width = TASK_WIDTH;  // kets per task: 32, 16 or 8 (a warp runs 32 / width tasks)
+  // the same ket ranges cut into runs of `chunk` kets for the split kernels
+  // (jk_split.cu); 0: the list is too short for them
+  int chunk = 0;
+  int ntasks_c = 0;
+  int* off_c = nullptr;   // device, nbra + 1
+  int task_begin_c = 0;
+};
+
+// The s/p pairs' primitive records once more, transposed for lanes that each
+// read their own ket: slot[class] + k * npair[class] + (pair within the
+// class) holds the k-th largest primitive pair, so that neighbouring kets are
+// neighbours in memory.  With the 96-byte records of PairData::prim a warp's
+// load touched 32 lines and cost ~14 wavefronts of the L1 data stage.
+// Row maxprim[class] holds, for a pair on one atom, the one primitive that is
+// equivalent to all of the pair's in the far limit (kabs 0: none).  With one
+// product centre P = A the pair's multipoles are sum k (ss), sum k/2p (ps),
+// sum k/2p and sum k/(2p)^2 (pp), which one (k, 1/2p) carries exactly.
+struct KetTables {
+  double2 *xy = nullptr, *zk = nullptr;   // {Px, Py}, {Pz, k}
+  double2 *pq = nullptr, *zo = nullptr;   // {P-A x, y}, {P-A z, 1/2p}
+  double2* pk = nullptr;                  // {p, K}
+  float4 *fp = nullptr, *fq = nullptr;    // {P, k}, {P-A, 1/2p}
+  float2* fk = nullptr;                   // {p, K}
+  float* kabs = nullptr;                  // |K|
+  int slot[NCLASS] = {0, 0, 0};
+  int class_off[NCLASS + 1] = {0, 0, 0, 0};
+  int maxprim[NCLASS] = {0, 0, 0};
+  static constexpr size_t SLOT_BYTES = 5 * sizeof(double2) + 2 * sizeof(float4) + sizeof(float2) + sizeof(float);
+  // carves the arrays for nslots slots (a multiple of 64) out of base
+  void carve(char* base, size_t nslots);
+  KetTables part(int c) const {  // the arrays of one class
+    KetTables t = *this;
+    const int o = slot[c];
+    t.xy += o; t.zk += o; t.pq += o; t.zo += o; t.pk += o; t.fp += o; t.fq += o; t.fk += o; t.kabs += o;
+    return t;
+  }
 };
 
 // Packed pair data of one molecule or of a batch (every pair stores the
@@ -166,6 +204,11 @@ struct PairData {
   double4* geom = nullptr;   // {ABx, ABy, ABz, Q}
   double4* prim = nullptr;   // 3 per primitive pair
   float4* primf = nullptr;   // the same records in float (FP32 quartets)
+  // for the candidate test of the split kernels, npair of each: {centre of
+  // the primitive pairs' product centres, extent}, then {extent, Q, shell a,
+  // shell b as bits} (the two extents of far.cuh)
+  float4* test = nullptr;
+  KetTables kt;              // arrays null without them
   std::vector<double> q_host;   // Q of the sorted pairs
   std::vector<int> cls_host;    // class of the sorted pairs
   std::vector<int> mol_host;    // molecule of the sorted pairs
@@ -223,7 +266,8 @@ void launch_schwarz(const PairData& pd, int npair_class_begin[NCLASS + 1], doubl
                     cudaStream_t side = nullptr, cudaEvent_t fork = nullptr, cudaEvent_t join = nullptr);
 void launch_gather_pairs(int npair, const int* perm, const int* new_pstart, const int4* i0, const int4* i1,
                          const int4* i2, const double4* g, const double4* pr, const double* q, double cut,
-                         int4* o0, int4* o1, int4* o2, double4* og, double4* opr, float4* oprf, cudaStream_t s);
+                         int4* o0, int4* o1, int4* o2, double4* og, double4* opr, float4* oprf, float4* otest, const KetTables& kt,
+                         cudaStream_t s);
 // Largest primitive-pair prefactor |K| of a basis (reached at |AB| = 0) and
 // the relative cut below which primitive pairs are dropped.
 double max_prim_prefactor(const Basis& b);
@@ -247,6 +291,20 @@ struct JkArgs {
 void launch_jk(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32, int nk,
                const JkArgs& a, int num_sms, cudaStream_t s);
 
+// The split kernels (jk_split.cu) take the lists of the classes below
+// (pp|pp) that are long enough to fill the GPU with runs of kets.
+constexpr int SPLIT_CHUNK_MAX = 512;
+constexpr int SPLIT_MAXPRIM = 64;  // bra primitive pairs staged per warp (STO-6G: 36)
+constexpr int SPLIT_RUNS_PER_SM = 32;
+constexpr double SPLIT_MIN_FAR = 3.0e5;   // estimated far quartets of a list (split_chunk)
+constexpr double FAR_DISTANCE = 16.0;     // bohr: quartets of diffuse pairs that far apart are far in FP64
+constexpr int SPLIT_COUNTERS = 4 * NQCLASS;  // task counters of a build: two kernels per class and precision
+int split_chunk(long long nquartets, double far_share, int prim_quartets, int num_sms);
+bool jk_splits(const PairData& pd, const TaskList& tl, int bra_class, int ket_class);
+void launch_jk_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32, int nk,
+                     const JkArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
+void upload_boys_rows();  // their Boys tables, on the current device
+
 // Task lists rebuilt on the GPU for one Fock build from the density bound
 // dmax (ns x ns): a bra pair i keeps the ket prefix with
 // Q_i Q_j max|D| >= thresh, the FP64 part being the prefix with
@@ -257,8 +315,9 @@ struct DynTaskSet {
   int* ntasks_dev = nullptr;   // 2 * NQCLASS counts
   double* dmax_global = nullptr;
 };
+// split: the FP32 lists of the split kernels' classes are cut into their runs.
 void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thresh, double fp32_thresh,
-                      DynTaskSet& dt, cudaStream_t s);
+                      DynTaskSet& dt, bool split, cudaStream_t s);
 
 struct GradArgs {
   const double* Pt;

@@ -17,9 +17,9 @@
 #include <mutex>
 #include <vector>
 
-#include "boys.cuh"
 #include "engine.h"
-#include "eri_classes.cuh"
+#include "far.cuh"
+#include "quartet.cuh"
 
 namespace pyfacc {
 
@@ -72,6 +72,7 @@ void ensure_boys_tables(int device) {
     PF_CUDA(cudaMemcpyToSymbol(g_boys_exp, ex.data(), ex.size() * sizeof(double)));
     PF_CUDA(cudaMemcpyToSymbol(g_boys_tlf, tabf.data(), tabf.size() * sizeof(float)));
     upload_boys_tables_d(tl.data(), tl.size(), ex.data(), ex.size());
+    upload_boys_rows();
     done[device] = 1;
   }
 }
@@ -180,189 +181,6 @@ void launch_build_pairs(const ShellDev& sh, int npair, const int4* pl0, const in
   count_launch();
 }
 
-// ---------------------------------------------------------------------------
-// One primitive quartet: prefactors, Boys, VRR (shared by J/K, Schwarz,
-// gradient and tensor kernels).
-// ---------------------------------------------------------------------------
-template <typename R>
-struct PrimGeo {
-  R I[PF_BOYS_MMAX + 1];
-  R WP[3], WQ[3];
-  R o2p, nrp, o2q, nrq, o2pq;  // nrp = -rho/p, nrq = -rho/q
-};
-
-template <typename R> struct Rec;  // primitive-pair record vector of a precision
-template <> struct Rec<double> { using T = double4; };
-template <> struct Rec<float> { using T = float4; };
-
-// bra record b0..b2 and ket record k0..k2 (3 vectors each)
-template <typename R, int LM, typename V>
-__device__ __forceinline__ void prim_setup(const V& b0, const V& b1, const V& k0, const V& k1, PrimGeo<R>& g) {
-  const R p = (R)b0.x, q = (R)k0.x;
-  const R PQx = (R)(b1.x - k1.x), PQy = (R)(b1.y - k1.y), PQz = (R)(b1.z - k1.z);
-  const R zeta = p + q;
-  R rs, oz;
-  if constexpr (sizeof(R) == 8) {
-    rs = rsqrt((double)zeta);
-  } else {
-    rs = rsqrtf((float)zeta);
-  }
-  oz = rs * rs;
-  const R rho = p * q * oz;
-  const R T = rho * (PQx * PQx + PQy * PQy + PQz * PQz);
-  const R pref = (R)b0.z * (R)k0.z * rs;
-  R F[LM + 1];
-  Boys<LM, R>::eval(T, F);
-#pragma unroll
-  for (int m = 0; m <= LM; ++m) g.I[m] = pref * F[m];
-  const R qz = q * oz, pz = p * oz;
-  g.WP[0] = -qz * PQx; g.WP[1] = -qz * PQy; g.WP[2] = -qz * PQz;
-  g.WQ[0] = pz * PQx;  g.WQ[1] = pz * PQy;  g.WQ[2] = pz * PQz;
-  g.o2p = (R)b0.y;
-  g.o2q = (R)k0.y;
-  g.nrp = -qz;  // -rho / p
-  g.nrq = -pz;  // -rho / q
-  g.o2pq = (R)0.5 * oz;
-}
-
-template <int L> struct NC { static constexpr int v = (L + 1) * (L + 2) / 2; };
-
-// Contracted (ab|cd) for one bra pair and one ket pair (records of the
-// kernel's precision: double4 for FP64 quartets, float4 for FP32 ones).
-// Primitive pairs are stored in order of decreasing |K|, so with kcut > 0
-// both loops stop at the first primitive quartet with |K_ab K_cd| < kcut.
-// With kq_step > 1 only the ket primitives kq0, kq0 + kq_step, ... are
-// summed (a share of the quartet; the shares add up to the integral).
-// brec: the bra pair's first primitive record (in global memory, or the
-// copy a warp staged in shared memory); prim: all records (the kets').
-template <typename R, int LA, int LB, int LC, int LD>
-__device__ __forceinline__ int contracted_quartet(const typename Rec<R>::T* __restrict__ prim,
-                                                  const typename Rec<R>::T* brec, int4 bi0, int4 ki0,
-                                                  const double4& bgeo, const double4& kgeo,
-                                                  R out[EriClass<R, LA, LB, LC, LD>::NOUT], double kcut = 0.0,
-                                                  int kq0 = 0, int kq_step = 1) {
-  using C = EriClass<R, LA, LB, LC, LD>;
-  using V = typename Rec<R>::T;
-  R acc[C::NACC];
-#pragma unroll
-  for (int i = 0; i < C::NACC; ++i) acc[i] = (R)0;
-  // the cut is compared in the records' precision (no FP64 work in the FP32
-  // loop); a cut beyond the float range becomes +inf, which skips everything
-  const R cut = (R)kcut;
-  const R kab_max = fabs((R)brec[0].z);
-  int nprim = 0;
-  for (int kq = kq0; kq < ki0.w; kq += kq_step) {
-    const V* kr = prim + 3 * (size_t)(ki0.z + kq);
-    const V k0 = kr[0], k1 = kr[1], k2 = kr[2];
-    const R kcd = fabs((R)k0.z);
-    if (kab_max * kcd < cut) break;
-    const R QC[3] = {(R)k2.x, (R)k2.y, (R)k2.z};
-#pragma unroll 1
-    for (int kp = 0; kp < bi0.w; ++kp) {
-      const V* br = brec + 3 * kp;
-      const V b0 = br[0], b1 = br[1], b2 = br[2];
-      if (fabs((R)b0.z) * kcd < cut) break;
-      const R PA[3] = {(R)b2.x, (R)b2.y, (R)b2.z};
-      PrimGeo<R> g;
-      prim_setup<R, C::L>(b0, b1, k0, k1, g);
-      C::vrr(g.I, PA, g.WP, QC, g.WQ, g.o2p, g.nrp, g.o2q, g.nrq, g.o2pq, acc);
-      ++nprim;
-    }
-  }
-  const R AB[3] = {(R)bgeo.x, (R)bgeo.y, (R)bgeo.z};
-  const R CD[3] = {(R)kgeo.x, (R)kgeo.y, (R)kgeo.z};
-  C::hrr(acc, AB, CD, out);
-  return nprim;
-}
-
-// The FP32 contracted quartet with two bra primitives per step in packed
-// float pairs (FFMA2, f2.cuh): the same primitive quartets, cuts and sums as
-// contracted_quartet<float>, but each Obara-Saika step of the generated
-// recursion does the work of both primitives in one instruction.  An odd
-// bra primitive count, or a second primitive below the cut, fills the upper
-// half with the lower primitive at zero weight.
-template <int L>
-__device__ __forceinline__ void prim_setup_f2(const float4& blo0, const float4& blo1, const float4& bhi0,
-                                              const float4& bhi1, float khi_weight, const float4& k0,
-                                              const float4& k1, PrimGeo<F2>& g) {
-  const F2 p(blo0.x, bhi0.x), q(k0.x);
-  const F2 PQx = F2(blo1.x, bhi1.x) + F2(-k1.x), PQy = F2(blo1.y, bhi1.y) + F2(-k1.y),
-           PQz = F2(blo1.z, bhi1.z) + F2(-k1.z);
-  const F2 zeta = p + q;
-  const F2 rs(rsqrtf(zeta.v.x), rsqrtf(zeta.v.y));
-  const F2 oz = rs * rs;
-  const F2 rho = p * q * oz;
-  const F2 T = rho * pf_fma(PQx, PQx, pf_fma(PQy, PQy, PQz * PQz));
-  const F2 pref = F2(blo0.z, bhi0.z * khi_weight) * F2(k0.z) * rs;
-  F2 F[L + 1];
-  boys_fp32x2<L>(T, F);
-#pragma unroll
-  for (int m = 0; m <= L; ++m) g.I[m] = pref * F[m];
-  const F2 qz = q * oz, pz = p * oz;
-  const F2 nqz = qz * F2(-1.0f);
-  g.WP[0] = nqz * PQx; g.WP[1] = nqz * PQy; g.WP[2] = nqz * PQz;
-  g.WQ[0] = pz * PQx;  g.WQ[1] = pz * PQy;  g.WQ[2] = pz * PQz;
-  g.o2p = F2(blo0.y, bhi0.y);
-  g.o2q = F2(k0.y);
-  g.nrp = nqz;               // -rho / p
-  g.nrq = pz * F2(-1.0f);    // -rho / q
-  g.o2pq = F2(0.5f) * oz;
-}
-
-template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ int contracted_quartet_f2(const float4* __restrict__ prim, const float4* brec, int4 bi0,
-                                                     int4 ki0, const double4& bgeo, const double4& kgeo,
-                                                     float out[EriClass<float, LA, LB, LC, LD>::NOUT],
-                                                     double kcut = 0.0, int kq0 = 0, int kq_step = 1) {
-  using C2 = EriClass<F2, LA, LB, LC, LD>;
-  using C1 = EriClass<float, LA, LB, LC, LD>;
-  F2 acc[C2::NACC];
-#pragma unroll
-  for (int i = 0; i < C2::NACC; ++i) acc[i] = F2(0.0f);
-  const float cut = (float)kcut;
-  const float kab_max = fabsf(brec[0].z);
-  int nprim = 0;
-  for (int kq = kq0; kq < ki0.w; kq += kq_step) {
-    const float4* kr = prim + 3 * (size_t)(ki0.z + kq);
-    const float4 k0 = kr[0], k1 = kr[1], k2 = kr[2];
-    const float kcd = fabsf(k0.z);
-    if (kab_max * kcd < cut) break;
-    const F2 QC[3] = {F2(k2.x), F2(k2.y), F2(k2.z)};
-#pragma unroll 1
-    for (int kp = 0; kp < bi0.w; kp += 2) {
-      const float4* br = brec + 3 * kp;
-      const float4 b0 = br[0], b1 = br[1], b2 = br[2];
-      if (fabsf(b0.z) * kcd < cut) break;
-      // the second primitive, or the first again at zero weight
-      bool two = kp + 1 < bi0.w;
-      float4 c0 = b0, c1 = b1, c2 = b2;
-      if (two) {
-        c0 = br[3];
-        two = fabsf(c0.z) * kcd >= cut;
-        if (two) {
-          c1 = br[4];
-          c2 = br[5];
-        } else {
-          c0 = b0;
-        }
-      }
-      const F2 PA[3] = {F2(b2.x, c2.x), F2(b2.y, c2.y), F2(b2.z, c2.z)};
-      PrimGeo<F2> g;
-      prim_setup_f2<C2::L>(b0, b1, c0, c1, two ? 1.0f : 0.0f, k0, k1, g);
-      C2::vrr(g.I, PA, g.WP, QC, g.WQ, g.o2p, g.nrp, g.o2q, g.nrq, g.o2pq, acc);
-      nprim += two ? 2 : 1;
-      if (!two) break;
-    }
-  }
-  float accs[C1::NACC];
-#pragma unroll
-  for (int i = 0; i < C1::NACC; ++i) accs[i] = acc[i].v.x + acc[i].v.y;
-  const float AB[3] = {(float)bgeo.x, (float)bgeo.y, (float)bgeo.z};
-  const float CD[3] = {(float)kgeo.x, (float)kgeo.y, (float)kgeo.z};
-  C1::hrr(accs, AB, CD, out);
-  return nprim;
-}
-
 // Schwarz factor of every pair of one class: Q = sqrt(max |(ab|ab)|).
 template <int LA, int LB>
 __global__ void schwarz_kernel(int begin, int end, const int4* __restrict__ info0, const double4* __restrict__ geom,
@@ -415,7 +233,7 @@ __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, con
                                     const double4* __restrict__ pr, const double* __restrict__ q, double cut,
                                     int4* __restrict__ o0, int4* __restrict__ o1, int4* __restrict__ o2,
                                     double4* __restrict__ og, double4* __restrict__ opr,
-                                    float4* __restrict__ oprf) {
+                                    float4* __restrict__ oprf, float4* __restrict__ otest, const KetTables kt) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= npair) return;
   const int j = perm[i];
@@ -446,21 +264,40 @@ __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, con
   }
   const int nkept = nk;
   nk = 0;
+  // the product centres lie on the line AB: their box's diagonal
+  double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, c2 = sqrt((double)FAR_C2);
   for (int kk = 0; kk < (old_np <= 64 ? nkept : old_np); ++kk) {
     const int k = (old_np <= 64) ? order[kk] : kk;
     const double4* src = pr + 3 * (size_t)(old_ps + k);
     const double4 r0 = src[0];
     if (fabs(r0.z) < cut) continue;
     double4* dst = opr + 3 * (size_t)(a.z + nk);
-    const double4 r1 = src[1], r2 = src[2];
+    double4 r1 = src[1], r2 = src[2];
+    r1.w = r0.z * 0.94139626377671482 * sqrt(2.0 * r0.y);  // K sqrt(sqrt(pi)/2) / sqrt(p)
+    r2.w = r0.y;
+    lo[0] = fmin(lo[0], r1.x); lo[1] = fmin(lo[1], r1.y); lo[2] = fmin(lo[2], r1.z);
+    hi[0] = fmax(hi[0], r1.x); hi[1] = fmax(hi[1], r1.y); hi[2] = fmax(hi[2], r1.z);
     dst[0] = r0;
     dst[1] = r1;
     dst[2] = r2;
     if (oprf) {
       float4* df = oprf + 3 * (size_t)(a.z + nk);
       df[0] = make_float4((float)r0.x, (float)r0.y, (float)r0.z, (float)r0.w);
-      df[1] = make_float4((float)r1.x, (float)r1.y, (float)r1.z, 0.0f);
-      df[2] = make_float4((float)r2.x, (float)r2.y, (float)r2.z, 0.0f);
+      df[1] = make_float4((float)r1.x, (float)r1.y, (float)r1.z, (float)r1.w);
+      df[2] = make_float4((float)r2.x, (float)r2.y, (float)r2.z, (float)r2.w);
+    }
+    if (kt.xy && i < kt.class_off[NCLASS]) {
+      const int c = i < kt.class_off[1] ? 0 : (i < kt.class_off[2] ? 1 : 2);
+      const size_t sl = kt.slot[c] + (size_t)nk * (kt.class_off[c + 1] - kt.class_off[c]) + (i - kt.class_off[c]);
+      kt.xy[sl] = make_double2(r1.x, r1.y);
+      kt.zk[sl] = make_double2(r1.z, r1.w);
+      kt.pq[sl] = make_double2(r2.x, r2.y);
+      kt.zo[sl] = make_double2(r2.z, r2.w);
+      kt.pk[sl] = make_double2(r0.x, r0.z);
+      kt.fp[sl] = make_float4((float)r1.x, (float)r1.y, (float)r1.z, (float)r1.w);
+      kt.fq[sl] = make_float4((float)r2.x, (float)r2.y, (float)r2.z, (float)r2.w);
+      kt.fk[sl] = make_float2((float)r0.x, (float)r0.z);
+      kt.kabs[sl] = fabsf((float)r0.z);
     }
     ++nk;
   }
@@ -471,14 +308,70 @@ __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, con
   double4 gg = g[j];
   gg.w = q[j];
   og[i] = gg;
+  if (kt.xy && i < kt.class_off[NCLASS]) {
+    const int c = i < kt.class_off[1] ? 0 : (i < kt.class_off[2] ? 1 : 2);
+    const size_t m = kt.slot[c] + (size_t)kt.maxprim[c] * (kt.class_off[c + 1] - kt.class_off[c]) + (i - kt.class_off[c]);
+    float km = 0.0f;
+    if (i1[j].z == i1[j].w && nk > 0) {
+      double s0 = 0.0, s1 = 0.0, s2 = 0.0, a0 = 0.0, a1 = 0.0, a2 = 0.0;
+      for (int k = 0; k < nk; ++k) {
+        const double o = opr[3 * (size_t)(a.z + k)].y, w = opr[3 * (size_t)(a.z + k) + 1].w;
+        s0 += w; s1 += w * o; s2 += w * o * o;
+        a0 += fabs(w); a1 += fabs(w) * o; a2 += fabs(w) * o * o;
+      }
+      // ss: o is not used; ps: any o; pp: o = s2 / s1, unless the sums cancel
+      const double o = c == 2 ? s2 / s1 : a1 / a0, w = c == 0 ? s0 : s1 / o;
+      if (c < 2 || (fabs(s1) > 1e-3 * a1 && fabs(s2) > 1e-3 * a2)) {
+        const double4 r1 = opr[3 * (size_t)a.z + 1], r2 = opr[3 * (size_t)a.z + 2];
+        km = fabsf((float)opr[3 * (size_t)a.z].z);
+        kt.xy[m] = make_double2(r1.x, r1.y);
+        kt.zk[m] = make_double2(r1.z, w);
+        kt.pq[m] = make_double2(r2.x, r2.y);
+        kt.zo[m] = make_double2(r2.z, o);
+        kt.fp[m] = make_float4((float)r1.x, (float)r1.y, (float)r1.z, (float)w);
+        kt.fq[m] = make_float4((float)r2.x, (float)r2.y, (float)r2.z, (float)o);
+      }
+    }
+    kt.kabs[m] = km;
+  }
+  if (otest) {
+    if (nk == 0) lo[0] = lo[1] = lo[2] = hi[0] = hi[1] = hi[2] = 0.0;
+    const double rx = 0.5 * (hi[0] - lo[0]), ry = 0.5 * (hi[1] - lo[1]), rz = 0.5 * (hi[2] - lo[2]);
+    const double cx = lo[0] + rx, cy = lo[1] + ry, cz = lo[2] + rz;
+    double e0 = 0.0, e1 = 0.0;
+    for (int k = 0; k < nk; ++k) {
+      const double4 r0 = opr[3 * (size_t)(a.z + k)], r1 = opr[3 * (size_t)(a.z + k) + 1];
+      const double dx = r1.x - cx, dy = r1.y - cy, dz = r1.z - cz;
+      const double r = sqrt(dx * dx + dy * dy + dz * dz), w = r0.y / c2 + 0.25 * c2;  // s/(2c) + c/4, s = 2 r0.y
+      e0 = fmax(e0, r + FAR_TAU0 * w);
+      e1 = fmax(e1, r + FAR_TAU1 * w);
+    }
+    const int4 sh = i1[j];
+    otest[i] = make_float4((float)cx, (float)cy, (float)cz, (float)e0 * 1.000001f);
+    otest[npair + i] = make_float4((float)e1 * 1.000001f, (float)gg.w, __int_as_float(sh.x), __int_as_float(sh.y));
+  }
+}
+
+void KetTables::carve(char* b, size_t n) {
+  auto take = [&](size_t bytes) { char* r = b; b += n * bytes; return r; };
+  xy = reinterpret_cast<double2*>(take(sizeof(double2)));
+  zk = reinterpret_cast<double2*>(take(sizeof(double2)));
+  pq = reinterpret_cast<double2*>(take(sizeof(double2)));
+  zo = reinterpret_cast<double2*>(take(sizeof(double2)));
+  pk = reinterpret_cast<double2*>(take(sizeof(double2)));
+  fp = reinterpret_cast<float4*>(take(sizeof(float4)));
+  fq = reinterpret_cast<float4*>(take(sizeof(float4)));
+  fk = reinterpret_cast<float2*>(take(sizeof(float2)));
+  kabs = reinterpret_cast<float*>(take(sizeof(float)));
 }
 
 void launch_gather_pairs(int npair, const int* perm, const int* new_pstart, const int4* i0, const int4* i1,
                          const int4* i2, const double4* g, const double4* pr, const double* q, double cut,
-                         int4* o0, int4* o1, int4* o2, double4* og, double4* opr, float4* oprf, cudaStream_t s) {
+                         int4* o0, int4* o1, int4* o2, double4* og, double4* opr, float4* oprf, float4* otest, const KetTables& kt,
+                         cudaStream_t s) {
   if (npair <= 0) return;
   gather_pairs_kernel<<<(npair + 127) / 128, 128, 0, s>>>(npair, perm, new_pstart, i0, i1, i2, g, pr, q, cut, o0,
-                                                          o1, o2, og, opr, oprf);
+                                                          o1, o2, og, opr, oprf, otest, kt);
   PF_CUDA(cudaGetLastError());
   count_launch();
 }
@@ -486,30 +379,6 @@ void launch_gather_pairs(int npair, const int* perm, const int* new_pstart, cons
 // ===========================================================================
 // J/K digestion
 // ===========================================================================
-__device__ __forceinline__ int find_bra(const int* __restrict__ task_off, int nbra, int t) {
-  int lo = 0, hi = nbra;  // task_off[lo] <= t < task_off[hi]
-  while (hi - lo > 1) {
-    int mid = (lo + hi) >> 1;
-    if (__ldg(task_off + mid) <= t) lo = mid; else hi = mid;
-  }
-  return lo;
-}
-
-__device__ __forceinline__ double warp_sum(double v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-__device__ __forceinline__ float dmax_bound(const float* __restrict__ dm, int ld, int a, int b, int c, int d) {
-  float m = 2.0f * fmaxf(__ldg(dm + a * ld + b), __ldg(dm + c * ld + d));
-  m = fmaxf(m, __ldg(dm + a * ld + c));
-  m = fmaxf(m, __ldg(dm + a * ld + d));
-  m = fmaxf(m, __ldg(dm + b * ld + c));
-  m = fmaxf(m, __ldg(dm + b * ld + d));
-  return m;
-}
-
 struct JkKernelArgs {
   JkArgs a;
   const int* ntasks_dev;
@@ -845,7 +714,7 @@ __global__ void dmax_global_kernel(long long n, const float* __restrict__ dm, do
 }
 
 struct DynListArgs {
-  int nbra, bra_base, ket_base, nket, same, part;  // part 0: FP64, 1: FP32
+  int nbra, bra_base, ket_base, nket, same, part, width;  // part 0: FP64, 1: FP32
   int* task_off;
   int* ket_lo;
   int* ket_hi;
@@ -856,7 +725,6 @@ struct DynAllArgs {
   const double4* geom;
   const double* dmax_global;
   double thresh, fp32_thresh;
-  int width;
 };
 
 __device__ __forceinline__ int ket_prefix(const double4* __restrict__ geom, int ket_base, int nket, double qb, double t) {
@@ -887,7 +755,7 @@ __global__ void __launch_bounds__(1024) dyn_tasks_kernel(const DynAllArgs A) {
       const int lo = L.part == 0 ? 0 : m64, hi = L.part == 0 ? m64 : m;
       L.ket_lo[i] = lo;
       L.ket_hi[i] = hi;
-      cnt = (hi - lo + A.width - 1) / A.width;
+      cnt = (hi - lo + L.width - 1) / L.width;
     }
     // block exclusive scan of cnt
     int v = cnt;
@@ -922,7 +790,7 @@ __global__ void __launch_bounds__(1024) dyn_tasks_kernel(const DynAllArgs A) {
 }
 
 void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thresh, double fp32_thresh,
-                      DynTaskSet& dt, cudaStream_t s) {
+                      DynTaskSet& dt, bool split, cudaStream_t s) {
   dmax_global_kernel<<<1, 1024, 0, s>>>((long long)ns * ns, dmax, dt.dmax_global);
   PF_CUDA(cudaGetLastError());
   count_launch();
@@ -931,7 +799,6 @@ void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thre
   A.dmax_global = dt.dmax_global;
   A.thresh = thresh;
   A.fp32_thresh = fp32_thresh;
-  A.width = dt.lists[0].width;
   int k = 0;
   for (int bc = 0; bc < NCLASS; ++bc)
     for (int kc = 0; kc <= bc; ++kc) {
@@ -945,6 +812,7 @@ void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thre
         L.nket = pd.class_off[kc + 1] - pd.class_off[kc];
         L.same = bc == kc;
         L.part = part;
+        L.width = split && part == 1 && jk_splits(pd, tl, bc, kc) ? tl.chunk : tl.width;
         L.task_off = tl.task_off;
         L.ket_lo = tl.ket_lo;
         L.ket_hi = tl.ket_hi;

@@ -79,7 +79,7 @@ void System::jk(const double* Dj, int nk, const double* const* Dk, double* Jo, d
   const bool mixed = precision == PYFACC_PRECISION_MIXED;
   if (opt.shard_count > 1) dynamic = false;  // shards use their static sub-lists
   const double t32 = fp32_thresh >= 0 ? fp32_thresh : opt.fp32_thresh;
-  if (dynamic) launch_dyn_tasks(pd, dmax, ns, thresh, mixed ? t32 : 0.0, dyn, stream);
+  if (dynamic) launch_dyn_tasks(pd, dmax, ns, thresh, mixed ? t32 : 0.0, dyn, true, stream);
   // an all-FP32 build (the coarse phase: t32 beyond every Q_ab Q_cd max|D|)
   // has empty FP64 lists, whose kernels are not launched
   const bool fp64_part = !(dynamic && mixed && t32 >= 1e299);
@@ -87,6 +87,7 @@ void System::jk(const double* Dj, int nk, const double* const* Dk, double* Jo, d
   // which swap from class to class; an FP64 build alternates its classes
   // between the two streams (every launch only adds into J and K)
   cudaStream_t s32 = ctx.side;
+  if (any_split) PF_CUDA(cudaMemsetAsync(jk_next, 0, SPLIT_COUNTERS * sizeof(int), stream));
   PF_CUDA(cudaEventRecord(ctx.fork, stream));
   PF_CUDA(cudaStreamWaitEvent(ctx.side, ctx.fork, 0));
   int nth = 0;
@@ -94,14 +95,23 @@ void System::jk(const double* Dj, int nk, const double* const* Dk, double* Jo, d
     for (int kc = bc; kc >= 0; --kc, ++nth) {
       const int qc = (bc == 0) ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
       cudaStream_t s64 = (nth & 1) ? s32 : stream, s32c = (nth & 1) ? stream : s32;
+      // long lists go to the split kernels, whose near half takes the stream
+      // given here and whose far half the other one
+      auto build = [&](const TaskList& tl, bool fp32, cudaStream_t s) {
+        if (jk_splits(pd, tl, bc, kc))
+          launch_jk_split(pd, tl, bc, kc, fp32, nk, a, num_sms, jk_next + 2 * (2 * qc + (fp32 ? 1 : 0)),
+                          s == stream ? ctx.side : stream, s);
+        else
+          launch_jk(pd, tl, bc, kc, fp32, nk, a, num_sms, s);
+      };
       if (dynamic) {
-        if (fp64_part) launch_jk(pd, dyn.lists[2 * qc], bc, kc, false, nk, a, num_sms, mixed ? s64 : stream);
-        if (mixed) launch_jk(pd, dyn.lists[2 * qc + 1], bc, kc, true, nk, a, num_sms, s32c);
+        if (fp64_part) build(dyn.lists[2 * qc], false, mixed ? s64 : stream);
+        if (mixed) build(dyn.lists[2 * qc + 1], true, s32c);
       } else if (mixed) {
-        launch_jk(pd, tasks[bc][kc][1], bc, kc, false, nk, a, num_sms, stream);
-        launch_jk(pd, tasks[bc][kc][2], bc, kc, true, nk, a, num_sms, s32);
+        build(tasks[bc][kc][1], false, stream);
+        build(tasks[bc][kc][2], true, s32);
       } else {
-        launch_jk(pd, tasks[bc][kc][0], bc, kc, false, nk, a, num_sms, (nth & 1) ? ctx.side : stream);
+        build(tasks[bc][kc][0], false, (nth & 1) ? ctx.side : stream);
       }
     }
   // quartets with a d pair: FP64, warp-cooperative kernels (full lists,
@@ -840,7 +850,7 @@ void System::gradient(double* g_host) {
   const bool dyn_split = split && opt.shard_count <= 1;
   if (dyn_split)
     launch_dyn_tasks(pd, dmax, ns, gthr,
-                     opt.gradient_fp32_thresh > 0 ? opt.gradient_fp32_thresh : opt.fp32_thresh, dyn, stream);
+                     opt.gradient_fp32_thresh > 0 ? opt.gradient_fp32_thresh : opt.fp32_thresh, dyn, false, stream);
   // the FP64 and FP32 halves run on different streams, which swap from
   // class to class (an FP64 gradient keeps its classes on one stream: its
   // register-heavy kernels measured slower when two of them share the SMs)

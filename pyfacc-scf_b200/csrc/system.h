@@ -87,6 +87,8 @@ struct System {
   unsigned long long* stats_dev = nullptr;
   const double** ptrs_dev = nullptr;
   double* grad_dev = nullptr;
+  int* jk_next = nullptr;  // task counters of the split J/K kernels
+  bool any_split = false;  // some list goes to them
   DeviceBuf syev_work;
   DeviceBuf small_buf;
   // four TC2 steps (cuBLAS DGEMM + update, ping-pong buffers) as one CUDA
