@@ -177,16 +177,18 @@ struct KetTables {
   float4 *fp = nullptr, *fq = nullptr;    // {P, k}, {P-A, 1/2p}
   float2* fk = nullptr;                   // {p, K}
   float* kabs = nullptr;                  // |K|
+  double* al = nullptr;                   // exponent of the first shell's primitive
   int slot[NCLASS] = {0, 0, 0};
   int class_off[NCLASS + 1] = {0, 0, 0, 0};
   int maxprim[NCLASS] = {0, 0, 0};
-  static constexpr size_t SLOT_BYTES = 5 * sizeof(double2) + 2 * sizeof(float4) + sizeof(float2) + sizeof(float);
+  static constexpr size_t SLOT_BYTES = 5 * sizeof(double2) + 2 * sizeof(float4) + sizeof(float2) + sizeof(float) + sizeof(double);
   // carves the arrays for nslots slots (a multiple of 64) out of base
   void carve(char* base, size_t nslots);
   KetTables part(int c) const {  // the arrays of one class
     KetTables t = *this;
     const int o = slot[c];
     t.xy += o; t.zk += o; t.pq += o; t.zo += o; t.pk += o; t.fp += o; t.fq += o; t.fk += o; t.kabs += o;
+    t.al += o;
     return t;
   }
 };
@@ -303,7 +305,13 @@ int split_chunk(long long nquartets, double far_share, int prim_quartets, int nu
 bool jk_splits(const PairData& pd, const TaskList& tl, int bra_class, int ket_class);
 void launch_jk_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32, int nk,
                      const JkArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
-void upload_boys_rows();  // their Boys tables, on the current device
+// Bound on a quartet's density products, relative to the threshold, below
+// which the split gradient leaves it out.
+constexpr double GRAD_SPLIT_REL = 1e-2;
+void launch_grad_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class,
+                       const struct GradArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
+void upload_boys_rows(int device);  // their Boys tables, on the current device
+const void* boys_rows_table(bool fp32, int L);
 
 // Task lists rebuilt on the GPU for one Fock build from the density bound
 // dmax (ns x ns): a bra pair i keeps the ket prefix with

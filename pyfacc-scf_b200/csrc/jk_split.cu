@@ -31,86 +31,16 @@
 #include <type_traits>
 #include <vector>
 
-#include "boys_rows.cuh"
-#include "engine.h"
-#include "far.cuh"
-#include "quartet.cuh"
+#include "split.cuh"
 
 namespace pyfacc {
 
 namespace {
 
-__device__ BoysRows<double> g_br64[BR_LMAX + 1];
-__device__ BoysRows<float> g_br32[BR_LMAX + 1];
-
-// F_m near and above T = 0 in long double (also for the small negative
-// arguments of the first row's interpolation points).
-long double boys_ld(int m, long double T) {
-  long double sum = 0.0L;
-  if (T < 1.0L) {
-    long double t = 1.0L;
-    for (int k = 0; k < 40; ++k) {
-      sum += t / (2 * m + 2 * k + 1);
-      t *= -T / (k + 1);
-    }
-    return sum;
-  }
-  long double t = 1.0L / (2 * m + 1);
-  for (int k = 1; k < 2000 && t > sum * 1e-22L; ++k) {
-    sum += t;
-    t *= 2.0L * T / (2 * m + 2 * k + 1);
-  }
-  return expl(-T) * sum;
-}
-
-// Monomial coefficients in x of the polynomial that interpolates F_L(c + x)
-// at the n Chebyshev points of |x| <= r.
-void row_coefficients(int L, long double c, long double r, int n, long double* out) {
-  std::vector<long double> f(n), a(n), t0(n, 0.0L), t1(n, 0.0L), t2(n);
-  const long double pi = 3.14159265358979323846264338327950288L;
-  for (int i = 0; i < n; ++i) f[i] = boys_ld(L, c + r * cosl(pi * (i + 0.5L) / n));
-  for (int j = 0; j < n; ++j) {
-    a[j] = 0.0L;
-    for (int i = 0; i < n; ++i) a[j] += f[i] * cosl(pi * j * (i + 0.5L) / n);
-    a[j] *= (j == 0 ? 1.0L : 2.0L) / n;
-  }
-  for (int j = 0; j < n; ++j) out[j] = 0.0L;
-  t0[0] = 1.0L;
-  t1[1] = 1.0L;
-  for (int j = 0; j < n; ++j) {  // t0 = T_j in powers of x / r
-    for (int k = 0; k <= j; ++k) out[k] += a[j] * t0[k];
-    for (int k = 0; k < n; ++k) t2[k] = (k > 0 ? 2.0L * t1[k - 1] : 0.0L) - t0[k];
-    t0 = t1;
-    t1 = t2;
-  }
-  long double s = 1.0L;
-  for (int k = 0; k < n; ++k, s *= r) out[k] /= s;
-}
-
-constexpr int QUEUE = 64;  // a ring: up to 31 left over plus 32 new quartets
-constexpr int MAXSLOT = 8;
-
 struct SplitArgs {
+  SplitLists l;
   JkArgs a;
-  const int* ntasks_dev;
-  const int4* info0;
-  const int4* info2;
-  const double4* geom;
-  const double4* prim;
-  const float4* primf;
-  const float4* test;   // {centre, extent} of all pairs
-  const float4* test2;  // {extent, Q, shells}
-  KetTables ket, bra;  // the classes' parts of the transposed records
-  int nbra_class, ketmaxp;
-  int nket;  // pairs of the ket class
-  const int* task_off;
-  const int* ket_lo;
-  const int* ket_hi;
-  int nbra, ntasks, bra_base, bra_off, ket_base, same_class, qclass, prec, task_begin;
-  int chunk;  // kets per task (a multiple of 32)
-  int maxp;   // bra primitive pairs staged per run
-  int nslot;  // runs staged at a time (a power of two)
-  int* next;  // tasks handed out beyond the first of every warp (zeroed)
+  int prec;
 };
 
 // Staged bra records, in 16-byte vectors per unit: FP64 one primitive pair,
@@ -134,7 +64,7 @@ template <typename R, bool BP, bool FAR> struct Stage {
 // Far bras on one atom have one product centre and are staged as their one
 // equivalent primitive (KetTables row maxp).  Returns the staged count.
 template <bool BP, bool FAR>
-__device__ __forceinline__ int stage_bra(const SplitArgs& a, int bra, const int4& bi0, double, unsigned char* st,
+__device__ __forceinline__ int stage_bra(const SplitLists& a, int bra, const int4& bi0, double, unsigned char* st,
                                          int lane) {
   using S = Stage<double, BP, FAR>;
   const double4* br = a.prim + 3 * (size_t)bi0.z;
@@ -173,7 +103,7 @@ __device__ __forceinline__ int stage_bra(const SplitArgs& a, int bra, const int4
 }
 
 template <bool BP, bool FAR>
-__device__ __forceinline__ int stage_bra(const SplitArgs& a, int bra, const int4& bi0, float, unsigned char* st,
+__device__ __forceinline__ int stage_bra(const SplitLists& a, int bra, const int4& bi0, float, unsigned char* st,
                                          int lane) {
   using S = Stage<float, BP, FAR>;
   const float4* br = a.primf + 3 * (size_t)bi0.z;
@@ -209,11 +139,6 @@ __device__ __forceinline__ int stage_bra(const SplitArgs& a, int bra, const int4
   return np;
 }
 
-// One unit of the bra and one ket primitive in the arithmetic type T (double
-// or F2).
-template <typename T> struct PrimSide {
-  T P[3], k, p, o2p, A[3];  // k: the far prefactor or K; A: P-A or Q-C
-};
 template <bool BP, bool FAR>
 __device__ __forceinline__ void load_unit(const unsigned char* st, int i, PrimSide<double>& b) {
   using S = Stage<double, BP, FAR>;
@@ -252,65 +177,6 @@ __device__ __forceinline__ void load_unit(const unsigned char* st, int i, PrimSi
     b.A[0] = F2(c0.x, c0.y); b.A[1] = F2(c0.z, c0.w); b.A[2] = F2(c1.x, c1.y); b.o2p = F2(c1.z, c1.w);
   }
 }
-template <bool KP, bool FAR>
-__device__ __forceinline__ void load_ket(const SplitArgs& a, size_t sl, PrimSide<double>& k) {
-  const double2 xy = a.ket.xy[sl], zk = a.ket.zk[sl];
-  k.P[0] = xy.x; k.P[1] = xy.y; k.P[2] = zk.x; k.k = zk.y;
-  if (!FAR) {
-    const double2 pk = a.ket.pk[sl];
-    k.p = pk.x; k.k = pk.y;
-  }
-  k.A[0] = k.A[1] = k.A[2] = k.o2p = 0.0;
-  if (KP) {
-    const double2 pq = a.ket.pq[sl], zo = a.ket.zo[sl];
-    k.A[0] = pq.x; k.A[1] = pq.y; k.A[2] = zo.x; k.o2p = zo.y;
-  }
-}
-template <bool KP, bool FAR>
-__device__ __forceinline__ void load_ket(const SplitArgs& a, size_t sl, PrimSide<F2>& k) {
-  const float4 f = a.ket.fp[sl];
-  k.P[0] = F2(f.x); k.P[1] = F2(f.y); k.P[2] = F2(f.z); k.k = F2(f.w);
-  if (!FAR) {
-    const float2 pk = a.ket.fk[sl];
-    k.p = F2(pk.x); k.k = F2(pk.y);
-  }
-  k.A[0] = k.A[1] = k.A[2] = k.o2p = F2(0.0f);
-  if (KP) {
-    const float4 q = a.ket.fq[sl];
-    k.A[0] = F2(q.x); k.A[1] = F2(q.y); k.A[2] = F2(q.z); k.o2p = F2(q.w);
-  }
-}
-
-template <typename T> struct Scalar { using R = double; };
-template <> struct Scalar<F2> { using R = float; };
-
-// A near primitive quartet (prim_setup of quartet.cuh with the short Boys table).
-template <typename T, int L>
-__device__ __forceinline__ void near_setup(const BoysRows<typename Scalar<T>::R>& tab, const T PQ[3],
-                                           const PrimSide<T>& b, const PrimSide<T>& k, PrimGeo<T>& g) {
-  const T rs = far_rsqrt(b.p + k.p);
-  const T oz = rs * rs;
-  const T tt = b.p * k.p * oz * pf_fma(PQ[0], PQ[0], pf_fma(PQ[1], PQ[1], PQ[2] * PQ[2]));
-  const T pref = b.k * k.k * rs;
-  T F[L + 1];
-  boys_rows<L>(tab, tt, F);
-#pragma unroll
-  for (int m = 0; m <= L; ++m) g.I[m] = pref * F[m];
-  if constexpr (L > 0) {
-    const T pz = b.p * oz;
-    g.nrp = k.p * oz * T(-1.0f);
-    g.nrq = pz * T(-1.0f);
-#pragma unroll
-    for (int x = 0; x < 3; ++x) {
-      g.WP[x] = g.nrp * PQ[x];
-      g.WQ[x] = pz * PQ[x];
-    }
-    g.o2p = b.o2p;
-    g.o2q = k.o2p;
-    g.o2pq = T(0.5f) * oz;
-  }
-}
-
 template <typename T, int LA, int LB, int LC, int LD, bool FAR>
 __device__ __forceinline__ void add_prim(const BoysRows<typename Scalar<T>::R>& tab, const PrimSide<T>& b,
                                          const PrimSide<T>& k, T* __restrict__ acc) {
@@ -332,7 +198,7 @@ __device__ __forceinline__ void sum_acc(const F2* a, int i, float* o) { o[i] = a
 // shrinks from one ket primitive to the next.  Light far classes take two ket
 // primitives per pass over the bra, which halves the bra's loads.
 template <typename R, int LA, int LB, int LC, int LD, bool FAR>
-__device__ __forceinline__ int quartet(const SplitArgs& a, const BoysRows<R>& tab, unsigned char* st, int np, int ket,
+__device__ __forceinline__ int quartet(const SplitLists& a, const BoysRows<R>& tab, unsigned char* st, int np, int ket,
                                        int nk, const double4& bgeo, const double4& kgeo, float cut,
                                        R* __restrict__ out) {
   constexpr bool BP = LA + LB > 0, KP = LC + LD > 0;
@@ -353,7 +219,7 @@ __device__ __forceinline__ int quartet(const SplitArgs& a, const BoysRows<R>& ta
     size_t sl = (size_t)kq * a.nket + ket;
     float kcd = a.ket.kabs[sl];
     PrimSide<T> k;
-    load_ket<KP, FAR>(a, sl, k);
+    load_ket<KP, FAR>(a.ket, sl, k);
     while (n > 0 && kab[n - 1] * kcd < cut) --n;
     if (n == 0) break;
     nprim += n;
@@ -364,7 +230,7 @@ __device__ __forceinline__ int quartet(const SplitArgs& a, const BoysRows<R>& ta
         sl += a.nket;
         kcd = a.ket.kabs[sl];
         PrimSide<T> k2;
-        load_ket<KP, FAR>(a, sl, k2);
+        load_ket<KP, FAR>(a.ket, sl, k2);
         while (n > 0 && kab[n - 1] * kcd < cut) --n;
         nprim += n;
         for (; i < n; ++i) {
@@ -398,16 +264,6 @@ __device__ __forceinline__ int quartet(const SplitArgs& a, const BoysRows<R>& ta
   return nprim;
 }
 
-template <typename R> __device__ __forceinline__ const BoysRows<R>* boys_row_table(int L);
-template <> __device__ __forceinline__ const BoysRows<double>* boys_row_table<double>(int L) { return g_br64 + L; }
-template <> __device__ __forceinline__ const BoysRows<float>* boys_row_table<float>(int L) { return g_br32 + L; }
-
-// Largest |D| of the exchange blocks of a quartet.
-__device__ __forceinline__ float dmax_exchange(const float* __restrict__ dm, int ld, int a, int b, int c, int d) {
-  return fmaxf(fmaxf(__ldg(dm + a * ld + c), __ldg(dm + a * ld + d)),
-               fmaxf(__ldg(dm + b * ld + c), __ldg(dm + b * ld + d)));
-}
-
 // Resident blocks per SM that the registers are held to (8 / 6 / 5 instead of
 // 7 / 5 / 4 for L = 0 / 1 / 2: FP32 builds -4%, FP64 the same despite spills).
 __host__ __device__ constexpr int min_blocks(int L) {
@@ -426,128 +282,57 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
   __shared__ typename std::conditional<FAR, int, BoysRows<R>>::type tab_smem;
   const BoysRows<R>& tab = reinterpret_cast<const BoysRows<R>&>(tab_smem);  // near half only
   if constexpr (!FAR) {
-    const unsigned* src = reinterpret_cast<const unsigned*>(boys_row_table<R>(C::L));
+    const unsigned* src = static_cast<const unsigned*>(args.l.boys);
     unsigned* dst = reinterpret_cast<unsigned*>(&tab_smem);
     for (int i = threadIdx.x; i < (int)(sizeof(BoysRows<R>) / 4); i += blockDim.x) dst[i] = src[i];
     __syncthreads();
   }
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-  const int nw = (gridDim.x * blockDim.x) >> 5;
+  const SplitLists& L = args.l;
   const JkArgs& A = args.a;
-  const size_t slot_bytes = S::bytes(args.maxp);
-  unsigned char* st = split_smem + (size_t)wib * args.nslot * slot_bytes;
-  const int ntasks = args.ntasks_dev ? *args.ntasks_dev : args.ntasks;
-  int nquart = 0, qh[NRING] = {}, qn[NRING] = {}, slot = -1;
-  unsigned long long used = 0;  // queued quartets per slot, one byte each
+  const size_t slot_bytes = S::bytes(L.maxp);
+  unsigned char* st = split_smem + (size_t)wib * L.nslot * slot_bytes;
+  int nquart = 0;
   unsigned nprim = 0;
-  int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int k = 0, k1 = 0, ib = 0;
-  while (true) {
-    int kind = -1;  // the ring to evaluate
-#pragma unroll
-    for (int r = 0; r < NRING; ++r)
-      if (qn[r] >= 32) kind = r;
-    if (kind < 0 && k >= k1 && t < ntasks) {
-      const int next = (slot + 1) & (args.nslot - 1);
-      if ((used >> (8 * next)) & 0xff) {  // its last bra still has queued quartets, the oldest of their rings
-#pragma unroll
-        for (int r = 0; r < NRING; ++r)
-          if (qn[r] > 0 && (queue[wib][r][qh[r]].x & (MAXSLOT - 1)) == next) kind = r;
-      } else {  // next run
-        slot = next;
-        const int tg = args.task_begin + t;
-        ib = find_bra(args.task_off, args.nbra, tg);
-        k = __ldg(args.ket_lo + ib) + (tg - __ldg(args.task_off + ib)) * args.chunk;
-        k1 = min(k + args.chunk, __ldg(args.ket_hi + ib));
-        int more = 0;
-        if (lane == 0) more = atomicAdd(args.next, 1);
-        t = nw + __shfl_sync(0xffffffffu, more, 0);
-        const int np = stage_bra<(LA + LB > 0), FAR>(args, args.bra_off + ib, args.info0[args.bra_base + ib], (R)0,
-                                                     st + slot * slot_bytes, lane);
-        if (lane == 0) slot_bra[wib][slot] = make_int2(ib, np);
-        __syncwarp();
-      }
+  auto stage = [&](int ib, int slot) {
+    return stage_bra<(LA + LB > 0), FAR>(L, L.bra_off + ib, L.info0[L.bra_base + ib], (R)0, st + slot * slot_bytes,
+                                         lane);
+  };
+  auto test = [&](int ib, int ket, float& cut) {
+    const int bp = L.bra_base + ib, kp = L.ket_base + ket;
+    const float4 bc = L.test[bp], bt = L.test2[bp], kc = L.test[kp], kt = L.test2[kp];
+    if (far_pair(bc, far_extent<R, C::L>(bc.w, bt.x), kc, far_extent<R, C::L>(kc.w, kt.x)) != FAR) return -1;
+    int to = NRING - 1;
+    if (A.dmax) {
+      const float* dmx = A.dmax + L.info2[bp].w;
+      const int sa = __float_as_int(bt.z), sb = __float_as_int(bt.w), sc = __float_as_int(kt.z),
+                sd = __float_as_int(kt.w);
+      const float dk = dmax_exchange(dmx, A.ns_ld, sa, sb, sc, sd);
+      const float dm = fmaxf(2.0f * fmaxf(__ldg(dmx + sa * A.ns_ld + sb), __ldg(dmx + sc * A.ns_ld + sd)), dk);
+      const float qq = bt.y * kt.y;
+      if (!(qq * dm >= (float)A.thresh)) return -1;
+      if (FAR && !(qq * dk >= (float)A.thresh)) to = 0;
+      cut = __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
     }
-    if (kind < 0 && k < k1) {
-      const int bp = args.bra_base + ib;
-      const float4 bc = args.test[bp], bt = args.test2[bp];
-      const int ket = k + lane;
-      int to = -1;
-      float cut = 0.0f;
-      if (ket < k1) {
-        const int kp = args.ket_base + ket;
-        const float4 kc = args.test[kp], kt = args.test2[kp];
-        if (far_pair(bc, far_extent<R, C::L>(bc.w, bt.x), kc, far_extent<R, C::L>(kc.w, kt.x)) == FAR) to = NRING - 1;
-        if (to >= 0 && A.dmax) {
-          const float* dmx = A.dmax + args.info2[bp].w;
-          const int sa = __float_as_int(bt.z), sb = __float_as_int(bt.w), sc = __float_as_int(kt.z),
-                    sd = __float_as_int(kt.w);
-          const float dk = dmax_exchange(dmx, A.ns_ld, sa, sb, sc, sd);
-          const float dm =
-              fmaxf(2.0f * fmaxf(__ldg(dmx + sa * A.ns_ld + sb), __ldg(dmx + sc * A.ns_ld + sd)), dk);
-          const float qq = bt.y * kt.y;
-          if (!(qq * dm >= (float)A.thresh)) to = -1;
-          else if (FAR && !(qq * dk >= (float)A.thresh)) to = 0;
-          cut = __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
-        }
-      }
-      int added = 0;
-#pragma unroll
-      for (int r = 0; r < NRING; ++r) {
-        const unsigned m = __ballot_sync(0xffffffffu, to == r);
-        if (to == r)
-          queue[wib][r][(qh[r] + qn[r] + __popc(m & ((1u << lane) - 1u))) & (QUEUE - 1)] =
-              make_int2(ket * MAXSLOT + slot, __float_as_int(cut));
-        qn[r] += __popc(m);
-        added += __popc(m);
-      }
-      used += (unsigned long long)added << (8 * slot);
-      k += 32;
-      __syncwarp();
-      continue;
-    }
-    if (kind < 0) {  // the last quartets
-#pragma unroll
-      for (int r = 0; r < NRING; ++r)
-        if (qn[r] > 0) kind = r;
-      if (kind < 0) break;
-    }
-    // ---- the ring's oldest 32 (or all there are): one quartet per lane
-    const int have = NRING == 2 && kind == 1 ? qn[NRING - 1] : qn[0];
-    const int head = NRING == 2 && kind == 1 ? qh[NRING - 1] : qh[0];
-    const int n = min(have, 32);
-    const bool active = lane < n;
-    const int2 e = queue[wib][kind][(head + (active ? lane : 0)) & (QUEUE - 1)];
-    const int es = e.x & (MAXSLOT - 1), ket = e.x / MAXSLOT;
-#pragma unroll
-    for (int r = 0; r < NRING; ++r)
-      if (kind == r) {
-        qh[r] = (qh[r] + n) & (QUEUE - 1);
-        qn[r] -= n;
-      }
-    const int es0 = __shfl_sync(0xffffffffu, es, 0);
-    const bool one_bra = __all_sync(0xffffffffu, !active || es == es0);
-    if (one_bra) used -= (unsigned long long)n << (8 * es0);
-    else
-      for (int x = 0; x < args.nslot; ++x)
-        used -= (unsigned long long)__popc(__ballot_sync(0xffffffffu, active && es == x)) << (8 * x);
-    const int2 sb = slot_bra[wib][es];
-    const int bp = args.bra_base + sb.x, kp = args.ket_base + ket;
-    const int4 bi0 = args.info0[bp], ki0 = args.info0[kp], bi2 = args.info2[bp];
+    return to;
+  };
+  auto eval = [&](int kind, const Queued& q) {
+    const int bp = L.bra_base + q.bra.x, kp = L.ket_base + q.ket;
+    const int4 bi0 = L.info0[bp], ki0 = L.info0[kp], bi2 = L.info2[bp];
     const int mo = bi2.x, ld = bi2.y, ma = bi0.x, mb = bi0.y, mc = ki0.x, md = ki0.y;
     double jab[NA * NB];
 #pragma unroll
     for (int i = 0; i < NA * NB; ++i) jab[i] = 0.0;
-    if (active) {
+    if (q.active) {
       R out[C::NOUT];
-      nprim += quartet<R, LA, LB, LC, LD, FAR>(args, tab, st + es * slot_bytes, sb.y, ket, ki0.w, args.geom[bp],
-                                               args.geom[kp], __int_as_float(e.y), out);
+      nprim += quartet<R, LA, LB, LC, LD, FAR>(L, tab, st + q.slot * slot_bytes, q.bra.y, q.ket, ki0.w, L.geom[bp],
+                                               L.geom[kp], q.cut, out);
       ++nquart;
       double fac = 1.0;
-      const float4 bt = args.test2[bp], kt = args.test2[kp];
+      const float4 bt = L.test2[bp], kt = L.test2[kp];
       if (__float_as_int(bt.z) == __float_as_int(bt.w)) fac *= 0.5;
       if (__float_as_int(kt.z) == __float_as_int(kt.w)) fac *= 0.5;
-      if (args.same_class && bp == kp) fac *= 0.5;
+      if (L.same_class && bp == kp) fac *= 0.5;
       // ---- Coulomb
       double Dab[NA * NB], jcd[NCc * ND];
 #pragma unroll
@@ -636,18 +421,18 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
       }
     }
     // J_ab: one atomic per warp while all lanes share the bra
-    if (one_bra) {
+    if (q.one_bra) {
 #pragma unroll
       for (int i = 0; i < NA * NB; ++i) {
         const double s = warp_sum(jab[i]);
         if (lane == 0) atomicAdd(A.J + mo + (ma + i / NB) * ld + mb + i % NB, 2.0 * s);
       }
-    } else if (active) {
+    } else if (q.active) {
 #pragma unroll
       for (int i = 0; i < NA * NB; ++i) atomicAdd(A.J + mo + (ma + i / NB) * ld + mb + i % NB, 2.0 * jab[i]);
     }
-    __syncwarp();  // the ring and slot entries read above may be overwritten
-  }
+  };
+  split_run<NRING>(L, queue[wib], slot_bra[wib], stage, test, eval);
   if (A.stats) {  // contracted and evaluated primitive quartets
     unsigned long long nq = (unsigned)nquart, p = nprim;
 #pragma unroll
@@ -656,8 +441,8 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
       p += __shfl_xor_sync(0xffffffffu, p, o);
     }
     if (lane == 0 && nq) {
-      atomicAdd(A.stats + args.prec * NQCLASS + args.qclass, nq);
-      atomicAdd(A.stats + (2 + args.prec) * NQCLASS + args.qclass, p);
+      atomicAdd(A.stats + args.prec * NQCLASS + L.qclass, nq);
+      atomicAdd(A.stats + (2 + args.prec) * NQCLASS + L.qclass, p);
     }
   }
 }
@@ -668,10 +453,10 @@ constexpr size_t STAGE_MAX_BYTES = 24 * 1024;
 
 template <typename R, int LA, int LB, int LC, int LD, int NK, bool FAR>
 void launch_one(int blocks, cudaStream_t s, SplitArgs k) {
-  const size_t b = Stage<R, (LA + LB > 0), FAR>::bytes(k.maxp);
-  k.nslot = MAXSLOT;
-  while (k.nslot > 2 && 4 * k.nslot * b > STAGE_MAX_BYTES) k.nslot /= 2;
-  const size_t smem = 4 * k.nslot * b;
+  const size_t b = Stage<R, (LA + LB > 0), FAR>::bytes(k.l.maxp);
+  k.l.nslot = MAXSLOT;
+  while (k.l.nslot > 2 && 4 * k.l.nslot * b > STAGE_MAX_BYTES) k.l.nslot /= 2;
+  const size_t smem = 4 * k.l.nslot * b;
   if (smem > 32 * 1024)
     PF_CUDA(cudaFuncSetAttribute(jk_split_kernel<R, LA, LB, LC, LD, NK, FAR>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -684,11 +469,11 @@ template <typename R, int LA, int LB, int LC, int LD>
 void launch_halves(int nk, int blocks, cudaStream_t s_far, cudaStream_t s_near, SplitArgs k) {
   if (nk == 1) {
     launch_one<R, LA, LB, LC, LD, 1, false>(blocks, s_near, k);
-    ++k.next;
+    ++k.l.next;
     launch_one<R, LA, LB, LC, LD, 1, true>(blocks, s_far, k);
   } else {
     launch_one<R, LA, LB, LC, LD, 2, false>(blocks, s_near, k);
-    ++k.next;
+    ++k.l.next;
     launch_one<R, LA, LB, LC, LD, 2, true>(blocks, s_far, k);
   }
 }
@@ -705,35 +490,6 @@ void dispatch(int qc, int nk, int blocks, cudaStream_t s_far, cudaStream_t s_nea
 }
 
 }  // namespace
-
-// Boys rows of the current device (called once per device, under the lock of
-// ensure_boys_tables).
-void upload_boys_rows() {
-  static std::vector<BoysRows<double>> t64;
-  static std::vector<BoysRows<float>> t32;
-  if (t64.empty()) {
-    t64.resize(BR_LMAX + 1);
-    t32.resize(BR_LMAX + 1);
-    for (int L = 0; L <= BR_LMAX; ++L)
-      for (int r = 0; r < BR_ROWS; ++r) {
-        long double c[BR_N64];
-        const long double h = br_step<double>(L);
-        row_coefficients(L, r * h, 0.5L * h, BR_N64, c);
-        for (int j = 0; j < BR_N64; ++j) {
-          const double v = (double)c[j];
-          unsigned long long u;
-          std::memcpy(&u, &v, 8);
-          t64[L].hi[j][r] = (unsigned)(u >> 32);
-          t64[L].lo[j][r] = (unsigned)u;
-        }
-        const long double hf = (float)br_step<float>(L);
-        row_coefficients(L, r * hf, 0.5L * hf, BR_N32, c);
-        for (int j = 0; j < BR_N32; ++j) t32[L].c[j][r] = (float)c[j];
-      }
-  }
-  PF_CUDA(cudaMemcpyToSymbol(g_br64, t64.data(), sizeof(g_br64)));
-  PF_CUDA(cudaMemcpyToSymbol(g_br32, t32.data(), sizeof(g_br32)));
-}
 
 // Kets per run of a list that the split kernels take, 0 for one they do not.
 // They pay for their second pass over the candidates with the far quartets:
@@ -760,32 +516,17 @@ bool jk_splits(const PairData& pd, const TaskList& tl, int bc, int kc) {
 void launch_jk_split(const PairData& pd, const TaskList& tl, int bc, int kc, bool fp32, int nk, const JkArgs& a,
                      int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near) {
   if (tl.ntasks_c <= 0) return;
+  if (fp32 && !pd.primf) throw Error(PYFACC_ERR_INVALID, "FP32 quartets need float primitive records");
   SplitArgs k{};
+  k.l = split_lists(pd, tl, bc, kc, next);
+  k.l.boys = boys_rows_table(fp32, class_flops(k.l.qclass).L);
   k.a = a;
-  k.ntasks_dev = tl.ntasks_dev;
-  k.info0 = pd.info0; k.info2 = pd.info2;
-  k.geom = pd.geom; k.prim = pd.prim; k.primf = pd.primf;
-  k.test = pd.test; k.test2 = pd.test + pd.npair;
-  k.ket = pd.kt.part(kc);
-  k.bra = pd.kt.part(bc);
-  k.nbra_class = pd.class_off[bc + 1] - pd.class_off[bc];
-  k.bra_off = tl.bra_offset;
-  k.ketmaxp = pd.class_maxprim[kc];
-  k.nket = pd.class_off[kc + 1] - pd.class_off[kc];
-  k.task_off = tl.off_c; k.ket_lo = tl.ket_lo; k.ket_hi = tl.ket_hi;
-  k.nbra = tl.nbra; k.ntasks = tl.ntasks_c; k.task_begin = tl.task_begin_c;
-  k.bra_base = pd.class_off[bc] + tl.bra_offset; k.ket_base = pd.class_off[kc];
-  k.same_class = bc == kc;
-  k.qclass = bc == 0 ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
   k.prec = fp32 ? 1 : 0;
-  k.chunk = tl.chunk;
-  k.maxp = pd.class_maxprim[bc];
-  k.next = next;
   // resident warps only; the tasks beyond their first go to whichever is free
-  const int per_sm = min_blocks(class_flops(k.qclass).L);
+  const int per_sm = min_blocks(class_flops(k.l.qclass).L);
   const int blocks = (int)std::max(1LL, std::min((tl.ntasks_c + 3LL) / 4, (long long)num_sms * per_sm));
-  if (fp32) dispatch<float>(k.qclass, nk, blocks, s_far, s_near, k);
-  else dispatch<double>(k.qclass, nk, blocks, s_far, s_near, k);
+  if (fp32) dispatch<float>(k.l.qclass, nk, blocks, s_far, s_near, k);
+  else dispatch<double>(k.l.qclass, nk, blocks, s_far, s_near, k);
 }
 
 }  // namespace pyfacc

@@ -72,7 +72,7 @@ void ensure_boys_tables(int device) {
     PF_CUDA(cudaMemcpyToSymbol(g_boys_exp, ex.data(), ex.size() * sizeof(double)));
     PF_CUDA(cudaMemcpyToSymbol(g_boys_tlf, tabf.data(), tabf.size() * sizeof(float)));
     upload_boys_tables_d(tl.data(), tl.size(), ex.data(), ex.size());
-    upload_boys_rows();
+    upload_boys_rows(device);
     done[device] = 1;
   }
 }
@@ -298,6 +298,7 @@ __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, con
       kt.fq[sl] = make_float4((float)r2.x, (float)r2.y, (float)r2.z, (float)r2.w);
       kt.fk[sl] = make_float2((float)r0.x, (float)r0.z);
       kt.kabs[sl] = fabsf((float)r0.z);
+      kt.al[sl] = r0.w;
     }
     ++nk;
   }
@@ -362,6 +363,7 @@ void KetTables::carve(char* b, size_t n) {
   fp = reinterpret_cast<float4*>(take(sizeof(float4)));
   fq = reinterpret_cast<float4*>(take(sizeof(float4)));
   fk = reinterpret_cast<float2*>(take(sizeof(float2)));
+  al = reinterpret_cast<double*>(take(sizeof(double)));
   kabs = reinterpret_cast<float*>(take(sizeof(float)));
 }
 

@@ -820,7 +820,8 @@ void System::gradient(double* g_host) {
   g1.natoms_total = natoms;
   // one-electron terms once (shard 0); the two-electron term is sharded
   if (opt.shard_count <= 1 || opt.shard_rank == 0) launch_grad1e(shd, n1e, pairs1e, g1, num_sms, stream);
-  launch_dmax(ns, bf_off_dev, nfun_dev, nbf, Pt, nullptr, nullptr, dmax, stream);
+  // the split kernels bound density products, spin by spin for an open shell
+  launch_dmax(ns, bf_off_dev, nfun_dev, nbf, Pt, uhf ? P[0] : nullptr, uhf ? P[1] : nullptr, dmax, stream);
   GradArgs g2;
   g2.Pt = Pt;
   g2.Pa = uhf ? Ps[0] : Pt;
@@ -855,20 +856,27 @@ void System::gradient(double* g_host) {
   // class to class (an FP64 gradient keeps its classes on one stream: its
   // register-heavy kernels measured slower when two of them share the SMs)
   cudaStream_t s32 = ctx.side;
+  if (any_split) PF_CUDA(cudaMemsetAsync(jk_next, 0, SPLIT_COUNTERS * sizeof(int), stream));
   PF_CUDA(cudaEventRecord(ctx.fork, stream));
   PF_CUDA(cudaStreamWaitEvent(ctx.side, ctx.fork, 0));
   int nth = 0;
   for (int bc = NCLASS - 1; bc >= 0; --bc)
     for (int kc = bc; kc >= 0; --kc, ++nth) {
+      const int qc = (bc == 0) ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
+      auto derive = [&](const TaskList& tl, bool fp32, cudaStream_t s) {
+        if (!fp32 && jk_splits(pd, tl, bc, kc))
+          launch_grad_split(pd, tl, bc, kc, g2, num_sms, jk_next + 4 * qc, s == stream ? ctx.side : stream, s);
+        else
+          launch_grad2e(pd, tl, bc, kc, fp32, g2, num_sms, s);
+      };
       if (dyn_split) {
-        const int qc = (bc == 0) ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
-        launch_grad2e(pd, dyn.lists[2 * qc], bc, kc, false, g2, num_sms, (nth & 1) ? s32 : stream);
-        launch_grad2e(pd, dyn.lists[2 * qc + 1], bc, kc, true, g2, num_sms, (nth & 1) ? stream : s32);
+        derive(dyn.lists[2 * qc], false, (nth & 1) ? s32 : stream);
+        derive(dyn.lists[2 * qc + 1], true, (nth & 1) ? stream : s32);
       } else if (split) {
-        launch_grad2e(pd, tasks[bc][kc][1], bc, kc, false, g2, num_sms, stream);
-        launch_grad2e(pd, tasks[bc][kc][2], bc, kc, true, g2, num_sms, s32);
+        derive(tasks[bc][kc][1], false, stream);
+        derive(tasks[bc][kc][2], true, s32);
       } else {
-        launch_grad2e(pd, tasks[bc][kc][0], bc, kc, false, g2, num_sms, stream);
+        derive(tasks[bc][kc][0], false, stream);
       }
     }
   if (has_d)
