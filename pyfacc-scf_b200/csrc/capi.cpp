@@ -466,12 +466,17 @@ int pyfacc_purify_dev(int n, int nocc, const double* F_dev, double* P_dev, int* 
     double* Xb = work.as<double>();
     double* state = Xb + n2 + n2;
     // the projector is built in P_dev itself (the graph's X_a)
-    cudaGraphExec_t g = pyfacc::build_tc2_graph(n, nocc, F_dev, P_dev, Xb, state, pyfacc::TC2_KMAX);
-    const cudaError_t e = cudaGraphLaunch(g, 0);
     double ctl[8];
-    cudaError_t e2 = e == cudaSuccess ? cudaMemcpy(ctl, state + 8, sizeof(ctl), cudaMemcpyDeviceToHost) : e;
-    cudaGraphExecDestroy(g);
-    PF_CUDA(e2);
+    if (n <= pyfacc::TC2_SMALL_MAX) {
+      pyfacc::launch_tc2_small(n, nocc, F_dev, P_dev, state, pyfacc::TC2_KMAX, 0);
+      PF_CUDA(cudaMemcpy(ctl, state + 8, sizeof(ctl), cudaMemcpyDeviceToHost));
+    } else {
+      cudaGraphExec_t g = pyfacc::build_tc2_graph(n, nocc, F_dev, P_dev, Xb, state, pyfacc::TC2_KMAX);
+      const cudaError_t e = cudaGraphLaunch(g, 0);
+      cudaError_t e2 = e == cudaSuccess ? cudaMemcpy(ctl, state + 8, sizeof(ctl), cudaMemcpyDeviceToHost) : e;
+      cudaGraphExecDestroy(g);
+      PF_CUDA(e2);
+    }
     if (steps) *steps = (int)ctl[2];
     if (ctl[1] == 0.0 || ctl[4] != 0.0) status = PYFACC_ERR_NOT_CONVERGED;
   });

@@ -620,7 +620,7 @@ void System::build_tasks() {
 
 void System::alloc_matrices() {
   const size_t n2 = (size_t)nbf * nbf;
-  const int nmat = 30 + 4 * std::max(opt.diis_size, 1);
+  const int nmat = 31 + 4 * std::max(opt.diis_size, 1);
   mats.ensure(nmat * n2 * sizeof(double) + 96 * sizeof(double) + ns * ns * sizeof(float) + 1024);
   double* m = mats.as<double>();
   auto take = [&]() { double* r = m; m += n2; return r; };
@@ -631,6 +631,7 @@ void System::alloc_matrices() {
   Wm = take();
   Pu[0] = take(); Pu[1] = take(); Pu[2] = take(); Pu[3] = take();
   Pp[0] = take(); Pp[1] = take();
+  Xt = take();
   const int nd = std::max(opt.diis_size, 1);
   for (int i = 0; i < nd; ++i) {
     diis_F.push_back(m); m += 2 * n2;

@@ -394,7 +394,8 @@ void launch_grad1e(const ShellDev& sh, const int* npair, const int2* const* pair
 void launch_symmetrize_add(int n, double* A, cudaStream_t s);
 void launch_set_diag(int n, const double* d, double f, double* A, cudaStream_t s);  // A = diag(f d)
 void launch_min_diag_sq(int n, const double* L, double* out, cudaStream_t s);   // out = min_i L_ii^2
-void launch_identity(int n, double* A, cudaStream_t s);                  // A = I (n x n)             // A = A + A^T
+void launch_identity(int n, double* A, cudaStream_t s);                  // A = I (n x n)
+void launch_transpose(int n, const double* A, double* B, cudaStream_t s);  // B = A^T (n x n)
 void launch_axpby(long long n, double a, const double* x, double b, double* y, cudaStream_t s);  // y = a x + b y
 void launch_antisym(int n, const double* B, double* E, cudaStream_t s);  // E = B - B^T (n x n)
 void launch_diff_update(long long n, const double* x, double* y, double* out, cudaStream_t s);  // out = x - y; y = x
@@ -447,6 +448,11 @@ void launch_dgemm(int m, int n, int k, bool ta, const double* A, int lda, bool t
 cudaGraphExec_t build_tc2_graph(int n, int nocc, const double* Fp, double* Xa, double* Xb, double* st, int kmax);
 constexpr int TC2_KMAX = 200;
 constexpr int TC2_BODY_STEPS = 4;  // TC2 steps per WHILE iteration (even: the result ends in Xa)
+constexpr int TC2_LEAD_STEPS = 16;  // ... and before the WHILE node (even)
+// The same for n <= TC2_SMALL_MAX, one kernel of one block: the projector into
+// X, the outcome into the same words of st.
+constexpr int TC2_SMALL_MAX = 72;
+void launch_tc2_small(int n, int nocc, const double* Fp, double* X, double* st, int kmax, cudaStream_t s);
 
 double probe_fp64(int device, double* fp32);
 

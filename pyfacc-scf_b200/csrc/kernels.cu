@@ -1718,6 +1718,22 @@ void launch_identity(int n, double* A, cudaStream_t s) {
   count_launch();
 }
 
+__global__ void transpose_kernel(int n, const double* __restrict__ A, double* __restrict__ B) {
+  __shared__ double t[32][33];
+  const int i0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
+  for (int r = threadIdx.y; r < 32; r += blockDim.y)
+    if (i0 + r < n && j0 + threadIdx.x < n) t[r][threadIdx.x] = A[(size_t)(i0 + r) * n + j0 + threadIdx.x];
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32; r += blockDim.y)
+    if (j0 + r < n && i0 + threadIdx.x < n) B[(size_t)(j0 + r) * n + i0 + threadIdx.x] = t[threadIdx.x][r];
+}
+void launch_transpose(int n, const double* A, double* B, cudaStream_t s) {
+  dim3 b(32, 8), g((n + 31) / 32, (n + 31) / 32);
+  transpose_kernel<<<g, b, 0, s>>>(n, A, B);
+  PF_CUDA(cudaGetLastError());
+  count_launch();
+}
+
 void launch_symmetrize_add(int n, double* A, cudaStream_t s) {
   dim3 b(32, 8), g((n + 31) / 32, (n + 7) / 8);
   symmetrize_add_kernel<<<g, b, 0, s>>>(n, A);

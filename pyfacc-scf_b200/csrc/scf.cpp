@@ -192,6 +192,7 @@ void System::orthogonalizer() {
   const double one = 1.0;
   PF_CUBLAS(cublasDtrsm(cublas, CUBLAS_SIDE_LEFT, CUBLAS_FILL_MODE_LOWER, CUBLAS_OP_T, CUBLAS_DIAG_NON_UNIT, nbf, nbf,
                         &one, L, nbf, X, nbf));
+  launch_transpose(nbf, X, Xt, stream);
 }
 
 // The overlap factorisation's outcome (after a synchronisation that follows
@@ -282,12 +283,14 @@ std::vector<double> System::atomic_occupations() const {
 
 // The buffer X holds, read row-major, R = L^{-1} (cuBLAS wrote X = L^{-T}
 // column-major), so X^T F X = R F R^T and X P' X^T = R^T P' R in the
-// row-major products of dense.cu.
+// row-major products of dense.cu.  With F and P' symmetric and Xt = R^T every
+// product of an iteration is A B^T of row-major matrices, (R F) R^T and
+// (R^T P') R, both operands contiguous along k.
 bool System::purify(const double* Fm, int nocc, double scale, double* Pm, double* Pp) {
   const int n = nbf;
   if (nocc > 0 && nocc < n) {  // F' = R F R^T into the graph's input
-    launch_dgemm(n, n, n, false, Fm, n, true, X, n, W1, n, 1.0, nullptr, n, 0.0, false, false, stream);
-    launch_dgemm(n, n, n, false, X, n, false, W1, n, Pu[0], n, 1.0, nullptr, n, 0.0, true, false, stream);
+    launch_dgemm(n, n, n, false, X, n, true, Fm, n, W1, n, 1.0, nullptr, n, 0.0, false, false, stream);
+    launch_dgemm(n, n, n, false, W1, n, true, X, n, Pu[0], n, 1.0, nullptr, n, 0.0, true, false, stream);
   }
   return purify_core(nocc, scale, Pm, Pp);
 }
@@ -313,10 +316,11 @@ bool System::purify_core(int nocc, double scale, double* Pm, double* Pp) {
     return true;
   }
   double* Xa = Pu[1];
-  // the whole TC2 iteration is one graph launch (conditional WHILE loop on
-  // the device); the host reads the outcome once
+  // the whole TC2 iteration is one launch (of a kernel, or of a graph with a
+  // conditional WHILE loop); the host reads the outcome once
   if (opt.verbose) PF_CUDA(cudaEventRecord(ctx.ev0, stream));
-  PF_CUDA(cudaGraphLaunch(tc2_graph(nocc), stream));
+  if (n <= TC2_SMALL_MAX) launch_tc2_small(n, nocc, Pu[0], Xa, pstate, TC2_KMAX, stream);
+  else PF_CUDA(cudaGraphLaunch(tc2_graph(nocc), stream));
   if (opt.verbose) PF_CUDA(cudaEventRecord(ctx.ev1, stream));
   // the outcome into pinned memory; the projector's copy and the
   // back-transform are queued before it is read, so they run while the host
@@ -327,13 +331,16 @@ bool System::purify_core(int nocc, double scale, double* Pm, double* Pp) {
   PF_CUDA(cudaEventRecord(ctx.ready, stream));
   if (Pp) PF_CUDA(cudaMemcpyAsync(Pp, Xa, bytes, cudaMemcpyDeviceToDevice, stream));
   // P = scale R^T Xp R
-  launch_dgemm(n, n, n, false, Xa, n, false, X, n, W1, n, 1.0, nullptr, n, 0.0, false, false, stream);
-  launch_dgemm(n, n, n, true, X, n, false, W1, n, Pm, n, scale, nullptr, n, 0.0, true, false, stream);
+  launch_dgemm(n, n, n, false, Xt, n, true, Xa, n, W1, n, 1.0, nullptr, n, 0.0, false, false, stream);
+  launch_dgemm(n, n, n, false, W1, n, true, Xt, n, Pm, n, scale, nullptr, n, 0.0, true, false, stream);
   PF_CUDA(cudaEventSynchronize(ctx.ready));
   double ctl[8];
   std::memcpy(ctl, ctl_pinned, sizeof(ctl));
   const int steps = (int)ctl[2];
-  count_launches(2 + (steps + TC2_BODY_STEPS - 1) / TC2_BODY_STEPS * TC2_BODY_STEPS);
+  if (n > TC2_SMALL_MAX) {
+    const int more = std::max(0, steps - TC2_LEAD_STEPS);
+    count_launches(2 + TC2_LEAD_STEPS + (more + TC2_BODY_STEPS - 1) / TC2_BODY_STEPS * TC2_BODY_STEPS);
+  }
   purify_steps += steps;
   if (opt.verbose) purify_ms += elapsed(ctx.ev0, ctx.ev1);
   return !(ctl[1] == 0.0 || ctl[4] != 0.0);
@@ -584,12 +591,12 @@ void System::run_scf() {
       if (slot >= 0) Eo[s] = diis_E[slot] + s * n2;
       if (orth_diis) {  // F' = R F R^T, the stored DIIS vector
         double* Fo = diis_F[slot] + s * n2;
-        launch_dgemm(nbf, nbf, nbf, false, F[s], nbf, true, X, nbf, W1, nbf, 1.0, nullptr, nbf, 0.0, false, false,
+        launch_dgemm(nbf, nbf, nbf, false, X, nbf, true, F[s], nbf, W1, nbf, 1.0, nullptr, nbf, 0.0, false, false,
                      stream);
-        launch_dgemm(nbf, nbf, nbf, false, X, nbf, false, W1, nbf, Fo, nbf, 1.0, nullptr, nbf, 0.0, true, false,
+        launch_dgemm(nbf, nbf, nbf, false, W1, nbf, true, X, nbf, Fo, nbf, 1.0, nullptr, nbf, 0.0, true, false,
                      stream);
         if (use_pp) {
-          launch_dgemm(nbf, nbf, nbf, false, Fo, nbf, false, Pp[s], nbf, W1, nbf, pscale, nullptr, nbf, 0.0, false,
+          launch_dgemm(nbf, nbf, nbf, false, Fo, nbf, true, Pp[s], nbf, W1, nbf, pscale, nullptr, nbf, 0.0, false,
                        false, stream);
           launch_antisym(nbf, W1, Eo[s], stream);
           continue;
@@ -794,9 +801,9 @@ void System::gradient(double* g_host) {
   const int nsp = uhf ? 2 : 1;
   for (int s = 0; s < nsp; ++s) {
     const double f = uhf ? 1.0 : 0.5;
-    launch_dgemm(nbf, nbf, nbf, false, F[s], nbf, false, P[s], nbf, W1, nbf, 1.0, nullptr, nbf, 0.0, false, false,
+    launch_dgemm(nbf, nbf, nbf, false, P[s], nbf, true, F[s], nbf, W1, nbf, 1.0, nullptr, nbf, 0.0, false, false,
                  stream);
-    launch_dgemm(nbf, nbf, nbf, false, P[s], nbf, false, W1, nbf, Wm, nbf, f, s == 0 ? nullptr : Wm, nbf, 1.0, true,
+    launch_dgemm(nbf, nbf, nbf, false, W1, nbf, true, P[s], nbf, Wm, nbf, f, s == 0 ? nullptr : Wm, nbf, 1.0, true,
                  false, stream);
   }
   // total density and spin densities of the converged SCF

@@ -65,7 +65,7 @@ struct System {
   DeviceBuf dyn_buf;
 
   DeviceBuf mats;
-  double *S = nullptr, *T = nullptr, *Vm = nullptr, *H = nullptr, *X = nullptr;
+  double *S = nullptr, *T = nullptr, *Vm = nullptr, *H = nullptr, *X = nullptr, *Xt = nullptr;
   double *F[2] = {nullptr, nullptr}, *J = nullptr, *K[2] = {nullptr, nullptr};
   double *P[2] = {nullptr, nullptr}, *Pbuilt[2] = {nullptr, nullptr}, *Pold[2] = {nullptr, nullptr};
   double *W1 = nullptr, *W2 = nullptr, *W3 = nullptr, *Err[2] = {nullptr, nullptr};
