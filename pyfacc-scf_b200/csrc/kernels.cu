@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <atomic>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "engine.h"
@@ -181,24 +182,43 @@ void launch_build_pairs(const ShellDev& sh, int npair, const int4* pl0, const in
   count_launch();
 }
 
-// Schwarz factor of every pair of one class: Q = sqrt(max |(ab|ab)|).
-template <int LA, int LB>
+// Schwarz factor of every pair of one class: Q = sqrt(max |(ab|ab)|).  G lanes
+// share a pair, each summing every G-th ket primitive (G = 8 for the few pairs
+// of a small molecule, whose one-lane quartets took 23-54 us).
+template <int LA, int LB, int G>
 __global__ void schwarz_kernel(int begin, int end, const int4* __restrict__ info0, const double4* __restrict__ geom,
                                const double4* __restrict__ prim, double* __restrict__ q) {
-  int i = begin + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= end) return;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, sub = t % G;
+  const int i = begin + t / G;
+  const bool valid = i < end;
+  if (G == 1 && !valid) return;
   using C = EriClass<double, LA, LB, LA, LB>;
   double out[C::NOUT];
-  const int4 i0 = info0[i];
-  const double4 g = geom[i];
-  contracted_quartet<double, LA, LB, LA, LB>(prim, prim + 3 * (size_t)i0.z, i0, i0, g, g, out);
+  const int4 i0 = info0[valid ? i : begin];
+  const double4 g = geom[valid ? i : begin];
+  contracted_quartet<double, LA, LB, LA, LB>(prim, prim + 3 * (size_t)i0.z, i0, i0, g, g, out, 0.0, sub, G);
   constexpr int NA = NC<LA>::v, NB = NC<LB>::v;
   double mx = 0.0;
 #pragma unroll
   for (int a = 0; a < NA; ++a)
 #pragma unroll
-    for (int b = 0; b < NB; ++b) mx = fmax(mx, fabs(out[((a * NB + b) * NA + a) * NB + b]));
-  q[i] = sqrt(mx);
+    for (int b = 0; b < NB; ++b) {
+      double v = out[((a * NB + b) * NA + a) * NB + b];
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+      mx = fmax(mx, fabs(v));
+    }
+  if (valid && sub == 0) q[i] = sqrt(mx);
+}
+
+constexpr int SCHWARZ_WIDE_MAX = 4096;  // pairs of a class that 8 lanes each still leave the GPU part empty
+
+template <int G>
+static void schwarz_class(int c, int begin, int end, const PairData& pd, double* q, cudaStream_t st) {
+  dim3 grid(((end - begin) * G + 63) / 64), block(64);
+  if (c == 0) schwarz_kernel<0, 0, G><<<grid, block, 0, st>>>(begin, end, pd.info0, pd.geom, pd.prim, q);
+  if (c == 1) schwarz_kernel<1, 0, G><<<grid, block, 0, st>>>(begin, end, pd.info0, pd.geom, pd.prim, q);
+  if (c == 2) schwarz_kernel<1, 1, G><<<grid, block, 0, st>>>(begin, end, pd.info0, pd.geom, pd.prim, q);
 }
 
 void launch_schwarz(const PairData& pd, int off[NCLASS + 1], double* q, cudaStream_t s, cudaStream_t side,
@@ -211,11 +231,9 @@ void launch_schwarz(const PairData& pd, int off[NCLASS + 1], double* q, cudaStre
   for (int c = NCLASS - 1; c >= 0; --c) {  // the longest class first
     int n = off[c + 1] - off[c];
     if (n <= 0) continue;
-    dim3 grid((n + 63) / 64), block(64);
     cudaStream_t st = (two && c == NCLASS - 1) ? side : s;
-    if (c == 0) schwarz_kernel<0, 0><<<grid, block, 0, st>>>(off[c], off[c + 1], pd.info0, pd.geom, pd.prim, q);
-    if (c == 1) schwarz_kernel<1, 0><<<grid, block, 0, st>>>(off[c], off[c + 1], pd.info0, pd.geom, pd.prim, q);
-    if (c == 2) schwarz_kernel<1, 1><<<grid, block, 0, st>>>(off[c], off[c + 1], pd.info0, pd.geom, pd.prim, q);
+    if (n <= SCHWARZ_WIDE_MAX) schwarz_class<8>(c, off[c], off[c + 1], pd, q, st);
+    else schwarz_class<1>(c, off[c], off[c + 1], pd, q, st);
     PF_CUDA(cudaGetLastError());
     count_launch();
   }
@@ -395,8 +413,9 @@ struct JkKernelArgs {
   const int* ket_hi;
   int nbra, ntasks, bra_base, ket_base, same_class, qclass, prec, task_begin;
   int lwidth;  // log2 of the task width: one warp runs 32 >> lwidth tasks of (1 bra) x (1 << lwidth kets)
-  int psplit;  // warps per task (each takes every psplit-th ket primitive)
+  int psplit;  // (pp|pp): warps per task (each takes every psplit-th ket primitive)
   int stage;   // primitive records staged per bra in shared memory (0: read from global memory)
+  int lpq;     // lanes per quartet
 };
 
 // Warps per task for a list of the given length: lists with too few warps
@@ -407,6 +426,17 @@ static int primitive_split(long long warps, int num_sms) {
   int ps = 1;
   while (ps < 8 && warps * ps < (long long)num_sms * 32) ps *= 2;
   return ps;
+}
+
+// Lanes per quartet of a J/K list below (pp|pp) of the given length: with few
+// warps one lane per quartet runs its up to 81 primitive quartets one after
+// the other on an empty GPU (water: 36-55 us a class).  The lanes of a quartet
+// sum four slices of the ket primitives and LPQ / 4 of the bra's and add their
+// integrals by shuffles; sharing a task between warps instead, each digesting
+// its share, multiplied the atomics on the same few addresses and was slower
+// than no split (10 carbons: Fock builds 3.7 -> 7.3 ms).
+static int lanes_per_quartet(long long warps, int num_sms) {
+  return warps <= num_sms ? 16 : (warps <= 8LL * num_sms ? 4 : 1);
 }
 
 // Whether any lane of this lane's aligned group of w lanes is active.
@@ -425,7 +455,9 @@ template <typename R> __device__ __forceinline__ const typename Rec<R>::T* recor
 template <> __device__ __forceinline__ const double4* records<double>(const JkKernelArgs& a) { return a.prim; }
 template <> __device__ __forceinline__ const float4* records<float>(const JkKernelArgs& a) { return a.primf; }
 
-template <typename R, int LA, int LB, int LC, int LD, int NK>
+// LPQ: lanes per quartet (tasks of 32 kets only when above 1: a task then
+// takes LPQ consecutive warps of 32 / LPQ kets each).
+template <typename R, int LA, int LB, int LC, int LD, int NK, int LPQ>
 __global__ void __launch_bounds__(128) jk_kernel(const JkKernelArgs args) {
   using C = EriClass<R, LA, LB, LC, LD>;
   constexpr int NA = NC<LA>::v, NB = NC<LB>::v, NCc = NC<LC>::v, ND = NC<LD>::v;
@@ -436,16 +468,21 @@ __global__ void __launch_bounds__(128) jk_kernel(const JkKernelArgs args) {
   const int lw = args.lwidth, W = 1 << lw, sub = lane & (W - 1), tpw = 32 >> lw;
   // (pp|pp) only: a task is shared by psplit consecutive warps, each summing
   // every psplit-th ket primitive and digesting its share (J and K are
-  // linear in the integrals); the other classes compile with a unit stride
+  // linear in the integrals); the other classes compile with constant strides
   constexpr bool kSplit = C::L == 4;
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int ps = kSplit ? args.psplit : 1, slice = kSplit ? gw % ps : 0;
+  const int ps = kSplit ? args.psplit : LPQ, slice = kSplit || LPQ > 1 ? gw % ps : 0;
+  // this lane's share of the primitive quartets
+  constexpr int KS = LPQ > 1 ? 4 : 1;
+  const int kq0 = LPQ > 1 ? lane % KS : (kSplit ? slice : 0), kqs = LPQ > 1 ? KS : (kSplit ? ps : 1);
+  const int kp0 = LPQ > 1 ? lane % LPQ / KS : 0, kps = LPQ / KS;
   for (int tb = (gw / ps) * tpw; tb < ntasks; tb += (nw / ps) * tpw) {
     const int tl = tb + (lane >> lw);
     const bool valid = tl < ntasks;
     const int t = args.task_begin + (valid ? tl : ntasks - 1);
     const int ib = find_bra(args.task_off, args.nbra, t);
-    const int ket = __ldg(args.ket_lo + ib) + (t - __ldg(args.task_off + ib)) * W + sub;
+    const int ket = __ldg(args.ket_lo + ib) + (t - __ldg(args.task_off + ib)) * W +
+                    (LPQ > 1 ? slice * (32 / LPQ) + lane / LPQ : sub);
     const int bp = args.bra_base + ib;
     const int kp = args.ket_base + ket;
     bool active = valid && ket < __ldg(args.ket_hi + ib);
@@ -464,7 +501,7 @@ __global__ void __launch_bounds__(128) jk_kernel(const JkKernelArgs args) {
         if (A.prim_thresh > 0.0) kcut = A.prim_thresh / fmax((double)dm, 1e-300);
       }
     }
-    const unsigned amask = __ballot_sync(0xffffffffu, active);
+    unsigned amask = __ballot_sync(0xffffffffu, active);
     if (amask == 0u) continue;
     // the bra's primitive records, read by every primitive of every lane of
     // the group: staged once per task into this warp's shared-memory area
@@ -488,19 +525,28 @@ __global__ void __launch_bounds__(128) jk_kernel(const JkKernelArgs args) {
       // FP32 quartets: two primitives per step in packed pairs, except
       // (pp|pp), whose 81 packed accumulators would not fit the registers
       if constexpr (sizeof(R) == 4 && C::L < 4)
-        nprim = contracted_quartet_f2<LA, LB, LC, LD>(args.primf, brec, bi0, ki0, bg, kg, out, kcut, slice, ps);
+        nprim = contracted_quartet_f2<LA, LB, LC, LD>(args.primf, brec, bi0, ki0, bg, kg, out, kcut, kq0, kqs, kp0, kps);
       else
-        nprim = contracted_quartet<R, LA, LB, LC, LD>(records<R>(args), brec, bi0, ki0, bg, kg, out, kcut, slice, ps);
+        nprim = contracted_quartet<R, LA, LB, LC, LD>(records<R>(args), brec, bi0, ki0, bg, kg, out, kcut, kq0, kqs, kp0,
+                                                      kps);
     } else {
 #pragma unroll
       for (int i = 0; i < C::NOUT; ++i) out[i] = (R)0;
+    }
+    if constexpr (LPQ > 1) {  // the quartet's first lane takes the sum and digests it
+#pragma unroll
+      for (int i = 0; i < C::NOUT; ++i)
+#pragma unroll
+        for (int o = LPQ / 2; o > 0; o >>= 1) out[i] += __shfl_xor_sync(0xffffffffu, out[i], o);
+      active = active && lane % LPQ == 0;
+      amask = __ballot_sync(0xffffffffu, active);
     }
     if (A.stats) {  // contracted and evaluated primitive quartets
       unsigned long long tot = (unsigned long long)nprim;
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
       if (lane == 0) {
-        if (slice == 0) atomicAdd(A.stats + args.prec * NQCLASS + args.qclass, (unsigned long long)__popc(amask));
+        if (slice == 0 || LPQ > 1) atomicAdd(A.stats + args.prec * NQCLASS + args.qclass, (unsigned long long)__popc(amask));
         atomicAdd(A.stats + (2 + args.prec) * NQCLASS + args.qclass, tot);
       }
     }
@@ -622,8 +668,15 @@ static int qclass_of(int bc, int kc) {
 
 template <typename R, int LA, int LB, int LC, int LD>
 static void jk_dispatch_nk(int nk, dim3 grid, dim3 block, size_t smem, cudaStream_t s, const JkKernelArgs& k) {
-  if (nk == 1) jk_kernel<R, LA, LB, LC, LD, 1><<<grid, block, smem, s>>>(k);
-  else jk_kernel<R, LA, LB, LC, LD, 2><<<grid, block, smem, s>>>(k);
+  constexpr int W4 = LA + LB + LC + LD == 4 ? 1 : 4, W16 = LA + LB + LC + LD == 4 ? 1 : 16;
+  auto launch = [&](auto lpq) {
+    constexpr int LPQ = decltype(lpq)::value;
+    if (nk == 1) jk_kernel<R, LA, LB, LC, LD, 1, LPQ><<<grid, block, smem, s>>>(k);
+    else jk_kernel<R, LA, LB, LC, LD, 2, LPQ><<<grid, block, smem, s>>>(k);
+  };
+  if (k.lpq == 16) launch(std::integral_constant<int, W16>());
+  else if (k.lpq == 4) launch(std::integral_constant<int, W4>());
+  else launch(std::integral_constant<int, 1>());
 }
 
 template <typename R>
@@ -681,8 +734,9 @@ void launch_jk(const PairData& pd, const TaskList& tl, int bc, int kc, bool fp32
   k.lwidth = width_log2(tl.width);
   const long long warps = (tl.ntasks + (32 / tl.width) - 1) / (32 / tl.width);
   k.psplit = k.qclass == NQCLASS - 1 ? primitive_split(warps, num_sms) : 1;
-  int nblk = grid_for((int)std::min<long long>(warps * k.psplit, 1LL << 30), num_sms);
-  nblk = (nblk + 1) / 2 * 2;
+  k.lpq = k.qclass < NQCLASS - 1 && tl.width == 32 ? lanes_per_quartet(warps, num_sms) : 1;
+  int nblk = grid_for((int)std::min<long long>(warps * k.psplit * k.lpq, 1LL << 30), num_sms);
+  nblk = (nblk + 3) / 4 * 4;  // whole groups of 8 or 16 warps
   dim3 grid(nblk), block(128);
   const size_t rec = fp32 ? sizeof(float4) : sizeof(double4);
   const int tpw = 32 / tl.width;
@@ -844,7 +898,10 @@ struct GradKernelArgs {
   int nbra, ntasks, bra_base, ket_base, same_class, qclass, task_begin;
   int lwidth;
   int smem_atoms;  // atoms summed in shared memory (0: global atomics)
-  int psplit;      // warps per task: warp k of a group takes ket primitives k, k + psplit, ...
+  // warps per task, psplit = slices of the ket primitives (psk) times slices
+  // of the bra primitives: slice s takes ket primitives s % psk, s % psk + psk,
+  // ... and bra primitives s / psk, ...
+  int psplit, psk;
   int stage;       // FP32: bra primitive records staged per task in shared memory (0: global)
   int stage_off;   // byte offset of the staging area in the dynamic shared memory
 };
@@ -875,6 +932,7 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
   // primitive quartets, so each warp adds its share with the same atomics)
   const int gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int ps = args.psplit, slice = gw % ps;
+  const int psk = args.psk, kq0 = slice % psk, kp0 = slice / psk, kps = ps / psk;
   for (int tb = (gw / ps) * tpw; tb < ntasks; tb += (nw / ps) * tpw) {
     const int tl = tb + (lane >> lw);
     const bool valid = tl < ntasks;
@@ -958,7 +1016,7 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
 #pragma unroll
         for (int i = 0; i < C::NGACC; ++i) acc[i] = (R)0;
 #pragma unroll 1
-        for (int kq = slice; kq < ki0.w; kq += ps) {
+        for (int kq = kq0; kq < ki0.w; kq += psk) {
           const V* kr = prim + 3 * (size_t)(ki0.z + kq);
           const V k0 = kr[0], k1 = kr[1], k2 = kr[2];
           const R kcd = fabs((R)k0.z);
@@ -966,7 +1024,7 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
           const R QC[3] = {(R)k2.x, (R)k2.y, (R)k2.z};
           const R tc = (R)(2 * k0.w);
 #pragma unroll 1
-          for (int kpp = 0; kpp < bi0.w; ++kpp) {
+          for (int kpp = kp0; kpp < bi0.w; kpp += kps) {
             const V* br = brec + 3 * kpp;
             const V b0 = br[0], b1 = br[1], b2 = br[2];
             if (fabs((R)b0.z) * kcd < cut) break;
@@ -992,14 +1050,14 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
         R* gam = kGamSmem ? reinterpret_cast<R*>(gsh + nsm) + (size_t)threadIdx.x * C::NOUT : gam_reg;
         fill_gam(gam);
 #pragma unroll 1
-        for (int kq = slice; kq < ki0.w; kq += ps) {
+        for (int kq = kq0; kq < ki0.w; kq += psk) {
           const V* kr = prim + 3 * (size_t)(ki0.z + kq);
           const V k0 = kr[0], k1 = kr[1], k2 = kr[2];
           const R kcd = fabs((R)k0.z);
           if (kab_max * kcd < cut) break;
           const R QC[3] = {(R)k2.x, (R)k2.y, (R)k2.z};
 #pragma unroll 1
-          for (int kpp = 0; kpp < bi0.w; ++kpp) {
+          for (int kpp = kp0; kpp < bi0.w; kpp += kps) {
             const V* br = brec + 3 * kpp;
             const V b0 = br[0], b1 = br[1], b2 = br[2];
             if (fabs((R)b0.z) * kcd < cut) break;
@@ -1104,9 +1162,14 @@ void launch_grad2e(const PairData& pd, const TaskList& tl, int bc, int kc, bool 
   k.stage = (fp32 && pd.class_maxprim[bc] > 0 && stage_bytes <= JK_STAGE_MAX_BYTES) ? pd.class_maxprim[bc] : 0;
   const size_t smem = k.stage ? (size_t)k.stage_off + stage_bytes : base;
   const long long warps = (tl.ntasks + tpw - 1) / tpw;
-  k.psplit = primitive_split(warps, num_sms);
+  // very short lists split the bra primitives too (water: (pp|pp), one warp of
+  // 81 derivative quartets, 480 us; the gradient's atomics are few)
+  int pb = 1;
+  k.psk = primitive_split(warps, num_sms);
+  while (k.psk == 8 && pb < 8 && 2 * pb <= pd.class_maxprim[bc] && warps * 8 * pb < (long long)num_sms * 8) pb *= 2;
+  k.psplit = k.psk * pb;
   int nblk = grid_for((int)std::min<long long>(warps * k.psplit, 1LL << 30), num_sms);
-  nblk = (nblk + 1) / 2 * 2;
+  nblk = (nblk + 15) / 16 * 16;  // whole groups of up to 64 warps
   dim3 grid(nblk), block(128);
   if (fp32) grad2e_dispatch<float>(k.qclass, grid, block, smem, s, k);
   else grad2e_dispatch<double>(k.qclass, grid, block, smem, s, k);

@@ -62,7 +62,8 @@ template <int L> struct NC { static constexpr int v = (L + 1) * (L + 2) / 2; };
 // Primitive pairs are stored in order of decreasing |K|, so with kcut > 0
 // both loops stop at the first primitive quartet with |K_ab K_cd| < kcut.
 // With kq_step > 1 only the ket primitives kq0, kq0 + kq_step, ... are
-// summed (a share of the quartet; the shares add up to the integral).
+// summed, and of the bra's only kp0, kp0 + kp_step, ... (a share of the
+// quartet; the shares add up to the integral).
 // brec: the bra pair's first primitive record (in global memory, or the
 // copy a warp staged in shared memory); prim: all records (the kets').
 template <typename R, int LA, int LB, int LC, int LD>
@@ -70,7 +71,7 @@ __device__ __forceinline__ int contracted_quartet(const typename Rec<R>::T* __re
                                                   const typename Rec<R>::T* brec, int4 bi0, int4 ki0,
                                                   const double4& bgeo, const double4& kgeo,
                                                   R out[EriClass<R, LA, LB, LC, LD>::NOUT], double kcut = 0.0,
-                                                  int kq0 = 0, int kq_step = 1) {
+                                                  int kq0 = 0, int kq_step = 1, int kp0 = 0, int kp_step = 1) {
   using C = EriClass<R, LA, LB, LC, LD>;
   using V = typename Rec<R>::T;
   R acc[C::NACC];
@@ -88,7 +89,7 @@ __device__ __forceinline__ int contracted_quartet(const typename Rec<R>::T* __re
     if (kab_max * kcd < cut) break;
     const R QC[3] = {(R)k2.x, (R)k2.y, (R)k2.z};
 #pragma unroll 1
-    for (int kp = 0; kp < bi0.w; ++kp) {
+    for (int kp = kp0; kp < bi0.w; kp += kp_step) {
       const V* br = brec + 3 * kp;
       const V b0 = br[0], b1 = br[1], b2 = br[2];
       if (fabs((R)b0.z) * kcd < cut) break;
@@ -143,7 +144,8 @@ template <int LA, int LB, int LC, int LD>
 __device__ __forceinline__ int contracted_quartet_f2(const float4* __restrict__ prim, const float4* brec, int4 bi0,
                                                      int4 ki0, const double4& bgeo, const double4& kgeo,
                                                      float out[EriClass<float, LA, LB, LC, LD>::NOUT],
-                                                     double kcut = 0.0, int kq0 = 0, int kq_step = 1) {
+                                                     double kcut = 0.0, int kq0 = 0, int kq_step = 1, int kp0 = 0,
+                                                     int kp_step = 1) {
   using C2 = EriClass<F2, LA, LB, LC, LD>;
   using C1 = EriClass<float, LA, LB, LC, LD>;
   F2 acc[C2::NACC];
@@ -159,7 +161,7 @@ __device__ __forceinline__ int contracted_quartet_f2(const float4* __restrict__ 
     if (kab_max * kcd < cut) break;
     const F2 QC[3] = {F2(k2.x), F2(k2.y), F2(k2.z)};
 #pragma unroll 1
-    for (int kp = 0; kp < bi0.w; kp += 2) {
+    for (int kp = 2 * kp0; kp < bi0.w; kp += 2 * kp_step) {
       const float4* br = brec + 3 * kp;
       const float4 b0 = br[0], b1 = br[1], b2 = br[2];
       if (fabsf(b0.z) * kcd < cut) break;
