@@ -25,6 +25,7 @@
 #include "f2.cuh"
 
 #define PF_BOYS_NGRID 361
+#define PF_BOYS_NGRID_PAD 364  // multiple of 4: the float4 groups stay aligned
 #define PF_BOYS_STEP 0.1
 #define PF_BOYS_INV_STEP 10.0
 #define PF_BOYS_TMAX 36.0
@@ -40,11 +41,15 @@ namespace pyfacc {
 // Grid tables, one copy per translation unit that includes this header
 // (kernels.cu and kernels_d.cu; each fills its copy per device with
 // cudaMemcpyToSymbol, see ensure_boys_tables):
-// g_boys_tl[L][k][j] = F_{L+j}(T_k) / j!, g_boys_exp[k] = e^{-T_k},
-// g_boys_tlf[L][k][j] = F_{L+j}(T_k) / j! in float (j < 5 used).
+// g_boys_tl[L][j / 2][k][j % 2] = F_{L+j}(T_k) / j!, g_boys_exp[k] = e^{-T_k},
+// g_boys_tlf[L][0][k][j] the same in float for j < 4, then [k] for j = 4.
+// Coefficients are grouped over the grid, not by grid point: the lanes of a
+// quarter warp then read 16-byte words at random multiples of 16 bytes, over
+// all eight bank groups (2.6 wavefronts on average), where rows of 64 bytes
+// left them two groups (5.1).
 static __device__ __align__(16) double g_boys_tl[(PF_BOYS_MMAX + 1) * PF_BOYS_NGRID * PF_BOYS_NT];
 static __device__ double g_boys_exp[PF_BOYS_NEXP];
-static __device__ __align__(16) float g_boys_tlf[(PF_BOYS_MMAX + 1) * PF_BOYS_NGRID * PF_BOYS_NT];
+static __device__ __align__(16) float g_boys_tlf[(PF_BOYS_MMAX + 1) * PF_BOYS_NGRID_PAD * PF_BOYS_NTF];
 
 // Branch-free: every lane evaluates the Taylor value (from row 0 when T is
 // beyond the grid) and the asymptotic value and selects, so a warp whose
@@ -60,8 +65,9 @@ __device__ __forceinline__ void boys_fp64(double T, double* __restrict__ F) {
   const double kd = biased - 6755399441055744.0;
   const int k = tab ? ke : 0;
   const double x = kd * PF_BOYS_STEP - T;  // F_L(T) = sum_j F_{L+j}(T_k) x^j / j! (T < 36)
-  const double2* row = reinterpret_cast<const double2*>(g_boys_tl + ((size_t)L * PF_BOYS_NGRID + k) * PF_BOYS_NT);
-  const double2 c01 = __ldg(row), c23 = __ldg(row + 1), c45 = __ldg(row + 2), c67 = __ldg(row + 3);
+  const double2* row = reinterpret_cast<const double2*>(g_boys_tl) + (size_t)L * PF_BOYS_NGRID * (PF_BOYS_NT / 2) + k;
+  const double2 c01 = __ldg(row), c23 = __ldg(row + PF_BOYS_NGRID), c45 = __ldg(row + 2 * PF_BOYS_NGRID),
+                c67 = __ldg(row + 3 * PF_BOYS_NGRID);
   double f = fma(c67.y, x, c67.x);
   f = fma(f, x, c45.y);
   f = fma(f, x, c45.x);
@@ -97,28 +103,29 @@ __device__ __forceinline__ void boys_fp64(double T, double* __restrict__ F) {
 
 template <int L>
 __device__ __forceinline__ void boys_fp32(float T, float* __restrict__ F) {
-  const bool tab = T < (float)PF_BOYS_TMAX;
+  const bool near = T < (float)PF_BOYS_TMAX;
   // nearest grid point by adding and subtracting 1.5 * 2^23 (see boys_fp64)
   const float biased = fminf(T, (float)PF_BOYS_TMAX) * (float)PF_BOYS_INV_STEP + 12582912.0f;
-  const int k = tab ? (__float_as_int(biased) & 0x7fffff) - 0x400000 : 0;
+  const int k = near ? (__float_as_int(biased) & 0x7fffff) - 0x400000 : 0;
   const float x = (biased - 12582912.0f) * (float)PF_BOYS_STEP - T;
-  const float4* row = reinterpret_cast<const float4*>(g_boys_tlf + ((size_t)L * PF_BOYS_NGRID + k) * PF_BOYS_NT);
-  const float4 c0 = __ldg(row), c1 = __ldg(row + 1);
-  float f = fmaf(c1.x, x, c0.w);  // 5 terms: F_{L+j}(T_k) / j!, j = 4 .. 0
+  const float* tab = g_boys_tlf + (size_t)L * PF_BOYS_NGRID_PAD * PF_BOYS_NTF;
+  const float4 c0 = __ldg(reinterpret_cast<const float4*>(tab) + k);
+  const float c4 = __ldg(tab + 4 * PF_BOYS_NGRID_PAD + k);
+  float f = fmaf(c4, x, c0.w);  // 5 terms: F_{L+j}(T_k) / j!, j = 4 .. 0
   f = fmaf(f, x, c0.z);
   f = fmaf(f, x, c0.y);
   f = fmaf(f, x, c0.x);
   const float rt = rsqrtf(fmaxf(T, (float)PF_BOYS_TMAX));
   float fa = 0.88622692545275801365f * rt;
   if (L == 0) {
-    F[0] = tab ? f : fa;
+    F[0] = near ? f : fa;
     return;
   }
   const float e = expf(-T);
   const float o2t = 0.5f * rt * rt;
 #pragma unroll
   for (int m = 0; m < L; ++m) fa = ((2 * m + 1) * fa - e) * o2t;
-  F[L] = tab ? f : fa;
+  F[L] = near ? f : fa;
   const float t2 = 2.0f * T;
 #pragma unroll
   for (int m = L - 1; m >= 0; --m) F[m] = (t2 * F[m + 1] + e) * (1.0f / (2 * m + 1));
@@ -139,10 +146,10 @@ __device__ __forceinline__ void boys_fp32x2(F2 T, F2* __restrict__ F) {
   const int ky = taby ? (__float_as_int(biased.v.y) & 0x7fffff) - 0x400000 : 0;
   const F2 kd = biased + F2(-12582912.0f);
   const F2 x = pf_fma(kd, F2((float)PF_BOYS_STEP), T * F2(-1.0f));
-  const float4* rx = reinterpret_cast<const float4*>(g_boys_tlf + ((size_t)L * PF_BOYS_NGRID + kx) * PF_BOYS_NT);
-  const float4* ry = reinterpret_cast<const float4*>(g_boys_tlf + ((size_t)L * PF_BOYS_NGRID + ky) * PF_BOYS_NT);
-  const float4 x0 = __ldg(rx), x1 = __ldg(rx + 1), y0 = __ldg(ry), y1 = __ldg(ry + 1);
-  F2 f = pf_fma(F2(x1.x, y1.x), x, F2(x0.w, y0.w));
+  const float* tab = g_boys_tlf + (size_t)L * PF_BOYS_NGRID_PAD * PF_BOYS_NTF;
+  const float4 x0 = __ldg(reinterpret_cast<const float4*>(tab) + kx), y0 = __ldg(reinterpret_cast<const float4*>(tab) + ky);
+  const float x4 = __ldg(tab + 4 * PF_BOYS_NGRID_PAD + kx), y4 = __ldg(tab + 4 * PF_BOYS_NGRID_PAD + ky);
+  F2 f = pf_fma(F2(x4, y4), x, F2(x0.w, y0.w));
   f = pf_fma(f, x, F2(x0.z, y0.z));
   f = pf_fma(f, x, F2(x0.y, y0.y));
   f = pf_fma(f, x, F2(x0.x, y0.x));

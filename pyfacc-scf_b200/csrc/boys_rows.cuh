@@ -1,9 +1,9 @@
 // Boys function from a short table in shared memory, for the split kernels.
 //
-// boys_fp64's 64-byte rows (boys.cuh) are gathered with four 16-byte loads;
-// a 64-byte stride puts the lanes of a quarter warp on two bank groups, so
-// each load took 16-20 wavefronts of the L1 data stage and the (ss|ss) kernel
-// spent 54 of its 63 wavefronts per primitive quartet there.  Here F_L(T) on
+// boys_fp64 (boys.cuh) gathers four 16-byte pairs per lane from global memory,
+// 2.6 wavefronts a quarter warp each (from rows of 64 bytes, as they were when
+// this table was made, 5; the (ss|ss) kernel then spent 54 of its 63
+// wavefronts per primitive quartet there).  Here F_L(T) on
 // [0, 31.5 h) is one of 32 polynomials about T = k h, stored coefficient by
 // coefficient, 32 words in 32 banks: a 4-byte load is conflict-free whatever
 // rows the lanes want (one wavefront; an FP64 coefficient takes two, high and

@@ -54,18 +54,21 @@ void ensure_boys_tables(int device) {
     for (int k = 0; k < PF_BOYS_NGRID; ++k)
       for (int m = 0; m < PF_BOYS_NCOL; ++m) F[(size_t)k * PF_BOYS_NCOL + m] = boys_series_ld(m, (long double)k * 0.1L);
     tl.resize((size_t)(PF_BOYS_MMAX + 1) * PF_BOYS_NGRID * PF_BOYS_NT);
+    tabf.resize((size_t)(PF_BOYS_MMAX + 1) * PF_BOYS_NGRID_PAD * PF_BOYS_NTF);
     for (int L = 0; L <= PF_BOYS_MMAX; ++L)
       for (int k = 0; k < PF_BOYS_NGRID; ++k) {
         long double fact = 1.0L;
         for (int j = 0; j < PF_BOYS_NT; ++j) {
           if (j > 0) fact *= j;
-          tl[((size_t)L * PF_BOYS_NGRID + k) * PF_BOYS_NT + j] = (double)(F[(size_t)k * PF_BOYS_NCOL + L + j] / fact);
+          const double c = (double)(F[(size_t)k * PF_BOYS_NCOL + L + j] / fact);
+          tl[(((size_t)L * (PF_BOYS_NT / 2) + j / 2) * PF_BOYS_NGRID + k) * 2 + j % 2] = c;
+          float* f = tabf.data() + (size_t)L * PF_BOYS_NGRID_PAD * PF_BOYS_NTF;
+          if (j < 4) f[4 * k + j] = (float)c;
+          else if (j == 4) f[4 * PF_BOYS_NGRID_PAD + k] = (float)c;
         }
       }
     ex.resize(PF_BOYS_NEXP);
     for (int k = 0; k < PF_BOYS_NEXP; ++k) ex[k] = (double)expl(-(long double)k * 0.1L);
-    tabf.resize(tl.size());
-    for (size_t i = 0; i < tl.size(); ++i) tabf[i] = (float)tl[i];
   }
   if ((int)done.size() <= device) done.resize(device + 1, 0);
   if (!done[device]) {
