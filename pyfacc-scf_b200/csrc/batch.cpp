@@ -620,7 +620,7 @@ void Batch::alloc() {
                                                     offsetof(StepReport, max_err));
   a.built_full = 1;
   a.coarse = 0;
-  a.smem_nmax = nbf_max;  // nbf <= 160: at most 200 KB of shared memory
+  a.smem_nmax = nbf_max;  // nbf <= 160: at most 205 KB of shared memory
   batch_set_smem(a);
   PF_CUDA(cudaStreamSynchronize(stream));
 }

@@ -14,6 +14,7 @@
 // from a coupled Newton-Schulz iteration, so no eigensolver is needed).
 #include <cuda_runtime.h>
 
+#include <climits>
 #include <cmath>
 
 #include "batch.h"
@@ -26,92 +27,131 @@ __device__ __forceinline__ double red_op(double a, double b, bool mx) { return m
 
 // Block-wide sum (mx = false) or maximum; every thread receives the result.
 __device__ double blk_reduce(double v, bool mx) {
-  __shared__ double red[33];
+  __shared__ double red[32];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = red_op(v, __shfl_xor_sync(0xffffffffu, v, o), mx);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
   if (l == 0) red[w] = v;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    double r = red[0];
-    for (int k = 1; k < (int)(blockDim.x >> 5); ++k) r = red_op(r, red[k], mx);
-    red[32] = r;
-  }
-  __syncthreads();
-  const double r = red[32];
+  double r = red[l < nw ? l : 0];
+  if (l >= nw && !mx) r = 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) r = red_op(r, __shfl_xor_sync(0xffffffffu, r, o), mx);
   __syncthreads();
   return r;
 }
 
-// C = alpha A B (+ beta C) for n x n row-major matrices with leading
-// dimension n, on the FP64 tensor cores: each warp owns 8 x 8 output tiles
-// and runs mma.sync.m8n8k4 (f64) over k in steps of 4; elements beyond n
-// are read as zero and not written.  A, B, C may be global or shared; C
-// must not alias A or B.  Ends with a block barrier.
+__device__ __forceinline__ void mma_f64(double& d0, double& d1, double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+               : "+d"(d0), "+d"(d1)
+               : "d"(a), "d"(b));
+}
+
+// The t-th 16 x 16 tile of the upper triangle of nm x nm tiles.
+__device__ __forceinline__ void upper_tile(int t, int nm, int& ti, int& tj) {
+  ti = 0;
+  while (t >= nm - ti) t -= nm - ti++;
+  tj = ti + t;
+}
+
+// C = alpha A B for n x n matrices with rows lda, ldb, ldc apart, on the FP64
+// tensor cores: a warp owns 16 x 16 output tiles, four m8n8k4 products per
+// two fragments of A and two of B.  The kernel is bound by the fragments'
+// loads (L1 tag lookups: a fragment of four rows of 64 bytes takes four, one
+// of eight rows of 32 bytes eight) where the 8 x 8 tiles it had before paid
+// two fragments per product: 3.9 -> 0.80 ms a step for 256 molecules of 28 to
+// 112 functions together with the purification below, 2.5 -> 0.54 ms for 64.  Hence AT: A is given
+// transposed (a symmetric A is its own transpose; TS stores a result that is
+// the next product's A).  SYM = 1 or -1: the result is symmetric or
+// antisymmetric, only its upper triangle is computed.  A, B, C may be global
+// or shared; C must not alias A or B.  Ends with a block barrier.
 //
 // Fragments of m8n8k4 (f64, row.col): lane l holds A[l/4][l%4],
 // B[l%4][l/4] and C[l/4][2(l%4)], C[l/4][2(l%4)+1].
-__device__ void bgemm(int n, const double* A, const double* B, double* C, double alpha, double beta) {
+template <bool AT, int SYM, bool TS>
+__device__ void bgemm(int n, const double* A, int lda, const double* B, int ldb, double* C, int ldc, double alpha) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
-  const int nt = (n + 7) >> 3;
-  for (int tile = warp; tile < nt * nt; tile += nwarp) {
-    const int i0 = (tile / nt) << 3, j0 = (tile % nt) << 3;
-    const int ra = i0 + g;          // row of A this lane reads
-    const int cb = j0 + g;          // column of B this lane reads
-    // two accumulator chains (even and odd k-steps) so that consecutive
-    // MMAs do not wait on each other
-    double d0 = 0.0, d1 = 0.0, e0 = 0.0, e1 = 0.0;
-    for (int k0 = 0; k0 < n; k0 += 8) {
-      const int ka = k0 + t, kb = k0 + 4 + t;
-      const double a = (ra < n && ka < n) ? A[(size_t)ra * n + ka] : 0.0;
-      const double b = (ka < n && cb < n) ? B[(size_t)ka * n + cb] : 0.0;
-      const double a2 = (ra < n && kb < n) ? A[(size_t)ra * n + kb] : 0.0;
-      const double b2 = (kb < n && cb < n) ? B[(size_t)kb * n + cb] : 0.0;
-      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                   : "+d"(d0), "+d"(d1)
-                   : "d"(a), "d"(b));
-      asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                   : "+d"(e0), "+d"(e1)
-                   : "d"(a2), "d"(b2));
+  const int nm = (n + 15) >> 4, ntile = SYM ? nm * (nm + 1) / 2 : nm * nm;
+  for (int tile = warp; tile < ntile; tile += nwarp) {
+    int ti = tile / nm, tj = tile - ti * nm;
+    if (SYM) upper_tile(tile, nm, ti, tj);
+    const int i0 = ti << 4, j0 = tj << 4;
+    // rows of A and columns of B beyond n repeat the last one; their results
+    // are not stored
+    const int ia0 = min(i0 + g, n - 1), ia1 = min(i0 + 8 + g, n - 1);
+    const int jb0 = min(j0 + g, n - 1), jb1 = min(j0 + 8 + g, n - 1);
+    const double* pa0 = A + (AT ? (size_t)t * lda + ia0 : (size_t)ia0 * lda + t);
+    const double* pa1 = A + (AT ? (size_t)t * lda + ia1 : (size_t)ia1 * lda + t);
+    const double* pb0 = B + (size_t)t * ldb + jb0;
+    const double* pb1 = B + (size_t)t * ldb + jb1;
+    const int sa = AT ? 4 * lda : 4, sb = 4 * ldb;
+    double acc[2][2][2] = {};
+    auto step = [&](double a0, double a1, double b0, double b1) {
+      mma_f64(acc[0][0][0], acc[0][0][1], a0, b0);
+      mma_f64(acc[0][1][0], acc[0][1][1], a0, b1);
+      mma_f64(acc[1][0][0], acc[1][0][1], a1, b0);
+      mma_f64(acc[1][1][0], acc[1][1][1], a1, b1);
+    };
+    int k = 0;
+#pragma unroll 4
+    for (; k + 4 <= n; k += 4) {
+      step(*pa0, *pa1, *pb0, *pb1);
+      pa0 += sa; pa1 += sa; pb0 += sb; pb1 += sb;
     }
-    d0 += e0;
-    d1 += e1;
-    const int r = i0 + g, c = j0 + 2 * t;
-    if (r < n) {
-      if (c < n) {
-        const size_t q = (size_t)r * n + c;
-        C[q] = (beta == 0.0) ? alpha * d0 : alpha * d0 + beta * C[q];
-      }
-      if (c + 1 < n) {
-        const size_t q = (size_t)r * n + c + 1;
-        C[q] = (beta == 0.0) ? alpha * d1 : alpha * d1 + beta * C[q];
-      }
+    if (k < n) {  // the last one to three k
+      const bool in = k + t < n;
+      step(in ? *pa0 : 0.0, in ? *pa1 : 0.0, in ? *pb0 : 0.0, in ? *pb1 : 0.0);
     }
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int row = i0 + 8 * r + g, col = j0 + 8 * c + 2 * t + h;
+          if (row >= n || col >= n || (SYM && row > col)) continue;
+          const double v = SYM < 0 && row == col ? 0.0 : alpha * acc[r][c][h];
+          C[TS ? (size_t)col * ldc + row : (size_t)row * ldc + col] = v;
+          if (SYM && row != col) C[(size_t)col * ldc + row] = SYM > 0 ? v : -v;
+        }
   }
   __syncthreads();
 }
 
+// Rows of the shared-memory matrix: whole 16 x 16 tiles, 4 bank pairs apart
+// (the eight rows of a fragment, four words each, then meet no bank twice).
+__host__ __device__ constexpr int xs_rows(int n) { return (n + 15) & ~15; }
+__host__ __device__ constexpr int xs_ld(int n) { return xs_rows(n) + 4; }
+
 // TC2 purification (Niklasson 2002) of the orthogonalised Fock matrix Fp:
-// Xs <- projector onto the nocc lowest eigenvectors.  X2 is n x n work
-// space.  The step choice and the stopping rule are those of the
-// single-molecule kernels (Tr X - Tr X^2 < 1e-9 at the right trace, then two
-// more steps).  Returns the steps taken, or -1 without convergence.
-__device__ int tc2(int n, int nocc, const double* Fp, double* Xs, double* X2) {
-  const int n2 = n * n;
+// xs (shared memory, rows xs_ld(n) apart) <- projector onto the nocc lowest
+// eigenvectors.  The iterate stays in xs, zero-padded to whole tiles; X^2 of
+// the upper triangle's tiles is accumulated in registers, up to TC2_TILES per
+// warp, and xs is updated in place behind a barrier, with both triangles
+// stored (X^T = X: the fragments of B are rows as well) and Tr X and Tr X^2
+// (the square sum) taken along.  The step choice and the stopping rule are
+// those of the single-molecule kernels (Tr X - Tr X^2 < 1e-9 at the right
+// trace, then two more steps).  Returns the steps taken, or -1 without
+// convergence.
+constexpr int TC2_TILES = 4;  // 55 tiles at n = 160 (BATCH_NBF_MAX) on 16 warps
+__device__ int tc2(int n, int nocc, const double* Fp, double* xs) {
+  __shared__ double red[2][32];
+  const int np = xs_rows(n), ld = xs_ld(n);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (nocc <= 0 || nocc >= n) {
-    for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-      const int i = idx / n, j = idx - (idx / n) * n;
-      Xs[idx] = (nocc > 0 && i == j) ? 1.0 : 0.0;
-    }
+    for (int i = warp; i < n; i += nw)
+      for (int j = lane; j < n; j += 32) xs[i * ld + j] = (nocc > 0 && i == j) ? 1.0 : 0.0;
     __syncthreads();
     return 0;
   }
   double lo = 1e300, hi = -1e300;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+  for (int i = warp; i < n; i += nw) {
     double r = 0.0;
-    for (int j = 0; j < n; ++j)
+    for (int j = lane; j < n; j += 32)
       if (j != i) r += fabs(Fp[(size_t)i * n + j]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
     const double d = Fp[(size_t)i * n + i];
     lo = fmin(lo, d - r);
     hi = fmax(hi, d + r);
@@ -119,21 +159,48 @@ __device__ int tc2(int n, int nocc, const double* Fp, double* Xs, double* X2) {
   lo = -blk_reduce(-lo, true);
   hi = blk_reduce(hi, true);
   const double sc = 1.0 / fmax(hi - lo, 1e-300);
-  for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-    const int i = idx / n, j = idx - (idx / n) * n;
-    Xs[idx] = ((i == j ? hi : 0.0) - Fp[idx]) * sc;
+  double t1 = 0.0, t2 = 0.0;
+  for (int i = warp; i < np; i += nw)
+    for (int j = lane; j < np; j += 32) {
+      double v = 0.0;
+      if (i < n && j < n) v = ((i == j ? hi : 0.0) - Fp[(size_t)i * n + j]) * sc;
+      if (i == j) t1 += v;
+      t2 += v * v;
+      xs[i * ld + j] = v;
+    }
+  t1 = blk_reduce(t1, false);
+  t2 = blk_reduce(t2, false);
+  const int g = lane >> 2, t = lane & 3;
+  const int nm = np >> 4, ntile = nm * (nm + 1) / 2;
+  int tij[TC2_TILES], mine = 0;
+#pragma unroll
+  for (int u = 0; u < TC2_TILES; ++u) {
+    int ti = 0, tj = 0;
+    if (warp + u * nw < ntile) {
+      upper_tile(warp + u * nw, nm, ti, tj);
+      mine = u + 1;
+    }
+    tij[u] = ti << 20 | tj << 4;
   }
-  __syncthreads();
   int countdown = 0;
   for (int k = 0; k < 200; ++k) {
-    bgemm(n, Xs, Xs, X2, 1.0, 0.0);
-    double t1 = 0.0, t2 = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      t1 += Xs[(size_t)i * n + i];
-      t2 += X2[(size_t)i * n + i];
+    double acc[TC2_TILES][2][2][2];
+#pragma unroll
+    for (int u = 0; u < TC2_TILES; ++u) {
+      if (u >= mine) break;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) acc[u][q >> 2][(q >> 1) & 1][q & 1] = 0.0;
+      const double* pa = xs + ((tij[u] >> 16) + g) * ld + t;
+      const double* pb = xs + ((tij[u] & 0xffff) + g) * ld + t;
+#pragma unroll 2
+      for (int kk = 0; kk < n; kk += 4) {
+        const double a0 = pa[kk], a1 = pa[kk + 8 * ld], b0 = pb[kk], b1 = pb[kk + 8 * ld];
+        mma_f64(acc[u][0][0][0], acc[u][0][0][1], a0, b0);
+        mma_f64(acc[u][0][1][0], acc[u][0][1][1], a0, b1);
+        mma_f64(acc[u][1][0][0], acc[u][1][0][1], a1, b0);
+        mma_f64(acc[u][1][1][0], acc[u][1][1][1], a1, b1);
+      }
     }
-    t1 = blk_reduce(t1, false);
-    t2 = blk_reduce(t2, false);
     bool finish = false;
     if (countdown > 0) {
       if (--countdown == 0) finish = true;
@@ -143,54 +210,105 @@ __device__ int tc2(int n, int nocc, const double* Fp, double* Xs, double* X2) {
     // X <- X^2 takes the trace to t2, X <- 2X - X^2 to 2 t1 - t2
     double a = 2.0, b = -1.0;
     if (fabs(t2 - nocc) < fabs(2.0 * t1 - t2 - nocc)) { a = 0.0; b = 1.0; }
-    for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) Xs[idx] = a * Xs[idx] + b * X2[idx];
+    __syncthreads();  // every product has been read
+    double s1 = 0.0, s2 = 0.0;
+#pragma unroll
+    for (int u = 0; u < TC2_TILES; ++u) {
+      if (u >= mine) break;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int row = (tij[u] >> 16) + 8 * (q >> 2) + g, col = (tij[u] & 0xffff) + 8 * ((q >> 1) & 1) + 2 * t + (q & 1);
+        if (row > col) continue;
+        const double v = a * xs[row * ld + col] + b * acc[u][q >> 2][(q >> 1) & 1][q & 1];
+        xs[row * ld + col] = v;
+        xs[col * ld + row] = v;
+        if (row == col) s1 += v;
+        s2 += row == col ? v * v : 2.0 * v * v;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+      s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+    }
+    if (lane == 0) {
+      red[0][warp] = s1;
+      red[1][warp] = s2;
+    }
     __syncthreads();
     if (finish) return k + 1;
+    t1 = lane < nw ? red[0][lane] : 0.0;
+    t2 = lane < nw ? red[1][lane] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+      t2 += __shfl_xor_sync(0xffffffffu, t2, o);
+    }
   }
   return -1;
 }
 
-// Pulay DIIS solve: B c = 0 with sum c = 1 over the slots in use (m <= 8),
-// Gaussian elimination with partial pivoting on the bordered system.
-__device__ bool diis_solve(int m, const double* B, double* c) {
-  double A[(BATCH_DIIS_MAX + 1) * (BATCH_DIIS_MAX + 1)], b[BATCH_DIIS_MAX + 1];
-  const int q = m + 1;
-  double scl = 0.0;
-  for (int i = 0; i < m; ++i) scl = fmax(scl, fabs(B[i * m + i]));
+// Pulay DIIS solve: B c = 0 with sum c = 1 over the m <= 8 slots in use,
+// Gaussian elimination with partial pivoting on the bordered system.  One
+// warp, lane r holds row r and the right-hand side; returns c_r in lane r and
+// whether the system was solvable.
+__device__ bool diis_solve(int m, const double* B, int ldb, const int* use, double& c) {
+  constexpr int Q = BATCH_DIIS_MAX + 1;
+  const unsigned ALL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, q = m + 1;
+  double scl = lane < m ? fabs(B[use[lane] * ldb + use[lane]]) : 0.0;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) scl = fmax(scl, __shfl_xor_sync(ALL, scl, o));
   scl = scl > 0.0 ? 1.0 / scl : 1.0;
-  for (int i = 0; i < q; ++i) {
-    for (int j = 0; j < q; ++j) A[i * q + j] = (i < m && j < m) ? B[i * m + j] * scl : ((i == m && j == m) ? 0.0 : -1.0);
-    b[i] = (i == m) ? -1.0 : 0.0;
+  double A[Q], b = lane == m ? -1.0 : 0.0;
+#pragma unroll
+  for (int j = 0; j < Q; ++j) {
+    A[j] = 0.0;
+    if (lane < m && j < m) A[j] = B[use[lane] * ldb + use[j]] * scl;
+    else if (lane < q && j < q && lane != j) A[j] = -1.0;
   }
-  for (int col = 0; col < q; ++col) {
-    int piv = col;
-    for (int r = col + 1; r < q; ++r)
-      if (fabs(A[r * q + col]) > fabs(A[piv * q + col])) piv = r;
-    if (fabs(A[piv * q + col]) < 1e-300) return false;
-    if (piv != col) {
-      for (int k = 0; k < q; ++k) {
-        const double t = A[col * q + k];
-        A[col * q + k] = A[piv * q + k];
-        A[piv * q + k] = t;
+  bool ok = true;
+#pragma unroll
+  for (int col = 0; col < Q; ++col) {
+    if (col >= q) break;
+    // the largest of column col at or below the diagonal, the first of equals
+    double v = lane >= col && lane < q ? fabs(A[col]) : -1.0;
+    int piv = lane;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double ov = __shfl_xor_sync(ALL, v, o);
+      const int op = __shfl_xor_sync(ALL, piv, o);
+      if (ov > v || (ov == v && op < piv)) {
+        v = ov;
+        piv = op;
       }
-      const double t = b[col];
-      b[col] = b[piv];
-      b[piv] = t;
     }
-    for (int r = col + 1; r < q; ++r) {
-      const double f = A[r * q + col] / A[col * q + col];
-      for (int k = col; k < q; ++k) A[r * q + k] -= f * A[col * q + k];
-      b[r] -= f * b[col];
+    piv = __shfl_sync(ALL, piv, 0);
+    const int from = lane == col ? piv : (lane == piv ? col : lane);
+    double f = 0.0;
+#pragma unroll
+    for (int k = 0; k < Q; ++k) {
+      A[k] = __shfl_sync(ALL, A[k], from);
+      if (k < col) continue;
+      const double p = __shfl_sync(ALL, A[k], col);
+      if (k == col) {
+        ok = ok && !(fabs(p) < 1e-300);
+        f = lane > col ? A[k] / p : 0.0;
+      }
+      A[k] -= f * p;
     }
+    b = __shfl_sync(ALL, b, from);
+    b -= f * __shfl_sync(ALL, b, col);
   }
-  for (int r = q - 1; r >= 0; --r) {
-    double s = b[r];
-    for (int k = r + 1; k < q; ++k) s -= A[r * q + k] * c[k];
-    c[r] = s / A[r * q + r];
+  c = 0.0;
+#pragma unroll
+  for (int r = Q - 1; r >= 0; --r) {
+    if (r >= q) continue;
+    const double x = __shfl_sync(ALL, b / A[r], r);
+    if (lane == r) c = x;
+    if (lane < r) b -= A[r] * x;
   }
-  for (int i = 0; i < m; ++i)
-    if (!isfinite(c[i])) return false;
-  return true;
+  return __all_sync(ALL, ok && (lane >= m || isfinite(c)));
 }
 
 struct MolPtrs {
@@ -212,13 +330,14 @@ __device__ __forceinline__ MolPtrs mol_ptrs(const BatchDenseArgs& a, const Batch
 
 // P = 2 X P' X of the TC2 projector of F' = X Fsrc X; T1 and T3 are
 // overwritten, the result goes to out.  Returns the TC2 steps or -1.
-__device__ int density_from_fock(const MolPtrs& p, int nocc, const double* Fsrc, double* Xs, double* out) {
-  bgemm(p.n, p.X, Fsrc, p.T3, 1.0, 0.0);
-  bgemm(p.n, p.T3, p.X, p.T1, 1.0, 0.0);
-  const int steps = tc2(p.n, nocc, p.T1, Xs, p.T3);
+__device__ int density_from_fock(const MolPtrs& p, int nocc, const double* Fsrc, double* xs, double* out) {
+  const int n = p.n;
+  bgemm<true, 0, true>(n, p.X, n, Fsrc, n, p.T3, n, 1.0);  // (X F)^T
+  bgemm<true, 1, false>(n, p.T3, n, p.X, n, p.T1, n, 1.0);
+  const int steps = tc2(n, nocc, p.T1, xs);
   if (steps < 0) return -1;
-  bgemm(p.n, p.X, Xs, p.T1, 1.0, 0.0);
-  bgemm(p.n, p.T1, p.X, out, 2.0, 0.0);
+  bgemm<true, 0, true>(n, p.X, n, xs, xs_ld(n), p.T3, n, 1.0);  // (X P')^T
+  bgemm<true, 1, false>(n, p.T3, n, p.X, n, out, n, 2.0);
   return steps;
 }
 
@@ -254,7 +373,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_lowdin_kernel(const Batch
   __syncthreads();
   bool ok = false;
   for (int it = 0; it < 100; ++it) {
-    bgemm(n, Z, Y, Tm, 1.0, 0.0);
+    bgemm<false, 0, false>(n, Z, n, Y, n, Tm, n, 1.0);
     double dev = 0.0;
     for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) {
       const int i = idx / n, j = idx - (idx / n) * n;
@@ -263,9 +382,9 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_lowdin_kernel(const Batch
       Tm[idx] = 1.5 * e - 0.5 * v;
     }
     dev = blk_reduce(dev, true);
-    bgemm(n, Y, Tm, fr, 1.0, 0.0);
+    bgemm<false, 0, false>(n, Y, n, Tm, n, fr, n, 1.0);
     { double* t = Y; Y = fr; fr = t; }
-    bgemm(n, Tm, Z, fr, 1.0, 0.0);
+    bgemm<false, 0, false>(n, Tm, n, Z, n, fr, n, 1.0);
     { double* t = Z; Z = fr; fr = t; }
     if (dev < 1e-13) {
       ok = true;
@@ -318,8 +437,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_init_kernel(const BatchDe
   }
   __syncthreads();
   if (!failed && core_guess) {
-    double* Xs = (p.n <= a.smem_nmax) ? xs_sh : p.T2;
-    const int steps = density_from_fock(p, d.nocc, p.H, Xs, p.P);
+    const int steps = density_from_fock(p, d.nocc, p.H, xs_sh, p.P);
     if (steps < 0 && threadIdx.x == 0) {
       st.failed = 1;
       st.done = 1;
@@ -334,7 +452,7 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_init_kernel(const BatchDe
 __global__ void __launch_bounds__(BATCH_THREADS) batch_step_kernel(const BatchDenseArgs a) {
   extern __shared__ double xs_sh[];
   __shared__ double bro[BATCH_DIIS_MAX], coef[BATCH_DIIS_MAX];
-  __shared__ int nuse;
+  __shared__ int nuse, use_slot[BATCH_DIIS_MAX];
   const int m = blockIdx.x;
   BatchMolState& st = a.st[m];
   if (st.done || st.failed) return;
@@ -344,34 +462,46 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_step_kernel(const BatchDe
   const int it = st.iter + 1;
   const double E_prev = st.E_prev, dD_prev = st.dD;
   const bool built_full = a.built_full != 0;
-  // ---- J, K (J = Jh + Jh^T of the build), F and the energy of P
+  const int ld = xs_ld(n), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  // ---- J, K (J = Jh + Jh^T of the build), F and the energy of P; the halves
+  // are transposed through shared memory
   double e = 0.0;
-  for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-    const int i = idx / n, j = idx - (idx / n) * n;
-    const size_t t = (size_t)j * n + i;
-    const double jn = (built_full ? 0.0 : p.J[idx]) + p.Jd[idx] + p.Jd[t];
-    const double kn = (built_full ? 0.0 : p.K[idx]) + p.Kd[idx] + p.Kd[t];
-    p.J[idx] = jn;
-    p.K[idx] = kn;
-    const double f = p.H[idx] + jn - 0.5 * kn;
-    p.F[idx] = f;
-    e += p.P[idx] * (p.H[idx] + f);
-  }
-  const double E = 0.5 * blk_reduce(e, false);
-  for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-    p.Jd[idx] = 0.0;
-    p.Kd[idx] = 0.0;
-  }
-  // ---- DIIS error X (F P S - S P F) X  (S P F = (F P S)^T)
-  bgemm(n, p.F, p.P, p.T1, 1.0, 0.0);
-  bgemm(n, p.T1, p.S, p.T2, 1.0, 0.0);
-  for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) {
-    const int i = idx / n, j = idx - (idx / n) * n;
-    p.T1[idx] = p.T2[idx] - p.T2[(size_t)j * n + i];
-  }
+  for (int i = warp; i < n; i += nw)
+    for (int j = lane; j < n; j += 32) xs_sh[i * ld + j] = p.Jd[(size_t)i * n + j];
   __syncthreads();
-  bgemm(n, p.X, p.T1, p.T3, 1.0, 0.0);
-  bgemm(n, p.T3, p.X, p.T1, 1.0, 0.0);
+  for (int i = warp; i < n; i += nw)
+    for (int j = lane; j < n; j += 32) {
+      const size_t q = (size_t)i * n + j;
+      p.J[q] = (built_full ? 0.0 : p.J[q]) + xs_sh[i * ld + j] + xs_sh[j * ld + i];
+      p.Jd[q] = 0.0;
+    }
+  __syncthreads();
+  for (int i = warp; i < n; i += nw)
+    for (int j = lane; j < n; j += 32) xs_sh[i * ld + j] = p.Kd[(size_t)i * n + j];
+  __syncthreads();
+  for (int i = warp; i < n; i += nw)
+    for (int j = lane; j < n; j += 32) {
+      const size_t q = (size_t)i * n + j;
+      const double kn = (built_full ? 0.0 : p.K[q]) + xs_sh[i * ld + j] + xs_sh[j * ld + i];
+      p.K[q] = kn;
+      p.Kd[q] = 0.0;
+      const double h = p.H[q], f = h + p.J[q] - 0.5 * kn;
+      p.F[q] = f;
+      e += p.P[q] * (h + f);
+    }
+  const double E = 0.5 * blk_reduce(e, false);
+  // ---- DIIS error X (F P S - S P F) X  (S P F = (F P S)^T)
+  bgemm<true, 0, true>(n, p.F, n, p.P, n, p.T3, n, 1.0);  // (F P)^T
+  bgemm<true, 0, false>(n, p.T3, n, p.S, n, xs_sh, ld, 1.0);
+  for (int i = warp; i < n; i += nw)
+    for (int j = lane; j <= i; j += 32) {
+      const double v = xs_sh[i * ld + j] - xs_sh[j * ld + i];
+      xs_sh[i * ld + j] = v;
+      xs_sh[j * ld + i] = -v;
+    }
+  __syncthreads();
+  bgemm<true, 0, true>(n, p.X, n, xs_sh, ld, p.T3, n, 1.0);
+  bgemm<true, -1, false>(n, p.T3, n, p.X, n, p.T1, n, 1.0);
   double em = 0.0;
   for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) em = fmax(em, fabs(p.T1[idx]));
   em = blk_reduce(em, true);
@@ -399,50 +529,69 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_step_kernel(const BatchDe
     double* dF = a.diis + d.diis_off;
     double* dEr = dF + (size_t)a.ndiis * n2;
     const int slot = st.head;
+    // the stored F and error, and the error's products with all stored ones
+    // (a slot in use, or this one) in one pass
+    bool used[BATCH_DIIS_MAX];
+    double v[BATCH_DIIS_MAX];
+#pragma unroll
+    for (int k = 0; k < BATCH_DIIS_MAX; ++k) {
+      used[k] = k < a.ndiis && k != slot && st.age[k] >= 0;
+      v[k] = 0.0;
+    }
     for (int idx = threadIdx.x; idx < n2; idx += blockDim.x) {
+      const double x = p.T1[idx];
       dF[(size_t)slot * n2 + idx] = p.F[idx];
-      dEr[(size_t)slot * n2 + idx] = p.T1[idx];
+      dEr[(size_t)slot * n2 + idx] = x;
+#pragma unroll
+      for (int k = 0; k < BATCH_DIIS_MAX; ++k)
+        if (used[k]) v[k] += x * dEr[(size_t)k * n2 + idx];
+        else if (k == slot) v[k] += x * x;
     }
-    __syncthreads();
-    for (int k = 0; k < a.ndiis; ++k) {
-      if (k != slot && st.age[k] < 0) continue;
-      double v = 0.0;
-      for (int idx = threadIdx.x; idx < n2; idx += blockDim.x)
-        v += dEr[(size_t)slot * n2 + idx] * dEr[(size_t)k * n2 + idx];
-      v = blk_reduce(v, false);
-      if (threadIdx.x == 0) bro[k] = v;
-    }
-    __syncthreads();  // every thread has read the slot ages before thread 0 changes them
-    if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < BATCH_DIIS_MAX; ++k)
+      if (used[k] || k == slot) {
+        const double w = blk_reduce(v[k], false);
+        if (threadIdx.x == 0) bro[k] = w;
+      }
+    __syncthreads();  // every thread has read the slot ages before warp 0 changes them
+    if (warp == 0) {
       const int D = BATCH_DIIS_MAX;
-      st.age[slot] = it;
-      for (int k = 0; k < a.ndiis; ++k)
-        if (st.age[k] >= 0) {
-          st.B[slot * D + k] = bro[k];
-          st.B[k * D + slot] = bro[k];
-        }
-      st.head = (slot + 1) % a.ndiis;
-      for (int k = 0; k < BATCH_DIIS_MAX; ++k) coef[k] = 0.0;
-      nuse = 0;
-      int use[BATCH_DIIS_MAX], nu = 0;
-      for (int k = 0; k < a.ndiis; ++k)
-        if (st.age[k] >= 0) use[nu++] = k;
+      if (lane == 0) {
+        st.age[slot] = it;
+        for (int k = 0; k < a.ndiis; ++k)
+          if (st.age[k] >= 0) {
+            st.B[slot * D + k] = bro[k];
+            st.B[k * D + slot] = bro[k];
+          }
+        st.head = (slot + 1) % a.ndiis;
+        nuse = 0;
+      }
+      if (lane < BATCH_DIIS_MAX) coef[lane] = 0.0;
+      __syncwarp();
+      int age = lane < a.ndiis ? st.age[lane] : -1;
       // drop the oldest vectors until the system is solvable
-      while (nu >= 2) {
-        double Bs[BATCH_DIIS_MAX * BATCH_DIIS_MAX], c[BATCH_DIIS_MAX + 1];
-        for (int i = 0; i < nu; ++i)
-          for (int j = 0; j < nu; ++j) Bs[i * nu + j] = st.B[use[i] * D + use[j]];
-        if (diis_solve(nu, Bs, c)) {
-          for (int i = 0; i < nu; ++i) coef[use[i]] = c[i];
-          nuse = nu;
+      while (true) {
+        const unsigned in_use = __ballot_sync(0xffffffffu, age >= 0);
+        const int nu = __popc(in_use);
+        if (nu < 2) break;
+        if (age >= 0) use_slot[__popc(in_use & ((1u << lane) - 1u))] = lane;
+        __syncwarp();
+        double c;
+        const bool solved = diis_solve(nu, st.B, D, use_slot, c);
+        if (solved) {
+          if (lane < nu) coef[use_slot[lane]] = c;
+          if (lane == 0) nuse = nu;
           break;
         }
-        int oldest = 0;
-        for (int i = 1; i < nu; ++i)
-          if (st.age[use[i]] < st.age[use[oldest]]) oldest = i;
-        st.age[use[oldest]] = -1;
-        for (int i = oldest; i + 1 < nu; ++i) use[i] = use[i + 1];
-        --nu;
+        // the ages differ: iterations
+        int oldest = age >= 0 ? age : INT_MAX;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) oldest = min(oldest, __shfl_xor_sync(0xffffffffu, oldest, o));
+        if (age == oldest) {
+          age = -1;
+          st.age[lane] = -1;
+        }
+        __syncwarp();
       }
     }
     __syncthreads();
@@ -458,9 +607,8 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_step_kernel(const BatchDe
     }
   }
   // ---- new density: Fuse (F or T2) is read before T2 is reused
-  double* Xs = (n <= a.smem_nmax) ? xs_sh : p.T2;
-  double* Pn = (p.T2 == Xs) ? p.F : p.T2;
-  const int steps = density_from_fock(p, d.nocc, Fuse, Xs, Pn);
+  double* Pn = p.T2;
+  const int steps = density_from_fock(p, d.nocc, Fuse, xs_sh, Pn);
   if (steps < 0) {
     if (threadIdx.x == 0) {
       st.failed = 1;
@@ -531,8 +679,8 @@ __global__ void __launch_bounds__(BATCH_THREADS) batch_wdens_kernel(const BatchD
   const int m = blockIdx.x;
   const BatchMolDev d = a.mol[m];
   const MolPtrs p = mol_ptrs(a, d);
-  bgemm(p.n, p.F, p.P, p.T1, 1.0, 0.0);
-  bgemm(p.n, p.P, p.T1, out + (size_t)d.mat_off, 0.5, 0.0);
+  bgemm<true, 0, false>(p.n, p.F, p.n, p.P, p.n, p.T1, p.n, 1.0);
+  bgemm<true, 0, false>(p.n, p.P, p.n, p.T1, p.n, out + (size_t)d.mat_off, p.n, 0.5);
 }
 
 __global__ void batch_dmax_kernel(int ns_max, const int4* __restrict__ mt, const int* __restrict__ bf_off,
@@ -555,7 +703,7 @@ __global__ void batch_dmax_kernel(int ns_max, const int4* __restrict__ mt, const
   out[idx] = (float)mx;
 }
 
-static size_t xs_bytes(const BatchDenseArgs& a) { return (size_t)a.smem_nmax * a.smem_nmax * sizeof(double); }
+static size_t xs_bytes(const BatchDenseArgs& a) { return (size_t)xs_rows(a.smem_nmax) * xs_ld(a.smem_nmax) * sizeof(double); }
 
 void batch_set_smem(const BatchDenseArgs& a) {
   const int sm = (int)xs_bytes(a);
