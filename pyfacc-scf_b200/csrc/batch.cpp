@@ -385,6 +385,7 @@ void Batch::build_pairs() {
                f_pr = carve((size_t)std::max<long long>(nprim_new, 1) * 3 * sizeof(double4)),
                f_prf = carve((size_t)std::max<long long>(nprim_new, 1) * 3 * sizeof(float4));
   pd.buf.ensure(std::max<size_t>(o, 256));
+  choose_split();
   char* pb = pd.buf.as<char>();
   pd.info0 = reinterpret_cast<int4*>(pb + f_i0);
   pd.info1 = reinterpret_cast<int4*>(pb + f_i1);
@@ -397,7 +398,7 @@ void Batch::build_pairs() {
     PF_CUDA(cudaMemcpyAsync(d_perm, perm.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
     PF_CUDA(cudaMemcpyAsync(d_ps, new_ps.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
     launch_gather_pairs(pd.npair, d_perm, d_ps, tmp.info0, tmp.info1, tmp.info2, tmp.geom, tmp.prim, d_q, cut,
-                        pd.info0, pd.info1, pd.info2, pd.geom, pd.prim, pd.primf, nullptr, KetTables(), stream);
+                        pd.info0, pd.info1, pd.info2, pd.geom, pd.prim, pd.primf, pd.test, pd.kt, stream);
   }
   PF_CUDA(cudaStreamSynchronize(stream));
   tp[6] = wall_ms();
@@ -409,6 +410,96 @@ void Batch::build_pairs() {
                  "  buffer alloc %.2f (%.0f MB)  gather %.2f  free %.2f\n",
                  tp[1] - tp[0], tp[2] - tp[1], scratch_mb, tp[3] - tp[2], tp[4] - tp[3], tp[5] - tp[4],
                  (double)pd.buf.bytes / 1048576.0, tp[6] - tp[5], tp[7] - tp[6]);
+}
+
+// Which (bra class, ket class) combinations go to the split kernels
+// (jk_split.cu, grad_split.cu), and the transposed records for them.  Their
+// near kernel alone is the faster one for a long list of near quartets: its
+// queues keep the lanes full across bras and molecules (a bra's kets end with
+// its molecule), its Boys table is read without bank conflicts.  256 clusters
+// of 4 to 16 waters, mixed SCF 162 -> 109 ms, 64 in FP64 103 -> 92 ms; below
+// BATCH_SPLIT_MIN candidates it loses (12 clusters, lists from 1e6 on:
+// 28.4 -> 33 ms).  The far kernel's second pass over the candidates pays where
+// a good share of the atom pairs is far (24 alkanes of 18 to 21 carbons, FP64
+// SCF: undivided 304, near alone 215, both 173 ms).  The FP64 gradient takes
+// the near kernel for the longer lists (256 clusters 95 -> 77 ms, 64 24.2 ->
+// 21.5), not for lists with far halves (the alkanes: 56 -> 63 ms).  An
+// explicit task width is for the undivided kernels, and without memory for the
+// records they run as well.
+void Batch::choose_split() {
+  pd.kt = KetTables();
+  pd.test = nullptr;
+  any_split = false;
+  for (auto& r : split_len) std::fill(std::begin(r), std::end(r), 0);
+  if (opt.task_width != 0 || pd.npair == 0) return;
+  // per molecule: candidates of a combination, weighted with the share of
+  // far atom pairs for the far ones
+  std::vector<double> far(nmol, 0.0);
+  parallel_for(nmol, [&](int m) {
+    const BatchMolHost& M = mols[m];
+    long long n = 0;
+    for (int i = 0; i < M.natoms; ++i)
+      for (int j = 0; j < i; ++j) {
+        double d2 = 0.0;
+        for (int x = 0; x < 3; ++x) d2 += (M.xyz[3 * i + x] - M.xyz[3 * j + x]) * (M.xyz[3 * i + x] - M.xyz[3 * j + x]);
+        n += d2 > FAR_DISTANCE * FAR_DISTANCE;
+      }
+    if (M.natoms > 1) far[m] = n / (0.5 * M.natoms * (M.natoms - 1));
+  });
+  for (int bc = 0; bc < NCLASS; ++bc)
+    for (int kc = 0; kc <= bc; ++kc) {
+      double nq = 0.0, nfar = 0.0;
+      for (int m = 0; m < nmol; ++m) {
+        const double nb = seg[bc][m + 1] - seg[bc][m], nk = seg[kc][m + 1] - seg[kc][m];
+        const double n = bc == kc ? 0.5 * nb * (nb + 1) : nb * nk;
+        nq += n;
+        nfar += n * far[m];
+      }
+      if (nq < BATCH_SPLIT_MIN || (bc == 2 && kc == 2) || pd.class_maxprim[bc] > SPLIT_MAXPRIM) continue;
+      split_len[bc][kc] = split_run((long long)(nq / BATCH_SPLIT_RUN_SHARE), pd.class_maxprim[bc] * pd.class_maxprim[kc], num_sms);
+      split_halves[bc][kc] = nfar >= SPLIT_MIN_FAR && nfar >= BATCH_SPLIT_FAR_SHARE * nq;
+      grad_split[bc][kc] = !split_halves[bc][kc] && nq >= BATCH_SPLIT_GRAD_MIN;
+      any_split = true;
+    }
+  if (!any_split) return;
+  size_t nslots = 0;
+  KetTables kt;
+  for (int c = 0; c < NCLASS; ++c) {
+    kt.slot[c] = (int)nslots;
+    kt.class_off[c] = pd.class_off[c];
+    kt.maxprim[c] = pd.class_maxprim[c];
+    nslots += (size_t)(pd.class_off[c + 1] - pd.class_off[c]) * (pd.class_maxprim[c] + 1);
+  }
+  kt.class_off[NCLASS] = pd.class_off[NCLASS];
+  nslots = (nslots + 64) / 64 * 64;
+  const size_t test_bytes = ((size_t)pd.npair * 2 * sizeof(float4) + 255) / 256 * 256;
+  bool fits = nslots * KetTables::SLOT_BYTES <= BATCH_KET_TABLE_MAX;
+  if (fits) {
+    try {
+      kt_buf.ensure(test_bytes + nslots * KetTables::SLOT_BYTES);
+    } catch (const Error&) {
+      fits = false;
+    }
+  }
+  if (!fits) {
+    drop_split();
+    return;
+  }
+  pd.test = kt_buf.as<float4>();
+  kt.carve(kt_buf.as<char>() + test_bytes, nslots);
+  pd.kt = kt;
+}
+
+// Back to the undivided kernels, whose lists every batch has.
+void Batch::drop_split() {
+  any_split = false;
+  for (auto& r : split_len) std::fill(std::begin(r), std::end(r), 0);
+  for (auto& r : split_tasks)
+    for (auto& c : r)
+      for (auto& t : c) t = TaskList();
+  pd.kt = KetTables();
+  pd.test = nullptr;
+  kt_buf.release();
 }
 
 // Task lists of every (bra class, ket class) combination, precision part
@@ -462,12 +553,19 @@ void Batch::build_tasks() {
           scans.push_back(Scan{bc, kc, p, wi, n});
           n += (size_t)nb + 1;
         }
+      if (split_len[bc][kc])  // FP32 derivative quartets have no split kernel
+        for (int p = 0; p < 4; ++p) {
+          scans.push_back(Scan{bc, kc, p, -1, n});
+          n += (size_t)nb + 1;
+        }
     }
   const size_t cnt_off = (n * sizeof(int) + 255) / 256 * 256;
-  const size_t bytes = cnt_off + scans.size() * (sizeof(int) + sizeof(long long)) + 256;
+  const size_t next_off = (cnt_off + scans.size() * (sizeof(int) + sizeof(long long)) + 256) / 256 * 256;
+  const size_t bytes = next_off + SPLIT_COUNTERS * sizeof(int);
   task_buf.ensure(std::max<size_t>(bytes, 256));
   int* d = task_buf.as<int>();
   int* d_nt = reinterpret_cast<int*>(task_buf.as<char>() + cnt_off);
+  jk_next = reinterpret_cast<int*>(task_buf.as<char>() + next_off);
   long long* d_nq = reinterpret_cast<long long*>(task_buf.as<char>() + cnt_off +
                                                  (scans.size() * sizeof(int) + 7) / 8 * 8);
   std::vector<int> segs((size_t)NCLASS * (nmol + 1));
@@ -506,7 +604,8 @@ void Batch::build_tasks() {
   for (size_t k = 0; k < scans.size(); ++k) {
     const Scan& sc = scans[k];
     const Range& r = range_of(sc.bc, sc.kc);
-    sa.l[k] = BatchScanList{d + r.lo[sc.prec], d + r.hi[sc.prec], d + sc.toff, r.nb, kWidths[sc.wi]};
+    sa.l[k] = BatchScanList{d + r.lo[sc.prec], d + r.hi[sc.prec], d + sc.toff, r.nb,
+                          sc.wi < 0 ? split_len[sc.bc][sc.kc] : kWidths[sc.wi]};
   }
   launch_batch_scans(sa, (int)scans.size(), stream);
   std::vector<int> nt(scans.size());
@@ -519,14 +618,20 @@ void Batch::build_tasks() {
   for (size_t k = 0; k < scans.size(); ++k) {
     const Scan& sc = scans[k];
     const Range& r = range_of(sc.bc, sc.kc);
-    TaskList& tl = tasks_w[sc.wi][sc.bc][sc.kc][sc.prec];
-    tl.width = kWidths[sc.wi];
+    TaskList& tl = sc.wi < 0 ? split_tasks[sc.bc][sc.kc][sc.prec] : tasks_w[sc.wi][sc.bc][sc.kc][sc.prec];
+    if (sc.wi >= 0) tl.width = kWidths[sc.wi];
     tl.nbra = r.nb;
     tl.ntasks = nt[k];
     tl.nquartets = nq[k];
     tl.ket_lo = d + r.lo[sc.prec];
     tl.ket_hi = d + r.hi[sc.prec];
     tl.task_off = d + sc.toff;
+    if (sc.wi < 0) {
+      tl.chunk = split_len[sc.bc][sc.kc];
+      tl.halves = split_halves[sc.bc][sc.kc];
+      tl.ntasks_c = tl.ntasks;
+      tl.off_c = tl.task_off;
+    }
   }
   for (int bc = 0; bc < NCLASS; ++bc)
     for (int kc = 0; kc <= bc; ++kc) {
@@ -559,7 +664,13 @@ void Batch::alloc() {
   const size_t o_grad = carve(3 * (size_t)natoms_tot * sizeof(double));
   const size_t o_act = carve(sizeof(StepReport));
   const size_t o_ctl = carve(sizeof(BatchScfCtl));
-  mats.ensure(o);
+  try {
+    mats.ensure(o);
+  } catch (const Error&) {  // no memory left: without the split kernels' records?
+    if (!any_split) throw;
+    drop_split();
+    mats.ensure(o);
+  }
   char* b = mats.as<char>();
   double* mp[nmat];
   for (size_t k = 0; k < nmat; ++k) mp[k] = reinterpret_cast<double*>(b + om[k]);
@@ -639,6 +750,7 @@ void Batch::fock_build(bool mixed_lists, double thresh, unsigned long long* stat
   a.thresh = thresh;
   a.stats = stats;
   a.prim_thresh = thresh * PRIM_QUARTET_REL;
+  if (any_split) launch_zero(jk_next, SPLIT_COUNTERS * sizeof(int), stream);
   const bool fork = overlap;
   cudaStream_t s32 = stream;
   if (fork) {
@@ -652,13 +764,20 @@ void Batch::fock_build(bool mixed_lists, double thresh, unsigned long long* stat
       // the two halves swap streams from class to class
       // (single-precision lists: the classes alternate between the streams)
       const bool swap = fork && (nth & 1);
+      auto build = [&](int part, bool fp32, cudaStream_t s) {
+        if (jk_splits(pd, split_tasks[bc][kc][part], bc, kc))
+          launch_jk_split(pd, split_tasks[bc][kc][part], bc, kc, fp32, 1, a, num_sms,
+                          jk_next + 2 * (2 * qclass_index(bc, kc) + (fp32 ? 1 : 0)), s == stream ? s32 : stream, s);
+        else
+          launch_jk(pd, tasks[bc][kc][part], bc, kc, fp32, 1, a, num_sms, s);
+      };
       if (all_fp32) {
-        launch_jk(pd, tasks[bc][kc][0], bc, kc, true, 1, a, num_sms, swap ? s32 : stream);
+        build(0, true, swap ? s32 : stream);
       } else if (mixed_lists) {
-        launch_jk(pd, tasks[bc][kc][1], bc, kc, false, 1, a, num_sms, swap ? s32 : stream);
-        launch_jk(pd, tasks[bc][kc][2], bc, kc, true, 1, a, num_sms, swap ? stream : s32);
+        build(1, false, swap ? s32 : stream);
+        build(2, true, swap ? stream : s32);
       } else {
-        launch_jk(pd, tasks[bc][kc][0], bc, kc, false, 1, a, num_sms, swap ? s32 : stream);
+        build(0, false, swap ? s32 : stream);
       }
     }
   if (fork) {
@@ -1026,6 +1145,7 @@ void Batch::gradient_run() {
   const bool split = pd.primf != nullptr &&
                      (opt.gradient_precision == PYFACC_PRECISION_MIXED ||
                       (opt.gradient_precision < 0 && opt.precision == PYFACC_PRECISION_MIXED));
+  if (any_split) launch_zero(jk_next, SPLIT_COUNTERS * sizeof(int), stream);
   if (split) {  // the FP32 half on the side stream, overlapping the FP64 half
     PF_CUDA(cudaEventRecord(ctx.fork, stream));
     PF_CUDA(cudaStreamWaitEvent(ctx.side, ctx.fork, 0));
@@ -1033,11 +1153,17 @@ void Batch::gradient_run() {
   int nth = 0;
   for (int bc = NCLASS - 1; bc >= 0; --bc)
     for (int kc = bc; kc >= 0; --kc, ++nth) {
+      auto derive = [&](int part, cudaStream_t s) {  // FP64
+        if (grad_split[bc][kc] && jk_splits(pd, split_tasks[bc][kc][part], bc, kc))
+          launch_grad_split(pd, split_tasks[bc][kc][part], bc, kc, g2, num_sms, jk_next + 4 * qclass_index(bc, kc), s, s);
+        else
+          launch_grad2e(pd, tasks[bc][kc][part], bc, kc, false, g2, num_sms, s);
+      };
       if (split) {  // the two halves swap streams from class to class
-        launch_grad2e(pd, tasks[bc][kc][3], bc, kc, false, g2, num_sms, (nth & 1) ? ctx.side : stream);
+        derive(3, (nth & 1) ? ctx.side : stream);
         launch_grad2e(pd, tasks[bc][kc][4], bc, kc, true, g2, num_sms, (nth & 1) ? stream : ctx.side);
       } else {
-        launch_grad2e(pd, tasks[bc][kc][0], bc, kc, false, g2, num_sms, stream);
+        derive(0, stream);
       }
     }
   if (split) {

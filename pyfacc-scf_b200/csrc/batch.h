@@ -30,6 +30,15 @@ constexpr int BATCH_DIIS_MAX = 8;
 // 512 for batches of more molecules than SMs: 0.80 -> 1.10 ms a step.
 constexpr int BATCH_THREADS = 512;
 constexpr int BATCH_NBF_MAX = 160;   // larger molecules run on their own
+// Lists for the split kernels (Batch::choose_split).
+constexpr double BATCH_SPLIT_MIN = 2.0e6;        // candidate quartets
+constexpr double BATCH_SPLIT_GRAD_MIN = 4.0e6;
+constexpr double BATCH_SPLIT_FAR_SHARE = 0.25;   // of them in far atom pairs
+// A run is as long as leaves every SM four times the runs that one molecule's
+// lists leave it: the molecules' ket lists are short and uneven (12 clusters,
+// FP64: 31.0 -> 29.0 ms; sixteen times: 64 clusters and the alkanes lose 5%).
+constexpr int BATCH_SPLIT_RUN_SHARE = 4;
+constexpr size_t BATCH_KET_TABLE_MAX = (size_t)4 << 30;  // bytes: 2500 molecules of 70 functions
 
 struct BatchMolDev {
   int nbf, nocc, ns, natoms;
@@ -144,7 +153,7 @@ struct BatchScanList {
   int* toff;  // nb + 1
   int nb, width;
 };
-constexpr int BATCH_MAX_SCANS = NQCLASS * BATCH_NPARTS * 3;
+constexpr int BATCH_MAX_SCANS = NQCLASS * BATCH_NPARTS * 4;  // three widths and the split kernels' runs
 struct BatchScanArgs {
   BatchScanList l[BATCH_MAX_SCANS];
   int* ntasks;           // per list
@@ -210,6 +219,14 @@ class Batch {
   std::vector<int> seg[NCLASS];   // per class: nmol + 1 pair offsets (relative to the class start)
   TaskList tasks_w[3][NCLASS][NCLASS][BATCH_NPARTS];  // per width (32, 16, 8)
   TaskList tasks[NCLASS][NCLASS][BATCH_NPARTS];       // the widths in use
+  // lists that go to the split kernels (chunk > 0) whatever the width, and
+  // the transposed records that those read
+  TaskList split_tasks[NCLASS][NCLASS][BATCH_NPARTS];
+  int split_len[NCLASS][NCLASS] = {};                 // kets per run, 0: undivided kernel
+  bool split_halves[NCLASS][NCLASS] = {}, grad_split[NCLASS][NCLASS] = {};
+  bool any_split = false;
+  int* jk_next = nullptr;                             // their task counters
+  DeviceBuf kt_buf;
   DeviceBuf task_buf;
   DeviceBuf mats, state_buf;
   BatchDenseArgs dargs{};
@@ -240,6 +257,8 @@ class Batch {
 
   void upload();
   void build_pairs();
+  void choose_split();
+  void drop_split();
   void build_tasks();
   void alloc();
   // J/K of Db into Jd/Kd: FP64 lists, or the FP64 + FP32 halves of mixed mode

@@ -159,6 +159,7 @@ struct TaskList {
   int ntasks_c = 0;
   int* off_c = nullptr;   // device, nbra + 1
   int task_begin_c = 0;
+  bool halves = true;     // far quartets in a kernel of their own; else all in the near one
 };
 
 // The s/p pairs' primitive records once more, transposed for lanes that each
@@ -301,6 +302,7 @@ constexpr int SPLIT_RUNS_PER_SM = 32;
 constexpr double SPLIT_MIN_FAR = 3.0e5;   // estimated far quartets of a list (split_chunk)
 constexpr double FAR_DISTANCE = 16.0;     // bohr: quartets of diffuse pairs that far apart are far in FP64
 constexpr int SPLIT_COUNTERS = 4 * NQCLASS;  // task counters of a build: two kernels per class and precision
+int split_run(long long nquartets, int prim_quartets, int num_sms);
 int split_chunk(long long nquartets, double far_share, int prim_quartets, int num_sms);
 bool jk_splits(const PairData& pd, const TaskList& tl, int bra_class, int ket_class);
 void launch_jk_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32, int nk,

@@ -106,7 +106,9 @@ __global__ void __launch_bounds__(128, grad_min_blocks(LA + LB + LC + LD)) grad_
   auto test = [&](int ib, int ket, float& cut) {
     const int bp = L.bra_base + ib, kp = L.ket_base + ket;
     const float4 bc = L.test[bp], bt = L.test2[bp], kc = L.test[kp], kt = L.test2[kp];
-    if (far_pair(bc, far_extent<double, LM>(bc.w, bt.x), kc, far_extent<double, LM>(kc.w, kt.x)) != FAR) return -1;
+    if ((FAR || L.halves) &&
+        far_pair(bc, far_extent<double, LM>(bc.w, bt.x), kc, far_extent<double, LM>(kc.w, kt.x)) != FAR)
+      return -1;
     if (A.dmax) {
       const float* dmx = A.dmax + L.info2[bp].w;
       const int ld = A.ns_ld, sa = __float_as_int(bt.z), sb = __float_as_int(bt.w), sc = __float_as_int(kt.z),
@@ -280,7 +282,7 @@ template <int LA, int LB, int LC, int LD>
 void launch_halves(int num_sms, cudaStream_t s_far, cudaStream_t s_near, GradSplitArgs k) {
   launch_one<LA, LB, LC, LD, false>(num_sms, s_near, k);
   ++k.l.next;
-  launch_one<LA, LB, LC, LD, true>(num_sms, s_far, k);
+  if (k.l.halves) launch_one<LA, LB, LC, LD, true>(num_sms, s_far, k);
 }
 
 void dispatch(int num_sms, cudaStream_t s_far, cudaStream_t s_near, const GradSplitArgs& k) {

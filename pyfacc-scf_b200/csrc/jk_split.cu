@@ -301,7 +301,9 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
   auto test = [&](int ib, int ket, float& cut) {
     const int bp = L.bra_base + ib, kp = L.ket_base + ket;
     const float4 bc = L.test[bp], bt = L.test2[bp], kc = L.test[kp], kt = L.test2[kp];
-    if (far_pair(bc, far_extent<R, C::L>(bc.w, bt.x), kc, far_extent<R, C::L>(kc.w, kt.x)) != FAR) return -1;
+    if ((FAR || L.halves) &&
+        far_pair(bc, far_extent<R, C::L>(bc.w, bt.x), kc, far_extent<R, C::L>(kc.w, kt.x)) != FAR)
+      return -1;
     int to = NRING - 1;
     if (A.dmax) {
       const float* dmx = A.dmax + L.info2[bp].w;
@@ -470,11 +472,11 @@ void launch_halves(int nk, int blocks, cudaStream_t s_far, cudaStream_t s_near, 
   if (nk == 1) {
     launch_one<R, LA, LB, LC, LD, 1, false>(blocks, s_near, k);
     ++k.l.next;
-    launch_one<R, LA, LB, LC, LD, 1, true>(blocks, s_far, k);
+    if (k.l.halves) launch_one<R, LA, LB, LC, LD, 1, true>(blocks, s_far, k);
   } else {
     launch_one<R, LA, LB, LC, LD, 2, false>(blocks, s_near, k);
     ++k.l.next;
-    launch_one<R, LA, LB, LC, LD, 2, true>(blocks, s_far, k);
+    if (k.l.halves) launch_one<R, LA, LB, LC, LD, 2, true>(blocks, s_far, k);
   }
 }
 
@@ -497,10 +499,14 @@ void dispatch(int qc, int nk, int blocks, cudaStream_t s_far, cudaStream_t s_nea
 // 4e5, FP64 build 1.00 -> 0.87 ms; C40H82 2.60 -> 2.47 ms with (pp|ss) and
 // (pp|ps), 3e5 and 5e5, too), while a cluster of 16 waters, 5e5 quartets of
 // which next to none are far, loses (0.50 -> 0.60 ms).  far_share is the share
-// of atom pairs beyond FAR_DISTANCE.  Runs as long as leave SPLIT_RUNS_PER_SM
-// per SM, more for deep contractions, whose quartets take longer.
+// of atom pairs beyond FAR_DISTANCE.
 int split_chunk(long long nquartets, double far_share, int prim_quartets, int num_sms) {
-  if ((double)nquartets * far_share < SPLIT_MIN_FAR) return 0;
+  return (double)nquartets * far_share < SPLIT_MIN_FAR ? 0 : split_run(nquartets, prim_quartets, num_sms);
+}
+
+// Runs as long as leave SPLIT_RUNS_PER_SM per SM, more for deep contractions,
+// whose quartets take longer.
+int split_run(long long nquartets, int prim_quartets, int num_sms) {
   const long long runs = (long long)num_sms * SPLIT_RUNS_PER_SM * std::min(4, std::max(1, prim_quartets / 81));
   int c = 32;
   while (c < SPLIT_CHUNK_MAX && nquartets / (2 * c) >= runs) c *= 2;

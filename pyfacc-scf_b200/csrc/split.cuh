@@ -29,6 +29,7 @@ struct SplitLists {
   const int* ket_hi;
   int nbra, ntasks, bra_base, bra_off, ket_base, same_class, qclass, task_begin;
   int chunk;  // kets per task (a multiple of 32)
+  int halves; // 0: no far kernel, the near one takes every quartet
   int maxp;   // bra primitive pairs staged per run
   int nslot;  // runs staged at a time (a power of two)
   const void* boys;  // the class's BoysRows table
@@ -53,6 +54,7 @@ inline SplitLists split_lists(const PairData& pd, const TaskList& tl, int bc, in
   k.same_class = bc == kc;
   k.qclass = bc == 0 ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
   k.chunk = tl.chunk;
+  k.halves = tl.halves ? 1 : 0;
   k.maxp = pd.class_maxprim[bc];
   k.next = next;
   return k;
