@@ -9,10 +9,11 @@ For a class (la lb|lc ld) with la >= lb, lc >= ld the generator emits
              vertical recursion, added into the contracted accumulators;
 * ``hrr``  : the horizontal recursion (a b| = (a+1_i b-1_i| + AB_i (a b-1_i|
              on the contracted accumulators, bra then ket, giving (ab|cd);
-* ``grad`` : one primitive quartet of the nuclear-gradient contraction
-             sum_abcd Gamma_abcd d(ab|cd)/dX for the centres A, B, C
-             (D follows from translational invariance), using
-             d/dA_x phi_a = 2 alpha phi_{a+1x} - a_x phi_{a-1x}.
+* ``gacc``, ``gfin`` (classes below (pp|ps)): the nuclear gradient
+             sum_abcd Gamma_abcd d(ab|cd)/dX for the centres A, B, C (D
+             follows from translational invariance); FP64 quartets of all
+             classes but (ss|ss), and FP32 ones from (pp|ps) on, take
+             grad_md.cuh instead.
 
 It also emits the algorithmic FP operation count (each + - * is one flop)
 of every routine; the kernels multiply them by the number of primitive and
@@ -249,114 +250,12 @@ def gen_class(la, lb, lc, ld):
     src.extend(out_lines)
     src.append("    (void)AB; (void)CD;")
     src.append("  }")
-    # --- gradient (primitive level, contracted with gam).  Below L = 4 one
-    # inlined routine per centre and direction (the compiler merges their
-    # common recursion terms); from L = 4 on one out-of-line routine per
-    # centre whose three directions share one recursion to L + 1 (half the
-    # operations of three separate ones; inlined, the (pp|pp) body exhausts
-    # the register file)
-    grad_flops = 0
-    for ctr in range(3 if L >= 4 else 0):
-        em = Emitter()
-        v = Vrr(em, L + 1, packed=False)
-        h = Hrr(em, lambda e, f, v=v: v.V(e, f, 0), packed=False)
-        outs = []
-        for x in range(3):
-            up_terms, dn_terms = [], []
-            k = 0
-            for a in comps(la):
-                for b in comps(lb):
-                    for c in comps(lc):
-                        for d in comps(ld):
-                            q = [a, b, c, d]
-                            qu = list(q)
-                            qu[ctr] = up(q[ctr], x)
-                            up_terms.append((f"gam[{k}]", h.full(*qu)))
-                            cnt = q[ctr][x]
-                            if cnt > 0:
-                                qd = list(q)
-                                qd[ctr] = down(q[ctr], x)
-                                dn_terms.append((scaled(cnt, f"gam[{k}]"), h.full(*qd)))
-                            k += 1
-            su = em.tmp(plain_sum(up_terms), 2 * len(up_terms) - 1)
-            expr = f"tw * {su}"
-            fl = 2
-            if dn_terms:
-                sd = em.tmp(plain_sum(dn_terms), 2 * len(dn_terms) - 1)
-                expr = f"tw * {su} - {sd}"
-                fl += 1
-            em.flops += fl
-            outs.append(expr)
-        grad_flops += em.flops
-        c = 'ABC'[ctr]
-        src.append(f"  // centre {c}: g[x] += tw * sum gam (..+1x..) - sum gam n_x (..-1x..), tw = 2 exponent")
-        src.append(f"  __device__ static __noinline__ void grad{c}(const R* __restrict__ I, const R* __restrict__ PA,")
-        src.append("      const R* __restrict__ WP, const R* __restrict__ QC, const R* __restrict__ WQ, R o2p, R nrp,")
-        src.append("      R o2q, R nrq, R o2pq, const R* __restrict__ AB, const R* __restrict__ CD,")
-        src.append("      R tw, const R* __restrict__ gam, R* __restrict__ g) {")
-        src.extend(em.lines)
-        for x in range(3):
-            src.append(f"    g[{x}] += {outs[x]};")
-        src.append("    (void)PA; (void)WP; (void)QC; (void)WQ; (void)o2p; (void)nrp; (void)o2q; (void)nrq; (void)o2pq;")
-        src.append("    (void)AB; (void)CD;")
-        src.append("  }")
-    for ctr in range(0 if L >= 4 else 3):
-        for x in range(3):
-            em = Emitter()
-            v = Vrr(em, L + 1, packed=False)
-            h = Hrr(em, lambda e, f, v=v: v.V(e, f, 0), packed=False)
-            up_terms, dn_terms = [], []
-            k = 0
-            for a in comps(la):
-                for b in comps(lb):
-                    for c in comps(lc):
-                        for d in comps(ld):
-                            q = [a, b, c, d]
-                            qu = list(q)
-                            qu[ctr] = up(q[ctr], x)
-                            up_terms.append((f"gam[{k}]", h.full(*qu)))
-                            cnt = q[ctr][x]
-                            if cnt > 0:
-                                qd = list(q)
-                                qd[ctr] = down(q[ctr], x)
-                                dn_terms.append((scaled(cnt, f"gam[{k}]"), h.full(*qd)))
-                            k += 1
-            su = em.tmp(plain_sum(up_terms), 2 * len(up_terms) - 1)
-            expr = f"tw * {su}"
-            fl = 2
-            if dn_terms:
-                sd = em.tmp(plain_sum(dn_terms), 2 * len(dn_terms) - 1)
-                expr = f"tw * {su} - {sd}"
-                fl += 1
-            em.flops += fl
-            grad_flops += em.flops
-            name = f"grad{'ABC'[ctr]}{'xyz'[x]}"
-            src.append(f"  __device__ static __forceinline__ R {name}(const R* __restrict__ I, const R* __restrict__ PA,")
-            src.append("      const R* __restrict__ WP, const R* __restrict__ QC, const R* __restrict__ WQ, R o2p, R nrp,")
-            src.append("      R o2q, R nrq, R o2pq, const R* __restrict__ AB, const R* __restrict__ CD,")
-            src.append("      R tw, const R* __restrict__ gam) {")
-            src.extend(em.lines)
-            src.append(f"    return {expr};")
-            src.append("    (void)PA; (void)WP; (void)QC; (void)WQ; (void)o2p; (void)nrp; (void)o2q; (void)nrq; (void)o2pq;")
-            src.append("    (void)AB; (void)CD;")
-            src.append("  }")
-        c = 'ABC'[ctr]
-        src.append(f"  // centre {c}: g[x] += tw * sum gam (..+1x..) - sum gam n_x (..-1x..), tw = 2 exponent")
-        src.append(f"  __device__ static __forceinline__ void grad{c}(const R* __restrict__ I, const R* __restrict__ PA,")
-        src.append("      const R* __restrict__ WP, const R* __restrict__ QC, const R* __restrict__ WQ, R o2p, R nrp,")
-        src.append("      R o2q, R nrq, R o2pq, const R* __restrict__ AB, const R* __restrict__ CD,")
-        src.append("      R tw, const R* __restrict__ gam, R* __restrict__ g) {")
-        for x in range(3):
-            src.append(f"    g[{x}] += grad{c}{'xyz'[x]}(I, PA, WP, QC, WQ, o2p, nrp, o2q, nrq, o2pq, AB, CD, tw, gam);")
-        src.append("  }")
     gsrc, ginfo = gen_contracted_grad(la, lb, lc, ld)
     src.extend(gsrc)
     src.append(f"  static constexpr int VRR_FLOPS = {vrr_flops};")
     src.append(f"  static constexpr int HRR_FLOPS = {hrr_flops};")
-    src.append(f"  static constexpr int GRAD_FLOPS = {grad_flops};")
     src.append("};")
-    return "\n".join(src), dict(tag=tag, L=L, nacc=nacc, nout=nout, vrr=vrr_flops, hrr=hrr_flops, grad=grad_flops,
-                                **ginfo)
+    return "\n".join(src), dict(tag=tag, L=L, nacc=nacc, nout=nout, vrr=vrr_flops, hrr=hrr_flops, **ginfo)
 
 
 # Classes whose gradient is contracted before the HRR (gen_contracted_grad):
@@ -376,10 +275,9 @@ def gen_contracted_grad(la, lb, lc, ld):
     terms).  ``gacc`` adds one primitive quartet into these accumulators
     (VRR to L + 1 and one multiply-add per accumulator); ``gfin`` runs the
     HRR on them once per contracted quartet and contracts with gam, giving
-    the same g[0..8] as the per-primitive routines gradA/B/C summed over the
-    primitives."""
+    g[0..8]."""
     if (la, lb, lc, ld) not in GCON_CLASSES:
-        return ["  static constexpr bool GCON = false;", "  static constexpr int NGACC = 1;",
+        return ["  static constexpr int NGACC = 1;",
                 "  static constexpr int GACC_FLOPS = 0;", "  static constexpr int GFIN_FLOPS = 0;"], \
             dict(ngacc=0, gacc=0, gfin=0)
     L = la + lb + lc + ld
@@ -436,7 +334,7 @@ def gen_contracted_grad(la, lb, lc, ld):
         else:
             acc_lines.append(f"    acc[{idx[key]}] += {val};")
             em.flops += 1
-    src = ["  static constexpr bool GCON = true;",
+    src = [
            f"  static constexpr int NGACC = {len(order)};",
            "  // one primitive quartet into the exponent-weighted accumulators",
            "  // (ta, tb, tc = 2 alpha, 2 beta, 2 gamma of the primitive)",
@@ -600,10 +498,10 @@ def generate() -> str:
     for cl in ONE_E_CLASSES:
         parts.append(gen_one_electron(*cl))
         parts.append("")
-    parts.append("// class | L | accumulators | outputs | vrr flops/prim | hrr flops/contr | grad flops/prim"
+    parts.append("// class | L | accumulators | outputs | vrr flops/prim | hrr flops/contr"
                  " | contracted-gradient accumulators | flops/prim | flops/contr")
     for t in table:
-        parts.append(f"//  {t['tag']}  | {t['L']} | {t['nacc']:3d} | {t['nout']:3d} | {t['vrr']:5d} | {t['hrr']:4d} | {t['grad']:6d}"
+        parts.append(f"//  {t['tag']}  | {t['L']} | {t['nacc']:3d} | {t['nout']:3d} | {t['vrr']:5d} | {t['hrr']:4d}"
                      f" | {t['ngacc']:3d} | {t['gacc']:4d} | {t['gfin']:5d}")
     return "\n".join(parts) + "\n"
 

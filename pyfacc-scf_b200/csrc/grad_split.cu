@@ -1,17 +1,17 @@
 // Two-electron nuclear gradient of long quartet lists, far and near quartets
-// apart: the walk, the queues and the far limit of jk_split.cu, the generated
-// derivative routines and the density products of grad2e_kernel
-// (kernels.cu).  A quartet is left out when Q_ab Q_cd times the bound on its
+// apart: the walk, the queues and the far limit of jk_split.cu, the derivatives
+// (grad_md.cuh) and the density products of grad2e_kernel (kernels.cu).  A quartet is left out when Q_ab Q_cd times the bound on its
 // density products, |D_ab D_cd| + |D_ac D_bd| + |D_ad D_bc|, stays below
 // GRAD_SPLIT_REL of the screening threshold: the undivided kernels test one
 // density factor, the largest, and evaluate quartets whose products are orders
-// of magnitude smaller.  FP64 only: C40H82 10.2 -> 8.6 ms, C100H202 60 -> 52 ms,
-// max |dg| against the undivided kernels 1e-11 Ha/bohr; in FP32 the derivative
-// arithmetic outweighs the Boys function and the split gained 0-5%.
+// of magnitude smaller.  FP64 only: C40H82 10.2 -> 8.6 ms, C100H202 60 -> 52 ms
+// (with the generated derivative routines of the time), max |dg| against the
+// undivided kernels 1e-11 Ha/bohr; in FP32 the split gained 0-5%.
 #include <cuda_runtime.h>
 
 #include <algorithm>
 
+#include "grad_md.cuh"
 #include "split.cuh"
 
 namespace pyfacc {
@@ -55,9 +55,9 @@ __device__ __forceinline__ void load_grad_ket(const KetTables& t, size_t sl, Pri
   load_ket<true, FAR>(t, sl, k);
   tc = 2 * t.al[sl];
 }
-// Resident blocks per SM: the derivative accumulators take the register file
-// of (ps|ps) and up as in the undivided kernels.
-__host__ __device__ constexpr int grad_min_blocks(int L) { return L == 0 ? 5 : (L == 1 ? 3 : 2); }
+// Resident blocks per SM that the registers are held to (5 / 3 / 2 / 2 for
+// L = 0 / 1 / 2 / 3: gly30 26.6 instead of 25.3 ms).
+__host__ __device__ constexpr int grad_min_blocks(int L) { return L < 2 ? 4 : (L == 2 ? 3 : 2); }
 
 template <int LA, int LB, int LC, int LD, bool FAR>
 __global__ void __launch_bounds__(128, grad_min_blocks(LA + LB + LC + LD)) grad_split_kernel(const GradSplitArgs args) {
@@ -158,8 +158,8 @@ __global__ void __launch_bounds__(128, grad_min_blocks(LA + LB + LC + LD)) grad_
       const double4* bra = reinterpret_cast<const double4*>(sb);
       const float* kab = GradStage::kab(st + q.slot * slot_bytes, L.maxp);
       double gr[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-      double acc[C::GCON ? C::NGACC : C::NOUT];  // accumulators, or the density products
-      if constexpr (C::GCON) {
+      double acc[C::L == 0 ? C::NGACC : C::NOUT];  // accumulators, or the density products
+      if constexpr (C::L == 0) {
 #pragma unroll
         for (int i = 0; i < C::NGACC; ++i) acc[i] = 0.0;
       } else {
@@ -194,16 +194,19 @@ __global__ void __launch_bounds__(128, grad_min_blocks(LA + LB + LC + LD)) grad_
             b.k = b2.w;
             near_setup<double, LM>(tab, PQ, b, k, pg);
           }
-          if constexpr (C::GCON) {
+          if constexpr (C::L == 0) {
             C::gacc(pg.I, b.A, pg.WP, k.A, pg.WQ, pg.o2p, pg.nrp, pg.o2q, pg.nrq, pg.o2pq, b2.x, b2.y, tc, acc);
           } else {
-            C::gradA(pg.I, b.A, pg.WP, k.A, pg.WQ, pg.o2p, pg.nrp, pg.o2q, pg.nrq, pg.o2pq, AB, CD, b2.x, acc, gr);
-            C::gradB(pg.I, b.A, pg.WP, k.A, pg.WQ, pg.o2p, pg.nrp, pg.o2q, pg.nrq, pg.o2pq, AB, CD, b2.y, acc, gr + 3);
-            C::gradC(pg.I, b.A, pg.WP, k.A, pg.WQ, pg.o2p, pg.nrp, pg.o2q, pg.nrq, pg.o2pq, AB, CD, tc, acc, gr + 6);
+            MdSide<double> bs, ks;
+            md_side(b.A, AB, b.o2p, b2.x, b2.y, bs);
+            md_side(k.A, CD, k.o2p, tc, 1.0 / k.o2p - tc, ks);
+            md_gradient<double, NB == 3, LC + LD>(
+                pg.I, FAR ? -2.0 : 2.0 * pg.nrp * b2.z, PQ, bs, ks,
+                [&](int i, int j, int c, int d) { return acc[((i * NB + j) * NCc + c) * ND + d]; }, gr);
           }
         }
       }
-      if constexpr (C::GCON) {
+      if constexpr (C::L == 0) {
         double gam[C::NOUT];
         fill_gam(gam);
         C::gfin(acc, AB, CD, gam, gr);

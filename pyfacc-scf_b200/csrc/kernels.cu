@@ -20,6 +20,7 @@
 
 #include "engine.h"
 #include "far.cuh"
+#include "grad_md.cuh"
 #include "quartet.cuh"
 
 namespace pyfacc {
@@ -1012,7 +1013,7 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
       const V* prim = grecords<R>(args);
       const R cut = (R)kcut;
       const R kab_max = fabs((R)brec[0].z);
-      if constexpr (C::GCON) {
+      if constexpr (C::L == 0 || (sizeof(R) == 4 && C::L < 3)) {
         // exponent-weighted sums over the primitive quartets, then one HRR
         // and one contraction with Gamma per contracted quartet
         R acc[C::NGACC];
@@ -1045,10 +1046,8 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
           C::gfin(acc, AB, CD, gam, gr);
         }
       } else {
-        // the (pp|pp) derivative routines are compiled out of line and read
-        // the density products through a pointer: for that class they live
-        // in shared memory (after the per-atom sums) rather than in local
-        // memory, which spilled to DRAM
+        // the 81 density products of (pp|pp) live in shared memory (after
+        // the per-atom sums): they do not fit the registers
         R gam_reg[kGamSmem ? 1 : C::NOUT];
         R* gam = kGamSmem ? reinterpret_cast<R*>(gsh + nsm) + (size_t)threadIdx.x * C::NOUT : gam_reg;
         fill_gam(gam);
@@ -1059,6 +1058,8 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
           const R kcd = fabs((R)k0.z);
           if (kab_max * kcd < cut) break;
           const R QC[3] = {(R)k2.x, (R)k2.y, (R)k2.z};
+          MdSide<R> ks;
+          md_side(QC, CD, (R)k0.y, (R)(2 * k0.w), (R)(2 * (k0.x - k0.w)), ks);
 #pragma unroll 1
           for (int kpp = kp0; kpp < bi0.w; kpp += kps) {
             const V* br = brec + 3 * kpp;
@@ -1066,14 +1067,14 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
             if (fabs((R)b0.z) * kcd < cut) break;
             ++nprim;
             const R PA[3] = {(R)b2.x, (R)b2.y, (R)b2.z};
+            const R PQ[3] = {(R)(b1.x - k1.x), (R)(b1.y - k1.y), (R)(b1.z - k1.z)};
             PrimGeo<R> pg;
             prim_setup<R, C::L + 1>(b0, b1, k0, k1, pg);
-            C::gradA(pg.I, PA, pg.WP, QC, pg.WQ, pg.o2p, pg.nrp, pg.o2q, pg.nrq, pg.o2pq, AB, CD, (R)(2 * b0.w), gam,
-                     gr);
-            C::gradB(pg.I, PA, pg.WP, QC, pg.WQ, pg.o2p, pg.nrp, pg.o2q, pg.nrq, pg.o2pq, AB, CD,
-                     (R)(2 * (b0.x - b0.w)), gam, gr + 3);
-            C::gradC(pg.I, PA, pg.WP, QC, pg.WQ, pg.o2p, pg.nrp, pg.o2q, pg.nrq, pg.o2pq, AB, CD, (R)(2 * k0.w), gam,
-                     gr + 6);
+            MdSide<R> bs;
+            md_side(PA, AB, (R)b0.y, (R)(2 * b0.w), (R)(2 * (b0.x - b0.w)), bs);
+            md_gradient<R, NB == 3, LC + LD>(
+                pg.I, (R)2 * pg.nrp * (R)b0.x, PQ, bs, ks,
+                [&](int i, int j, int c, int d) { return gam[((i * NB + j) * NCc + c) * ND + d]; }, gr);
           }
         }
       }
@@ -2250,7 +2251,8 @@ double probe_fp64(int device, double* fp32) {
 namespace pyfacc {
 
 // ---------------------------------------------------------------------------
-// Algorithmic flop counts (from the generated class routines)
+// Algorithmic flop counts (from the generated class routines; gradient: of
+// grad_md.cuh, also for the FP32 classes that keep contracted accumulators)
 // ---------------------------------------------------------------------------
 const ClassFlops& class_flops(int qc) {
   using C0 = EriClass<double, 0, 0, 0, 0>;
@@ -2260,12 +2262,12 @@ const ClassFlops& class_flops(int qc) {
   using C4 = EriClass<double, 1, 1, 1, 0>;
   using C5 = EriClass<double, 1, 1, 1, 1>;
   static const ClassFlops tab[NQCLASS] = {
-      {C0::L, C0::NOUT, C0::VRR_FLOPS, C0::HRR_FLOPS, C0::GCON ? C0::GACC_FLOPS : C0::GRAD_FLOPS, C0::GFIN_FLOPS},
-      {C1::L, C1::NOUT, C1::VRR_FLOPS, C1::HRR_FLOPS, C1::GCON ? C1::GACC_FLOPS : C1::GRAD_FLOPS, C1::GFIN_FLOPS},
-      {C2::L, C2::NOUT, C2::VRR_FLOPS, C2::HRR_FLOPS, C2::GCON ? C2::GACC_FLOPS : C2::GRAD_FLOPS, C2::GFIN_FLOPS},
-      {C3::L, C3::NOUT, C3::VRR_FLOPS, C3::HRR_FLOPS, C3::GCON ? C3::GACC_FLOPS : C3::GRAD_FLOPS, C3::GFIN_FLOPS},
-      {C4::L, C4::NOUT, C4::VRR_FLOPS, C4::HRR_FLOPS, C4::GCON ? C4::GACC_FLOPS : C4::GRAD_FLOPS, C4::GFIN_FLOPS},
-      {C5::L, C5::NOUT, C5::VRR_FLOPS, C5::HRR_FLOPS, C5::GCON ? C5::GACC_FLOPS : C5::GRAD_FLOPS, C5::GFIN_FLOPS},
+      {C0::L, C0::NOUT, C0::VRR_FLOPS, C0::HRR_FLOPS, C0::GACC_FLOPS, C0::GFIN_FLOPS},
+      {C1::L, C1::NOUT, C1::VRR_FLOPS, C1::HRR_FLOPS, md_flops(false, 0), 0},
+      {C2::L, C2::NOUT, C2::VRR_FLOPS, C2::HRR_FLOPS, md_flops(false, 1), 0},
+      {C3::L, C3::NOUT, C3::VRR_FLOPS, C3::HRR_FLOPS, md_flops(true, 0), 0},
+      {C4::L, C4::NOUT, C4::VRR_FLOPS, C4::HRR_FLOPS, md_flops(true, 1), 0},
+      {C5::L, C5::NOUT, C5::VRR_FLOPS, C5::HRR_FLOPS, md_flops(true, 2), 0},
   };
   return tab[qc];
 }
