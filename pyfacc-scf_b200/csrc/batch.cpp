@@ -478,6 +478,7 @@ void Batch::choose_split() {
     try {
       kt_buf.ensure(test_bytes + nslots * KetTables::SLOT_BYTES);
     } catch (const Error&) {
+      (void)cudaGetLastError();
       fits = false;
     }
   }
@@ -668,6 +669,7 @@ void Batch::alloc() {
     mats.ensure(o);
   } catch (const Error&) {  // no memory left: without the split kernels' records?
     if (!any_split) throw;
+    (void)cudaGetLastError();
     drop_split();
     mats.ensure(o);
   }
