@@ -554,8 +554,8 @@ void Batch::build_tasks() {
           scans.push_back(Scan{bc, kc, p, wi, n});
           n += (size_t)nb + 1;
         }
-      if (split_len[bc][kc])  // FP32 derivative quartets have no split kernel
-        for (int p = 0; p < 4; ++p) {
+      if (split_len[bc][kc])
+        for (int p = 0; p < BATCH_NPARTS; ++p) {
           scans.push_back(Scan{bc, kc, p, -1, n});
           n += (size_t)nb + 1;
         }
@@ -1155,17 +1155,18 @@ void Batch::gradient_run() {
   int nth = 0;
   for (int bc = NCLASS - 1; bc >= 0; --bc)
     for (int kc = bc; kc >= 0; --kc, ++nth) {
-      auto derive = [&](int part, cudaStream_t s) {  // FP64
+      auto derive = [&](int part, bool fp32, cudaStream_t s) {
         if (grad_split[bc][kc] && jk_splits(pd, split_tasks[bc][kc][part], bc, kc))
-          launch_grad_split(pd, split_tasks[bc][kc][part], bc, kc, g2, num_sms, jk_next + 4 * qclass_index(bc, kc), s, s);
+          launch_grad_split(pd, split_tasks[bc][kc][part], bc, kc, fp32, g2, num_sms,
+                            jk_next + 2 * (2 * qclass_index(bc, kc) + (fp32 ? 1 : 0)), s, s);
         else
-          launch_grad2e(pd, tasks[bc][kc][part], bc, kc, false, g2, num_sms, s);
+          launch_grad2e(pd, tasks[bc][kc][part], bc, kc, fp32, g2, num_sms, s);
       };
       if (split) {  // the two halves swap streams from class to class
-        derive(3, (nth & 1) ? ctx.side : stream);
-        launch_grad2e(pd, tasks[bc][kc][4], bc, kc, true, g2, num_sms, (nth & 1) ? stream : ctx.side);
+        derive(3, false, (nth & 1) ? ctx.side : stream);
+        derive(4, true, (nth & 1) ? stream : ctx.side);
       } else {
-        derive(0, stream);
+        derive(0, false, stream);
       }
     }
   if (split) {

@@ -534,6 +534,7 @@ void System::build_tasks() {
         hostbuf.insert(hostbuf.end(), lo.begin(), lo.end());
         hostbuf.insert(hostbuf.end(), hi.begin(), hi.end());
         tl.chunk = chunk;
+        tl.far = (double)quart * far_share;
         any_split = any_split || chunk > 0;
         if (chunk) {
           p.off_c = hostbuf.size();
@@ -569,6 +570,7 @@ void System::build_tasks() {
         tl.nbra = nb;
         tl.ntasks = std::max(1, tasks[bc][kc][0].ntasks);
         tl.chunk = part == 1 ? tasks[bc][kc][0].chunk : 0;
+        tl.far = tasks[bc][kc][0].far;
         tl.nquartets = tasks[bc][kc][0].nquartets;  // a bound
         tl.ntasks_c = std::max(1, tasks[bc][kc][0].ntasks_c);
         tl.task_off = tl.off_c = dd;

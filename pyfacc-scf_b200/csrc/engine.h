@@ -160,6 +160,7 @@ struct TaskList {
   int* off_c = nullptr;   // device, nbra + 1
   int task_begin_c = 0;
   bool halves = true;     // far quartets in a kernel of their own; else all in the near one
+  double far = 0.0;       // estimated far quartets
 };
 
 // The s/p pairs' primitive records once more, transposed for lanes that each
@@ -310,7 +311,11 @@ void launch_jk_split(const PairData& pd, const TaskList& tl, int bra_class, int 
 // Bound on a quartet's density products, relative to the threshold, below
 // which the split gradient leaves it out.
 constexpr double GRAD_SPLIT_REL = 1e-2;
-void launch_grad_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class,
+// Far quartets of a list (estimate) from which its FP32 derivative quartets go
+// to the split kernels: C20H42, 4e5 to 5e5 a list, 1.19 ms undivided, 1.28
+// divided; C40H82, (ss|ss) and (ps|ss) 1.5e6, 4.1 -> 3.6 ms.
+constexpr double GRAD_SPLIT_FP32_FAR = 6.0e5;
+void launch_grad_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32,
                        const struct GradArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
 void upload_boys_rows(int device);  // their Boys tables, on the current device
 const void* boys_rows_table(bool fp32, int L);
@@ -325,9 +330,10 @@ struct DynTaskSet {
   int* ntasks_dev = nullptr;   // 2 * NQCLASS counts
   double* dmax_global = nullptr;
 };
-// split: the FP32 lists of the split kernels' classes are cut into their runs.
+// The FP32 lists that the split kernels take, of at least min_far far
+// quartets, are cut into their runs.
 void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thresh, double fp32_thresh,
-                      DynTaskSet& dt, bool split, cudaStream_t s);
+                      DynTaskSet& dt, double min_far, cudaStream_t s);
 
 struct GradArgs {
   const double* Pt;

@@ -13,9 +13,10 @@
 // and 69 accumulators a lane for (pp|ss) and (ps|ps), which filled the register
 // file.  The kernels are bound by the FP64 pipe and by the registers: FP64
 // gradient of C40H82 8.6 -> 5.7 ms, gly30 51 -> 25 ms, C30H61 (STO-6G, UHF) 55
-// -> 35 ms, FP32 (pp|pp) of gly30 5.3 -> 1.2 ms, (pp|ps) 4.9 -> 2.6 ms.  FP32
-// (ps|ss), (ps|ps), (pp|ss) wait for loads either way (C100H202: 10.5 / 4.2 /
-// 1.8 ms, with this 10.5 / 4.1 / 1.6) and keep the contracted accumulators.
+// -> 35 ms, FP32 (pp|pp) of gly30 5.3 -> 1.2 ms, (pp|ps) 4.9 -> 2.6 ms.  In the
+// undivided FP32 kernels (ps|ss), (ps|ps), (pp|ss) wait for loads either way
+// (C100H202: 10.5 / 4.2 / 1.8 ms, with this 10.5 / 4.1 / 1.6) and keep the
+// contracted accumulators.
 #pragma once
 #include <cuda_runtime.h>
 
@@ -104,15 +105,15 @@ __device__ __forceinline__ void md_side(const T* PA, const T* AB, T h, T ta, T t
   }
 }
 
-// BB: the bra's second shell is p (else s); KL: the ket is (ss), (ps) or (pp).
+// BL, KL: the bra and the ket are (ss), (ps) or (pp).
 // I[m], m = 0 .. L + 1, are the Boys values with prefactor and scale = -2 rho
 // (in the far limit, where I carries rho^m, -2).  gam(i, j, k, l): the density
 // products, indices of an s shell 0.  Adds dE/dA, dE/dB, dE/dC to g.
-template <typename T, bool BB, int KL, class Gam>
+template <typename T, int BL, int KL, class Gam>
 __device__ __forceinline__ void md_gradient(const T* I, T scale, const T* PQ, const MdSide<T>& b, const MdSide<T>& k,
                                             Gam&& gam, T* g) {
-  constexpr int L = 1 + (BB ? 1 : 0) + KL, NB = BB ? 3 : 1, NC = KL > 0 ? 3 : 1, ND = KL == 2 ? 3 : 1;
-  constexpr int NHB = BB ? 10 : 4;
+  constexpr bool BB = BL == 2;
+  constexpr int L = BL + KL, NB = BB ? 3 : 1, NC = KL > 0 ? 3 : 1, ND = KL == 2 ? 3 : 1, NHB = herm_count(BL);
   const T zero = T(0.0f), mone = T(-1.0f);
   const T h2 = b.h * b.h, kh = k.h * mone, kh2 = k.h * k.h;
   // ket coefficients of L_0, L_c, L_d (L_cd: kh2); the signs are those of d/dQ
@@ -155,6 +156,8 @@ __device__ __forceinline__ void md_gradient(const T* I, T scale, const T* PQ, co
       h[herm_index(1, 1, 0)] = h2 * (G[0][1] + G[1][0]);
       h[herm_index(1, 0, 1)] = h2 * (G[0][2] + G[2][0]);
       h[herm_index(0, 1, 1)] = h2 * (G[1][2] + G[2][1]);
+    } else if constexpr (BL == 0) {
+      h[0] = gam(0, 0, c, d);
     } else {
       const T G[3] = {gam(0, 0, c, d), gam(1, 0, c, d), gam(2, 0, c, d)};
       h[0] = pf_fma(G[0], b.A[0], pf_fma(G[1], b.A[1], G[2] * b.A[2]));
@@ -214,7 +217,7 @@ __device__ __forceinline__ void md_gradient(const T* I, T scale, const T* PQ, co
     dY[x] = k.mu2 * (k.B[x] + mone * k.A[x]) * me;
   }
   const T mfb = mone * b.fb, mkb = mone * k.fb;
-  static_for<NC * ND>([&](auto cd) {
+  static_for<(BL > 0 ? NC * ND : 0)>([&](auto cd) {
     constexpr int c = decltype(cd)::value / ND, d = decltype(cd)::value % ND;
     T c0, cc, c1, V[4];
     ket(c, d, c0, cc, c1);

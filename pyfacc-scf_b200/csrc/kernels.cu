@@ -850,7 +850,7 @@ __global__ void __launch_bounds__(1024) dyn_tasks_kernel(const DynAllArgs A) {
 }
 
 void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thresh, double fp32_thresh,
-                      DynTaskSet& dt, bool split, cudaStream_t s) {
+                      DynTaskSet& dt, double min_far, cudaStream_t s) {
   dmax_global_kernel<<<1, 1024, 0, s>>>((long long)ns * ns, dmax, dt.dmax_global);
   PF_CUDA(cudaGetLastError());
   count_launch();
@@ -872,7 +872,7 @@ void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thre
         L.nket = pd.class_off[kc + 1] - pd.class_off[kc];
         L.same = bc == kc;
         L.part = part;
-        L.width = split && part == 1 && jk_splits(pd, tl, bc, kc) ? tl.chunk : tl.width;
+        L.width = part == 1 && tl.far >= min_far && jk_splits(pd, tl, bc, kc) ? tl.chunk : tl.width;
         L.task_off = tl.task_off;
         L.ket_lo = tl.ket_lo;
         L.ket_hi = tl.ket_hi;
@@ -1072,7 +1072,7 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
             prim_setup<R, C::L + 1>(b0, b1, k0, k1, pg);
             MdSide<R> bs;
             md_side(PA, AB, (R)b0.y, (R)(2 * b0.w), (R)(2 * (b0.x - b0.w)), bs);
-            md_gradient<R, NB == 3, LC + LD>(
+            md_gradient<R, LA + LB, LC + LD>(
                 pg.I, (R)2 * pg.nrp * (R)b0.x, PQ, bs, ks,
                 [&](int i, int j, int c, int d) { return gam[((i * NB + j) * NCc + c) * ND + d]; }, gr);
           }

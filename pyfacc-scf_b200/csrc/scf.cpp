@@ -79,7 +79,7 @@ void System::jk(const double* Dj, int nk, const double* const* Dk, double* Jo, d
   const bool mixed = precision == PYFACC_PRECISION_MIXED;
   if (opt.shard_count > 1) dynamic = false;  // shards use their static sub-lists
   const double t32 = fp32_thresh >= 0 ? fp32_thresh : opt.fp32_thresh;
-  if (dynamic) launch_dyn_tasks(pd, dmax, ns, thresh, mixed ? t32 : 0.0, dyn, true, stream);
+  if (dynamic) launch_dyn_tasks(pd, dmax, ns, thresh, mixed ? t32 : 0.0, dyn, 0.0, stream);
   // an all-FP32 build (the coarse phase: t32 beyond every Q_ab Q_cd max|D|)
   // has empty FP64 lists, whose kernels are not launched
   const bool fp64_part = !(dynamic && mixed && t32 >= 1e299);
@@ -858,7 +858,8 @@ void System::gradient(double* g_host) {
   const bool dyn_split = split && opt.shard_count <= 1;
   if (dyn_split)
     launch_dyn_tasks(pd, dmax, ns, gthr,
-                     opt.gradient_fp32_thresh > 0 ? opt.gradient_fp32_thresh : opt.fp32_thresh, dyn, false, stream);
+                     opt.gradient_fp32_thresh > 0 ? opt.gradient_fp32_thresh : opt.fp32_thresh, dyn, GRAD_SPLIT_FP32_FAR,
+                     stream);
   // the FP64 and FP32 halves run on different streams, which swap from
   // class to class (an FP64 gradient keeps its classes on one stream: its
   // register-heavy kernels measured slower when two of them share the SMs)
@@ -871,8 +872,9 @@ void System::gradient(double* g_host) {
     for (int kc = bc; kc >= 0; --kc, ++nth) {
       const int qc = (bc == 0) ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
       auto derive = [&](const TaskList& tl, bool fp32, cudaStream_t s) {
-        if (!fp32 && jk_splits(pd, tl, bc, kc))
-          launch_grad_split(pd, tl, bc, kc, g2, num_sms, jk_next + 4 * qc, s == stream ? ctx.side : stream, s);
+        if ((!fp32 || tl.far >= GRAD_SPLIT_FP32_FAR) && jk_splits(pd, tl, bc, kc))
+          launch_grad_split(pd, tl, bc, kc, fp32, g2, num_sms, jk_next + 2 * (2 * qc + (fp32 ? 1 : 0)),
+                            s == stream ? ctx.side : stream, s);
         else
           launch_grad2e(pd, tl, bc, kc, fp32, g2, num_sms, s);
       };
