@@ -175,9 +175,7 @@ __device__ __forceinline__ bool block_tile(const GemmArgs& g, int i0, int j0, do
 // operand row from L2 twice as often (n = 702: 178 MB per symmetric product).
 // Rows are LD32 = 36 doubles apart: the fragment loads of a half warp (four
 // rows, four k) fall into 16 different bank pairs.
-#ifndef TILE32_MIN
-#define TILE32_MIN 400
-#endif
+constexpr int TILE32_MIN = 400;
 constexpr int LD32 = 36, STAGES32 = 4;
 constexpr size_t SMEM32 = STAGES32 * 2 * 32 * LD32 * sizeof(double);
 
@@ -570,7 +568,8 @@ template <int TILE> __global__ void __launch_bounds__(32 * SPLITK) tc2g_step_ker
 // product's own 0.5 us at n = 7 and 1.5 us at n = 56 (water: 192 steps of an
 // SCF 1.2 -> 0.2 ms).  Above TC2_SMALL_MAX one SM's FP64 tensor rate costs more
 // than that (n = 96: 1900 m8n8k4 products, 3.6 us).
-constexpr int SMALL_TILES = 3;  // 8 x 8 tiles per warp: 78 of n = 96 on 26 warps
+constexpr int SMALL_TILES = 2;  // 8 x 8 tiles per warp: 45 of n = 72 on 23 warps
+static_assert((TC2_SMALL_MAX / 8) * (TC2_SMALL_MAX / 8 + 1) / 2 <= 26 * SMALL_TILES, "tiles of the largest n");
 __global__ void __launch_bounds__(1024) tc2_small_kernel(int n, int ld, double nocc, const double* __restrict__ F,
                                                          double* __restrict__ X, double* __restrict__ st, int kmax) {
   extern __shared__ __align__(16) double xs[];

@@ -413,6 +413,9 @@ void System::build_pairs() {
   }
   pd.kt.class_off[NCLASS] = pd.class_off[NCLASS];
   nslots = (nslots + 64) / 64 * 64;
+  // (rows are as many as the deepest contraction has: without the tables, and
+  // with the undivided kernels, where that is out of proportion)
+  const bool tables = nslots * KetTables::SLOT_BYTES <= KET_TABLE_MAX;
   // final records
   o = 0;
   const size_t f_i0 = carve(pd.npair * sizeof(int4)), f_i1 = carve(pd.npair * sizeof(int4)),
@@ -420,7 +423,7 @@ void System::build_pairs() {
                f_pr = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(double4)),
                f_prf = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(float4)),
                f_test = carve(pd.npair * 2 * sizeof(float4)),
-               f_kt = carve(nslots * KetTables::SLOT_BYTES);
+               f_kt = carve(tables ? nslots * KetTables::SLOT_BYTES : 0);
   pd.buf.ensure(std::max<size_t>(o, 256));
   char* pb = pd.buf.as<char>();
   pd.info0 = reinterpret_cast<int4*>(pb + f_i0);
@@ -429,7 +432,8 @@ void System::build_pairs() {
   pd.geom = reinterpret_cast<double4*>(pb + f_g);
   pd.prim = reinterpret_cast<double4*>(pb + f_pr);
   pd.primf = reinterpret_cast<float4*>(pb + f_prf);
-  pd.kt.carve(pb + f_kt, nslots);
+  if (tables) pd.kt.carve(pb + f_kt, nslots);
+  else pd.kt = KetTables();
   pd.test = reinterpret_cast<float4*>(pb + f_test);
   if (pd.npair > 0) {
     PF_CUDA(cudaMemcpyAsync(d_perm, perm.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));

@@ -195,6 +195,8 @@ struct KetTables {
   }
 };
 
+constexpr size_t KET_TABLE_MAX = (size_t)16 << 30;  // bytes, one molecule (C100H202: 0.17 GB)
+
 // Packed pair data of one molecule or of a batch (every pair stores the
 // offset and leading dimension of its molecule's matrices).
 struct PairData {

@@ -498,7 +498,7 @@ void dispatch(int qc, int nk, int blocks, cudaStream_t s_far, cudaStream_t s_nea
 // with 3e5 of them per class and more the whole build gains (C20H42 (ss|ss):
 // 4e5, FP64 build 1.00 -> 0.87 ms; C40H82 2.60 -> 2.47 ms with (pp|ss) and
 // (pp|ps), 3e5 and 5e5, too), while a cluster of 16 waters, 5e5 quartets of
-// which next to none are far, loses (0.50 -> 0.60 ms).  far_share is the share
+// which next to none are far, loses (0.46 -> 0.63 ms).  far_share is the share
 // of atom pairs beyond FAR_DISTANCE.
 int split_chunk(long long nquartets, double far_share, int prim_quartets, int num_sms) {
   return (double)nquartets * far_share < SPLIT_MIN_FAR ? 0 : split_run(nquartets, prim_quartets, num_sms);
