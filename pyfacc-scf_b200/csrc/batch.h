@@ -17,6 +17,7 @@
 #pragma once
 #include <array>
 #include <cmath>
+#include <memory>
 #include <string>
 #include <vector>
 
@@ -257,6 +258,7 @@ class Batch {
 
   void upload();
   void build_pairs();
+  void pair_offsets(std::vector<int>* off) const;
   void choose_split();
   void drop_split();
   void build_tasks();
