@@ -264,8 +264,7 @@ void Batch::build_pairs() {
   // pairs of class c of molecule m occupy [moff[c][m], moff[c][m + 1]) of
   // the class-major list, in (i, j <= i) shell order (as one molecule's
   // engine lists them), and their primitive pairs follow one another from
-  // poff[c][m]; every molecule fills its own ranges.  256 clusters of 4 to 16
-  // waters: 6 -> 1 ms (serial sums over 330000 zeroed entries before)
+  // poff[c][m]; batch_pairs_kernel fills them
   std::vector<int> moff[NCLASS];
   pair_offsets(moff);
   int off[NCLASS + 1] = {0, 0, 0, 0};
@@ -294,23 +293,13 @@ void Batch::build_pairs() {
       poff[c][m] = nprim_tot;
       nprim_tot += n;
     }
-  std::unique_ptr<int4[]> all0(new int4[std::max(np_all, 1)]), all1(new int4[std::max(np_all, 1)]);
-  parallel_for(nmol, [&](int m) {
-    const BatchMolHost& M = mols[m];
-    int pos[NCLASS] = {moff[0][m], moff[1][m], moff[2][m]};
-    long long pp[NCLASS] = {poff[0][m], poff[1][m], poff[2][m]};
-    for (int i = 0; i < M.ns; ++i)
-      for (int j = 0; j <= i; ++j) {
-        int a = i, b = j;
-        if (M.basis.shells[a].l < M.basis.shells[b].l) std::swap(a, b);
-        const int c = M.basis.shells[a].l + M.basis.shells[b].l;
-        const int k = pos[c]++;
-        all0[k] = make_int4(M.shell_off + a, M.shell_off + b, (int)std::min<long long>(pp[c], INT32_MAX), M.shell_off);
-        all1[k] = make_int4((int)M.mat_off, M.nbf, m, m * ns_max * ns_max);
-        pp[c] += (long long)(M.basis.shells[a].ex.size() * M.basis.shells[b].ex.size());
-      }
-  });
   if (nprim_tot >= (1LL << 31)) throw Error(PYFACC_ERR_INVALID, "batch too large: split it into several calls");
+  std::vector<int> offs(2 * NCLASS * (size_t)nmol);
+  for (int c = 0; c < NCLASS; ++c)
+    for (int m = 0; m < nmol; ++m) {
+      offs[(size_t)c * nmol + m] = moff[c][m];
+      offs[((size_t)NCLASS + c) * nmol + m] = (int)poff[c][m];
+    }
   size_t o = 0;
   auto carve = [&](size_t bytes) {
     size_t r = o;
@@ -323,7 +312,8 @@ void Batch::build_pairs() {
                s_i2 = carve(np_all * sizeof(int4)), s_g = carve(np_all * sizeof(double4)),
                s_pr = carve((size_t)std::max<long long>(nprim_tot, 1) * 3 * sizeof(double4)),
                s_q = carve(np_all * sizeof(double)), s_perm = carve(np_all * sizeof(int)),
-               s_ps = carve(np_all * sizeof(int)), s_kept = carve(np_all * sizeof(int));
+               s_ps = carve(np_all * sizeof(int)), s_kept = carve(np_all * sizeof(int)),
+               s_offs = carve(offs.size() * sizeof(int));
   DeviceBuf scratch;
   scratch.ensure(o);
   const double scratch_mb = (double)o / 1048576.0;
@@ -344,8 +334,11 @@ void Batch::build_pairs() {
   double maxpref = 0.0;
   for (const auto& m : mols) maxpref = std::max(maxpref, max_prim_prefactor(m.basis));
   const double cut = PRIM_CUT_REL * maxpref;
-  PF_CUDA(cudaMemcpyAsync(d_pl0, all0.get(), np_all * sizeof(int4), cudaMemcpyHostToDevice, stream));
-  PF_CUDA(cudaMemcpyAsync(d_pl1, all1.get(), np_all * sizeof(int4), cudaMemcpyHostToDevice, stream));
+  int* d_offs = reinterpret_cast<int*>(sb + s_offs);
+  PF_CUDA(cudaMemcpyAsync(d_offs, offs.data(), offs.size() * sizeof(int), cudaMemcpyHostToDevice, stream));
+  launch_batch_pairs(BatchPairArgs{shd.desc, shd.nprim, mt_dev, d_offs, d_offs + (size_t)NCLASS * nmol, nmol, ns_max,
+                                   d_pl0, d_pl1},
+                     stream);
   launch_build_pairs(shd, np_all, d_pl0, d_pl1, tmp.info0, tmp.info1, tmp.info2, tmp.geom, tmp.prim, cut, d_kept,
                      stream);
   launch_schwarz(tmp, off, d_q, stream);

@@ -161,6 +161,20 @@ struct BatchScanArgs {
   long long* nquartets;  // per list
 };
 void launch_batch_ranges(const BatchRangeArgs& a, int nlists, int nb_max, cudaStream_t s);
+// Pair lists of all molecules for launch_build_pairs: class by class, molecule
+// by molecule (pair_off, prim_off: first pair and first primitive pair of class
+// c of molecule m at [c * nmol + m]), in (i, j <= i) shell order.
+struct BatchPairArgs {
+  const int4* desc;  // shells
+  const int* nprim;
+  const int4* mt;    // {first shell, ns, mat_off, nbf} per molecule
+  const int* pair_off;
+  const int* prim_off;
+  int nmol, ns_max;
+  int4* pl0;
+  int4* pl1;
+};
+void launch_batch_pairs(const BatchPairArgs& a, cudaStream_t s);
 void launch_batch_scans(const BatchScanArgs& a, int nlists, cudaStream_t s);
 
 struct BatchMolHost {

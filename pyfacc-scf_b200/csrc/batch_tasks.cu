@@ -1,4 +1,4 @@
-// Task lists of the batched engine, built on the device.
+// Pair and task lists of the batched engine, built on the device.
 //
 // Pairs of a class are sorted by molecule, then by Schwarz factor Q
 // (descending), so the kets a bra reaches are a prefix of its molecule's
@@ -115,7 +115,67 @@ __global__ void __launch_bounds__(1024) batch_scan_kernel(const BatchScanArgs A)
   }
 }
 
+// The pair lists of all molecules, a block per molecule: with the numbers of s
+// and p shells before every shell, and the sums of their primitive counts, the
+// place of a pair within its class and its first primitive pair are products
+// and triangle numbers.  256 water clusters: 10 MB of lists written here instead
+// of on the host and copied, setup 18.4 -> 13.6 ms.
+__global__ void __launch_bounds__(256) batch_pairs_kernel(const BatchPairArgs A) {
+  extern __shared__ int sh[];
+  const int m = blockIdx.x;
+  const int4 mt = A.mt[m];  // {first shell, ns, mat_off, nbf}
+  const int ns = mt.y;
+  // per shell: type, primitives, then of each type before it: shells,
+  // primitives, squares of the primitives
+  int *l = sh, *n = l + A.ns_max, *cnt = n + A.ns_max, *sum = cnt + 2 * A.ns_max, *sq = sum + 2 * A.ns_max;
+  for (int i = threadIdx.x; i < ns; i += blockDim.x) {
+    l[i] = A.desc[mt.x + i].x > 0 ? 1 : 0;
+    n[i] = A.nprim[mt.x + i];
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    int c = 0, s = 0, q = 0;
+    for (int i = 0; i < ns; ++i) {
+      cnt[2 * i + threadIdx.x] = c;
+      sum[2 * i + threadIdx.x] = s;
+      sq[2 * i + threadIdx.x] = q;
+      if (l[i] == (int)threadIdx.x) {
+        ++c;
+        s += n[i];
+        q += n[i] * n[i];
+      }
+    }
+  }
+  __syncthreads();
+  for (int t = threadIdx.x; t < ns * (ns + 1) / 2; t += blockDim.x) {
+    int i = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+    while (i * (i + 1) / 2 > t) --i;
+    while ((i + 1) * (i + 2) / 2 <= t) ++i;
+    const int j = t - i * (i + 1) / 2, li = l[i], lj = l[j], c = li + lj;
+    int k = cnt[2 * j + lj], z = n[i] * sum[2 * j + lj];  // within row i
+    if (c == 1) {
+      k += cnt[2 * i] * cnt[2 * i + 1];
+      z += sum[2 * i] * sum[2 * i + 1];
+    } else {
+      k += cnt[2 * i + li] * (cnt[2 * i + li] + 1) / 2;
+      z += (sum[2 * i + li] * sum[2 * i + li] + sq[2 * i + li]) / 2;
+    }
+    k += A.pair_off[c * A.nmol + m];
+    z += A.prim_off[c * A.nmol + m];
+    const int a = li < lj ? j : i, b = li < lj ? i : j;
+    A.pl0[k] = make_int4(mt.x + a, mt.x + b, z, mt.x);
+    A.pl1[k] = make_int4(mt.z, mt.w, m, m * A.ns_max * A.ns_max);
+  }
+}
+
 }  // namespace
+
+void launch_batch_pairs(const BatchPairArgs& a, cudaStream_t s) {
+  if (a.nmol <= 0) return;
+  batch_pairs_kernel<<<a.nmol, 256, 8 * (size_t)a.ns_max * sizeof(int), s>>>(a);
+  PF_CUDA(cudaGetLastError());
+  count_launch();
+}
 
 void launch_batch_ranges(const BatchRangeArgs& a, int nlists, int nb_max, cudaStream_t s) {
   if (nlists <= 0 || nb_max <= 0) return;
