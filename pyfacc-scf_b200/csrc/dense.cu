@@ -578,7 +578,8 @@ __global__ void __launch_bounds__(1024) tc2_small_kernel(int n, int ld, double n
   double* cur = xs;
   double* nxt = xs + (size_t)np * ld;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5, gr = lane >> 2, tq = lane & 3;
-  // Gershgorin bounds, a warp per row
+  // Gershgorin bounds, a warp per row (through the words that the second call
+  // of block_sums writes: the first one's barrier lies in between)
   double lo = 1e300, hi = -1e300;
   for (int i = warp; i < n; i += nw) {
     double r = 0.0;
@@ -591,18 +592,20 @@ __global__ void __launch_bounds__(1024) tc2_small_kernel(int n, int ld, double n
     hi = fmax(hi, d + r);
   }
   if (lane == 0) {
-    red[0][warp][0] = lo;
-    red[0][warp][1] = hi;
+    red[1][warp][0] = lo;
+    red[1][warp][1] = hi;
   }
   __syncthreads();
   for (int w = 0; w < nw; ++w) {
-    lo = fmin(lo, red[0][w][0]);
-    hi = fmax(hi, red[0][w][1]);
+    lo = fmin(lo, red[1][w][0]);
+    hi = fmax(hi, red[1][w][1]);
   }
   const double sc = 1.0 / (hi - lo);
-  // the sums of two words over the block; slot alternates, so that one
-  // barrier per call is enough
-  auto block_sums = [&](int slot, double& s1, double& s2) {
+  // the sums of two words over the block.  One barrier per call: consecutive
+  // calls use different slots (each call flips it), so a warp that is ahead
+  // writes where nobody reads until it has passed the next call's barrier
+  int slot = 0;
+  auto block_sums = [&](double& s1, double& s2) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       s1 += __shfl_xor_sync(0xffffffffu, s1, o);
@@ -620,6 +623,7 @@ __global__ void __launch_bounds__(1024) tc2_small_kernel(int n, int ld, double n
       s1 += __shfl_xor_sync(0xffffffffu, s1, o);
       s2 += __shfl_xor_sync(0xffffffffu, s2, o);
     }
+    slot ^= 1;
   };
   double t1 = 0.0, t2 = 0.0;
   for (int q = tid; q < np * ld; q += blockDim.x) {
@@ -633,7 +637,7 @@ __global__ void __launch_bounds__(1024) tc2_small_kernel(int n, int ld, double n
     cur[q] = v;
     nxt[q] = 0.0;
   }
-  block_sums(1, t1, t2);
+  block_sums(t1, t2);
   const int nt = np >> 3, ntiles = nt * (nt + 1) / 2;
   // this warp's tiles, at most SMALL_TILES: operand rows and result offset
   int toff[SMALL_TILES], ra[SMALL_TILES], rb[SMALL_TILES], mine = 0;
@@ -691,7 +695,7 @@ __global__ void __launch_bounds__(1024) tc2_small_kernel(int n, int ld, double n
         s2 += row == col + 1 ? v1 * v1 : 2.0 * v1 * v1;
       }
     }
-    block_sums(steps & 1, s1, s2);
+    block_sums(s1, s2);
     t1 = s1;
     t2 = s2;
     double* x = cur;
