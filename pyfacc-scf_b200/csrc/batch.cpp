@@ -766,7 +766,7 @@ void Batch::alloc() {
   a.built_full = 1;
   a.coarse = 0;
   a.smem_nmax = nbf_max;  // nbf <= 160: at most 205 KB of shared memory
-  batch_set_smem(a);
+  batch_set_smem();
   PF_CUDA(cudaStreamSynchronize(stream));
 }
 

@@ -104,9 +104,9 @@ void add_batch_update_node(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraph
 // X = S^{-1/2} of every molecule (coupled Newton-Schulz), into Xout; F, T1..T3
 // are work space.  A molecule whose iteration does not converge is marked failed.
 void launch_batch_lowdin(int nmol, const BatchDenseArgs& a, double* Xout, cudaStream_t s);
-// Dynamic shared memory of the dense-step kernels (a matrix of a.smem_nmax
-// functions); called once before any launch/capture.
-void batch_set_smem(const BatchDenseArgs& a);
+// Allows the dense-step kernels the shared memory of the largest molecule
+// (BATCH_NBF_MAX functions); called before any launch/capture.
+void batch_set_smem();
 // P = diag(occ[occ_off + i]) of every molecule (atomic-occupation guess).
 void launch_batch_guess(int nmol, const BatchDenseArgs& a, const double* occ, cudaStream_t s);
 // Density of F = H (core guess) or of the guess already in P: sets P,

@@ -703,12 +703,11 @@ __global__ void batch_dmax_kernel(int ns_max, const int4* __restrict__ mt, const
   out[idx] = (float)mx;
 }
 
-static size_t xs_bytes(const BatchDenseArgs& a) { return (size_t)xs_rows(a.smem_nmax) * xs_ld(a.smem_nmax) * sizeof(double); }
+static constexpr size_t xs_bytes(int nmax) { return (size_t)xs_rows(nmax) * xs_ld(nmax) * sizeof(double); }
 
-void batch_set_smem(const BatchDenseArgs& a) {
-  const int sm = (int)xs_bytes(a);
-  PF_CUDA(cudaFuncSetAttribute(batch_init_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
-  PF_CUDA(cudaFuncSetAttribute(batch_step_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, sm));
+void batch_set_smem() {
+  allow_smem(batch_init_kernel, xs_bytes(BATCH_NBF_MAX));
+  allow_smem(batch_step_kernel, xs_bytes(BATCH_NBF_MAX));
 }
 
 __global__ void __launch_bounds__(BATCH_THREADS) batch_full_density_kernel(const BatchDenseArgs a) {
@@ -745,7 +744,7 @@ void launch_batch_guess(int nmol, const BatchDenseArgs& a, const double* occ, cu
 
 void launch_batch_init(int nmol, const BatchDenseArgs& a, int core_guess, cudaStream_t s) {
   if (nmol <= 0) return;
-  batch_init_kernel<<<nmol, BATCH_THREADS, xs_bytes(a), s>>>(a, core_guess);
+  batch_init_kernel<<<nmol, BATCH_THREADS, xs_bytes(a.smem_nmax), s>>>(a, core_guess);
   PF_CUDA(cudaGetLastError());
   count_launch();
 }
@@ -815,7 +814,7 @@ void add_batch_update_node(cudaGraph_t g, cudaGraphNode_t* node, const cudaGraph
 
 void launch_batch_step(int nmol, const BatchDenseArgs& a, cudaStream_t s) {
   if (nmol <= 0) return;
-  batch_step_kernel<<<nmol, BATCH_THREADS, xs_bytes(a), s>>>(a);
+  batch_step_kernel<<<nmol, BATCH_THREADS, xs_bytes(a.smem_nmax), s>>>(a);
   PF_CUDA(cudaGetLastError());
   count_launch();
 }

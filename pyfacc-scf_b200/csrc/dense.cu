@@ -319,7 +319,7 @@ void gemm_launch(const GemmArgs& g, cudaStream_t s) {
   if constexpr (!ASYMA) {  // (the commutator of the first iteration keeps the small tiles)
     if (std::min(g.m, g.n) >= TILE32_MIN) {
       const int nm = (g.m + 31) / 32, nn = (g.n + 31) / 32;
-      PF_CUDA(cudaFuncSetAttribute(dgemm32_kernel<TA, TB, SYM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM32));
+      allow_smem(dgemm32_kernel<TA, TB, SYM>, SMEM32);
       dgemm32_kernel<TA, TB, SYM><<<SYM ? nn * (nn + 1) / 2 : nm * nn, 256, SMEM32, s>>>(g);
       return;
     }
@@ -714,11 +714,14 @@ __global__ void __launch_bounds__(1024) tc2_small_kernel(int n, int ld, double n
 
 }  // namespace
 
+static constexpr int small_rows(int n) { return (n + 7) & ~7; }
+static constexpr int small_ld(int n) { return (small_rows(n) - 4 + 15) / 16 * 16 + 4; }  // rows 4 bank pairs apart
+static constexpr size_t small_smem(int n) { return 2 * (size_t)small_rows(n) * small_ld(n) * sizeof(double); }
+
 void launch_tc2_small(int n, int nocc, const double* Fp, double* X, double* st, int kmax, cudaStream_t s) {
-  const int np = (n + 7) & ~7, ld = (np - 4 + 15) / 16 * 16 + 4;  // rows 4 bank pairs apart
-  const size_t smem = 2 * (size_t)np * ld * sizeof(double);
-  if (smem > 48 * 1024)
-    PF_CUDA(cudaFuncSetAttribute(tc2_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int np = small_rows(n), ld = small_ld(n);
+  const size_t smem = small_smem(n);
+  if (smem > 48 * 1024) allow_smem(tc2_small_kernel, small_smem(TC2_SMALL_MAX));
   // two tiles per warp where the warps suffice: the block's sums cost a warp as
   // much as a tile
   const int nt = np / 8, tiles = nt * (nt + 1) / 2, warps = std::max(1, std::min(26, (tiles + 1) / 2));
@@ -799,8 +802,7 @@ static cudaGraphExec_t build_tc2_graph_impl(int n, int nocc, const double* Fp, d
       PF_CUDA(cudaGraphAddKernelNode(&ni, graph, &nb, 1, &p));
     }
     const int tile = n >= TILE32_MIN ? 32 : 16;
-    if (tile == 32)
-      PF_CUDA(cudaFuncSetAttribute(tc2g_step_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM32));
+    if (tile == 32) allow_smem(tc2g_step_kernel<32>, SMEM32);
     const int nt = (n + tile - 1) / tile;
     const int blocks = nt * (nt + 1) / 2;
     cudaGraphConditionalHandle h;

@@ -40,6 +40,15 @@ struct Error : std::runtime_error {
       throw ::pyfacc::Error(PYFACC_ERR_CUDA, std::string(#x) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Allows a kernel `bound` bytes of dynamic shared memory on the current device.
+// The limit belongs to the kernel and the device, and a lower value set for one
+// launch would fail a larger launch of another thread's system between that
+// one's call and its launch: callers pass the kernel's own bound, the same on
+// every call, never the size of one launch.
+template <class Kernel> void allow_smem(Kernel* kernel, size_t bound) {
+  PF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bound));
+}
+
 constexpr int NCLASS = 3;        // ss, ps, pp: the pair classes of the straight-line kernels
 constexpr int NQCLASS = 6;       // (ss|ss) (ps|ss) (ps|ps) (pp|ss) (pp|ps) (pp|pp)
 // With d shells three more pair classes follow: ds, dp, dd (l_a >= l_b);

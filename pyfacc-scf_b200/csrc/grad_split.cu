@@ -307,8 +307,9 @@ void launch_one(int num_sms, cudaStream_t s, GradSplitArgs k) {
   while (k.l.nslot > 2 && 4 * k.l.nslot * b > GRAD_STAGE_MAX_BYTES) k.l.nslot /= 2;
   const size_t smem = (3 * (size_t)k.smem_atoms * sizeof(double) + 15) / 16 * 16 + 4 * k.l.nslot * b;
   if (smem > 32 * 1024)
-    PF_CUDA(cudaFuncSetAttribute(grad_split_kernel<R, LA, LB, LC, LD, FAR>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(grad_split_kernel<R, LA, LB, LC, LD, FAR>,
+               3 * GRAD_SPLIT_SMEM_ATOMS * sizeof(double) +
+                   std::max(GRAD_STAGE_MAX_BYTES, 4 * 2 * GradStage<R>::bytes(SPLIT_MAXPRIM)));
   const int blocks = (int)std::max(
       1LL, std::min((k.l.ntasks + 3LL) / 4, (long long)num_sms * grad_min_blocks(LA + LB + LC + LD)));
   grad_split_kernel<R, LA, LB, LC, LD, FAR><<<blocks, 128, smem, s>>>(k);

@@ -460,8 +460,8 @@ void launch_one(int blocks, cudaStream_t s, SplitArgs k) {
   while (k.l.nslot > 2 && 4 * k.l.nslot * b > STAGE_MAX_BYTES) k.l.nslot /= 2;
   const size_t smem = 4 * k.l.nslot * b;
   if (smem > 32 * 1024)
-    PF_CUDA(cudaFuncSetAttribute(jk_split_kernel<R, LA, LB, LC, LD, NK, FAR>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    allow_smem(jk_split_kernel<R, LA, LB, LC, LD, NK, FAR>,
+               std::max(STAGE_MAX_BYTES, 4 * 2 * Stage<R, (LA + LB > 0), FAR>::bytes(SPLIT_MAXPRIM)));
   jk_split_kernel<R, LA, LB, LC, LD, NK, FAR><<<blocks, 128, smem, s>>>(k);
   PF_CUDA(cudaGetLastError());
   count_launch();

@@ -1119,11 +1119,16 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
   }
 }
 
+// Atoms summed in shared memory: 6 KB of per-block sums; above that the
+// end-of-block flush costs more than the contention it saves.
+constexpr int GRAD_SMEM_ATOMS = 256;
+// Bound on a block's shared memory: those sums, the (pp|pp) density products
+// of 128 threads, or staged FP32 records.
+constexpr size_t GRAD_SMEM_MAX = 3 * GRAD_SMEM_ATOMS * sizeof(double) + 128 * 81 * sizeof(double) + JK_STAGE_MAX_BYTES + 16;
+
 template <typename R, int LA, int LB, int LC, int LD>
 static void grad2e_launch(dim3 grid, dim3 block, size_t smem, cudaStream_t s, const GradKernelArgs& k) {
-  if (smem > 48 * 1024)
-    PF_CUDA(cudaFuncSetAttribute(grad2e_kernel<R, LA, LB, LC, LD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem));
+  if (smem > 48 * 1024) allow_smem(grad2e_kernel<R, LA, LB, LC, LD>, GRAD_SMEM_MAX);
   grad2e_kernel<R, LA, LB, LC, LD><<<grid, block, smem, s>>>(k);
 }
 
@@ -1154,9 +1159,7 @@ void launch_grad2e(const PairData& pd, const TaskList& tl, int bc, int kc, bool 
   k.same_class = (bc == kc);
   k.qclass = qclass_of(bc, kc);
   k.lwidth = width_log2(tl.width);
-  // up to 256 atoms (6 KB of per-block sums; above that the end-of-block
-  // flush costs more than the contention it saves)
-  k.smem_atoms = (a.natoms_total > 0 && a.natoms_total <= 256) ? a.natoms_total : 0;
+  k.smem_atoms = (a.natoms_total > 0 && a.natoms_total <= GRAD_SMEM_ATOMS) ? a.natoms_total : 0;
   // the (pp|pp) kernels keep each thread's density products in shared memory
   const size_t gam_bytes = k.qclass == NQCLASS - 1 ? 128 * 81 * (fp32 ? sizeof(float) : sizeof(double)) : 0;
   const int tpw = 32 / tl.width;
@@ -1692,10 +1695,12 @@ __global__ void __launch_bounds__(128) grad1e_kernel(int npair, const int2* __re
     if (gsh[i] != 0.0) atomicAdd(args.grad + i, gsh[i]);
 }
 
+constexpr size_t GRAD1E_SMEM_MAX = 96 * 1024;
+
 template <int LA, int LB>
 static void grad1e_launch(int blocks, size_t smem, int use_smem, int n, const int2* pairs, const ShellDev& sh,
                           const OneEGradArgs& a, cudaStream_t s) {
-  PF_CUDA(cudaFuncSetAttribute(grad1e_kernel<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) allow_smem(grad1e_kernel<LA, LB>, GRAD1E_SMEM_MAX);
   grad1e_kernel<LA, LB><<<blocks, 128, smem, s>>>(n, pairs, sh.cen, sh.desc, sh.nprim, sh.ex, sh.co, sh.mol, use_smem,
                                                   a);
 }
@@ -1705,7 +1710,7 @@ void launch_grad1e(const ShellDev& sh, const int* npair, const int2* const* pair
   // per-atom partial sums in shared memory while they fit (one molecule),
   // straight global atomics for the many atoms of a batch
   const size_t need = 3 * (size_t)a.natoms_total * sizeof(double);
-  const int use_smem = need <= 96 * 1024;
+  const int use_smem = need <= GRAD1E_SMEM_MAX;
   const size_t smem = use_smem ? need : 0;
   for (int c = 0; c < NPAIRCLASS; ++c) {
     if (npair[c] <= 0) continue;

@@ -461,18 +461,20 @@ __global__ void eri_tensor_d_kernel(const DListArgs L, int n, double* __restrict
   }
 }
 
+constexpr size_t D_SMEM_MAX = 200 * 1024;
+
 // Warps per block and shared memory per warp for a table of `words`
 // doubles: as many warps as fit 200 KB, at most 4.
 void block_shape(int words, int* wpb, size_t* smem) {
   const size_t per = (size_t)words * sizeof(double);
-  int w = (int)std::max<size_t>(1, std::min<size_t>(4, (200u * 1024u) / std::max<size_t>(per, 1)));
+  int w = (int)std::max<size_t>(1, std::min<size_t>(4, D_SMEM_MAX / std::max<size_t>(per, 1)));
   *wpb = w;
   *smem = per * w;
 }
 
 template <typename K>
 void set_smem(K kernel, size_t smem) {
-  if (smem > 48 * 1024) PF_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  if (smem > 48 * 1024) allow_smem(kernel, std::max(smem, D_SMEM_MAX));  // (no table is larger than that)
 }
 
 DListArgs list_args(const PairData& pd, const TaskList& tl, int bc, int kc) {
