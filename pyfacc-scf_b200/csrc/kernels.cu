@@ -247,6 +247,24 @@ void launch_schwarz(const PairData& pd, int off[NCLASS + 1], double* q, cudaStre
   }
 }
 
+// Primitive records (three vectors each) in order of decreasing |K| (Shell's
+// sort, gaps (3^k - 1) / 2).
+__device__ void sort_records(double4* rec, int n) {
+  int gap = 1;
+  while (gap < n / 3) gap = 3 * gap + 1;
+  for (; gap > 0; gap /= 3)
+    for (int x = gap; x < n; ++x) {
+      const double4 r0 = rec[3 * (size_t)x], r1 = rec[3 * (size_t)x + 1], r2 = rec[3 * (size_t)x + 2];
+      const double kv = fabs(r0.z);
+      int y = x;
+      for (; y >= gap && fabs(rec[3 * (size_t)(y - gap)].z) < kv; y -= gap)
+        for (int v = 0; v < 3; ++v) rec[3 * (size_t)y + v] = rec[3 * (size_t)(y - gap) + v];
+      rec[3 * (size_t)y] = r0;
+      rec[3 * (size_t)y + 1] = r1;
+      rec[3 * (size_t)y + 2] = r2;
+    }
+}
+
 // Sorted copy of the pair records; primitive pairs with |K| < cut are left
 // out (their count was taken by build_pairs_kernel).
 __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, const int* __restrict__ new_ps,
@@ -263,8 +281,7 @@ __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, con
   const int old_ps = a.z, old_np = a.w;
   a.z = new_ps[i];
   // kept primitive pairs in order of decreasing |K| (so that a loop over
-  // them can stop at a cut); pairs with more than 64 primitive pairs keep
-  // the input order
+  // them can stop at a cut)
   int order[64];
   int nk = 0;
   for (int k = 0; k < old_np; ++k)
@@ -286,13 +303,23 @@ __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, con
   }
   const int nkept = nk;
   nk = 0;
+  const bool in_place = old_np > 64;
+  if (in_place) {  // more than the index list holds: the records themselves
+    double4* rec = opr + 3 * (size_t)a.z;
+    for (int k = 0; k < old_np; ++k) {
+      const double4* src = pr + 3 * (size_t)(old_ps + k);
+      if (fabs(src[0].z) < cut) continue;
+      for (int x = 0; x < 3; ++x) rec[3 * (size_t)nk + x] = src[x];
+      ++nk;
+    }
+    sort_records(rec, nkept);
+    nk = 0;
+  }
   // the product centres lie on the line AB: their box's diagonal
   double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, c2 = sqrt((double)FAR_C2);
-  for (int kk = 0; kk < (old_np <= 64 ? nkept : old_np); ++kk) {
-    const int k = (old_np <= 64) ? order[kk] : kk;
-    const double4* src = pr + 3 * (size_t)(old_ps + k);
+  for (int kk = 0; kk < nkept; ++kk) {
+    const double4* src = in_place ? opr + 3 * (size_t)(a.z + kk) : pr + 3 * (size_t)(old_ps + order[kk]);
     const double4 r0 = src[0];
-    if (fabs(r0.z) < cut) continue;
     double4* dst = opr + 3 * (size_t)(a.z + nk);
     double4 r1 = src[1], r2 = src[2];
     r1.w = r0.z * 0.94139626377671482 * sqrt(2.0 * r0.y);  // K sqrt(sqrt(pi)/2) / sqrt(p)
