@@ -236,6 +236,10 @@ int pyfacc_system_result(pyfacc_system *sys, pyfacc_result *res);
 int pyfacc_system_density_dev(pyfacc_system *sys, const double **P_dev);
 /* Number of kernel launches this library has issued in this process. */
 long long pyfacc_launch_count(void);
+/* ... of them launches of the kernels for long quartet lists (J/K and
+ * gradient): far == 0 the near kernels, else the far ones.  A launch captured
+ * into a graph counts once. */
+long long pyfacc_split_launch_count(int far);
 
 #define PYFACC_BOYS_MMAX 6
 /* Boys function F_m(x), m = 0..mmax (mmax <= PYFACC_BOYS_MMAX), for n arguments (device buffers;

@@ -16,6 +16,7 @@
 #include <mutex>
 #include <sstream>
 
+#include "pool.h"
 #include "system.h"
 
 namespace pyfacc {
@@ -127,13 +128,29 @@ Batch::Batch(const std::vector<BatchMolHost>& ms, const pyfacc_options& o) : opt
   if (mtot >= (1LL << 31) || (long long)nmol * ns_max * ns_max >= (1LL << 31))
     throw Error(PYFACC_ERR_INVALID, "batch too large: split it into several calls");
   const double t1 = wall_ms();
+  const long long mallocs = pool_mallocs();
   upload();
   const double t2 = wall_ms();
   build_pairs();
   const double t3 = wall_ms();
-  build_tasks();
+  // where memory is short, once more without the split kernels' records
+  auto or_undivided = [&](auto&& step) {
+    try {
+      step();
+    } catch (const Error&) {
+      if (!any_split) throw;
+      (void)cudaGetLastError();
+      drop_split();
+      step();
+    }
+  };
+  or_undivided([&] { build_tasks(); });
   const double t4 = wall_ms();
-  alloc();
+  or_undivided([&] { alloc(); });
+  if (any_split && !memory_left(mallocs)) {  // for the graphs and what the driver loads
+    drop_split();
+    pool_trim(device);
+  }
   timing.ms_setup = wall_ms() - t0;
   if (opt.verbose)
     std::fprintf(stderr, "pyfacc batch setup (ms): context %.2f  shells %.2f  pairs %.2f  tasks %.2f  matrices %.2f\n",
@@ -487,40 +504,14 @@ void Batch::choose_split() {
         nq += n;
         nfar += n * far[m];
       }
-      if (nq < BATCH_SPLIT_MIN || (bc == 2 && kc == 2) || pd.class_maxprim[bc] > SPLIT_MAXPRIM) continue;
+      if (nq < BATCH_SPLIT_MIN || !split_class(pd, bc, kc)) continue;
       split_len[bc][kc] = split_run((long long)(nq / BATCH_SPLIT_RUN_SHARE), pd.class_maxprim[bc] * pd.class_maxprim[kc], num_sms);
       split_halves[bc][kc] = nfar >= SPLIT_MIN_FAR && nfar >= BATCH_SPLIT_FAR_SHARE * nq;
       grad_split[bc][kc] = !split_halves[bc][kc] && nq >= BATCH_SPLIT_GRAD_MIN;
       any_split = true;
     }
   if (!any_split) return;
-  size_t nslots = 0;
-  KetTables kt;
-  for (int c = 0; c < NCLASS; ++c) {
-    kt.slot[c] = (int)nslots;
-    kt.class_off[c] = pd.class_off[c];
-    kt.maxprim[c] = pd.class_maxprim[c];
-    nslots += (size_t)(pd.class_off[c + 1] - pd.class_off[c]) * (pd.class_maxprim[c] + 1);
-  }
-  kt.class_off[NCLASS] = pd.class_off[NCLASS];
-  nslots = (nslots + 64) / 64 * 64;
-  const size_t test_bytes = ((size_t)pd.npair * 2 * sizeof(float4) + 255) / 256 * 256;
-  bool fits = nslots * KetTables::SLOT_BYTES <= BATCH_KET_TABLE_MAX;
-  if (fits) {
-    try {
-      kt_buf.ensure(test_bytes + nslots * KetTables::SLOT_BYTES);
-    } catch (const Error&) {
-      (void)cudaGetLastError();
-      fits = false;
-    }
-  }
-  if (!fits) {
-    drop_split();
-    return;
-  }
-  pd.test = kt_buf.as<float4>();
-  kt.carve(kt_buf.as<char>() + test_bytes, nslots);
-  pd.kt = kt;
+  if (!alloc_split_records(pd, kt_buf, BATCH_KET_TABLE_MAX)) drop_split();
 }
 
 // Back to the undivided kernels, whose lists every batch has.
@@ -697,14 +688,7 @@ void Batch::alloc() {
   const size_t o_grad = carve(3 * (size_t)natoms_tot * sizeof(double));
   const size_t o_act = carve(sizeof(StepReport));
   const size_t o_ctl = carve(sizeof(BatchScfCtl));
-  try {
-    mats.ensure(o);
-  } catch (const Error&) {  // no memory left: without the split kernels' records?
-    if (!any_split) throw;
-    (void)cudaGetLastError();
-    drop_split();
-    mats.ensure(o);
-  }
+  mats.ensure(o);
   char* b = mats.as<char>();
   double* mp[nmat];
   for (size_t k = 0; k < nmat; ++k) mp[k] = reinterpret_cast<double*>(b + om[k]);
@@ -799,7 +783,7 @@ void Batch::fock_build(bool mixed_lists, double thresh, unsigned long long* stat
       // (single-precision lists: the classes alternate between the streams)
       const bool swap = fork && (nth & 1);
       auto build = [&](int part, bool fp32, cudaStream_t s) {
-        if (jk_splits(pd, split_tasks[bc][kc][part], bc, kc))
+        if (jk_splits(pd, split_tasks[bc][kc][part]))
           launch_jk_split(pd, split_tasks[bc][kc][part], bc, kc, fp32, 1, a, num_sms,
                           jk_next + 2 * (2 * qclass_index(bc, kc) + (fp32 ? 1 : 0)), s == stream ? s32 : stream, s);
         else
@@ -1188,7 +1172,7 @@ void Batch::gradient_run() {
   for (int bc = NCLASS - 1; bc >= 0; --bc)
     for (int kc = bc; kc >= 0; --kc, ++nth) {
       auto derive = [&](int part, bool fp32, cudaStream_t s) {
-        if (grad_split[bc][kc] && jk_splits(pd, split_tasks[bc][kc][part], bc, kc))
+        if (grad_split[bc][kc] && jk_splits(pd, split_tasks[bc][kc][part]))
           launch_grad_split(pd, split_tasks[bc][kc][part], bc, kc, fp32, g2, num_sms,
                             jk_next + 2 * (2 * qclass_index(bc, kc) + (fp32 ? 1 : 0)), s, s);
         else

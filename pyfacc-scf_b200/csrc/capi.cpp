@@ -427,6 +427,7 @@ int pyfacc_system_result(pyfacc_system* sys, pyfacc_result* res) {
 }
 
 long long pyfacc_launch_count(void) { return pyfacc::launch_count(); }
+long long pyfacc_split_launch_count(int far) { return pyfacc::split_launch_count(far != 0); }
 
 int pyfacc_system_density_dev(pyfacc_system* sys, const double** P_dev) {
   if (!sys || !P_dev) return PYFACC_ERR_INVALID;

@@ -403,27 +403,12 @@ void System::build_pairs() {
   }
   pd.npair = (int)perm.size();
   pd.nprim = nprim_new;
-  // slots of the transposed records (s/p classes)
-  size_t nslots = 0;
-  for (int c = 0; c < NCLASS; ++c) {
-    pd.kt.slot[c] = (int)nslots;
-    pd.kt.class_off[c] = pd.class_off[c];
-    pd.kt.maxprim[c] = pd.class_maxprim[c];
-    nslots += (size_t)(pd.class_off[c + 1] - pd.class_off[c]) * (pd.class_maxprim[c] + 1);
-  }
-  pd.kt.class_off[NCLASS] = pd.class_off[NCLASS];
-  nslots = (nslots + 64) / 64 * 64;
-  // (rows are as many as the deepest contraction has: without the tables, and
-  // with the undivided kernels, where that is out of proportion)
-  const bool tables = nslots * KetTables::SLOT_BYTES <= KET_TABLE_MAX;
   // final records
   o = 0;
   const size_t f_i0 = carve(pd.npair * sizeof(int4)), f_i1 = carve(pd.npair * sizeof(int4)),
                f_i2 = carve(pd.npair * sizeof(int4)), f_g = carve(pd.npair * sizeof(double4)),
                f_pr = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(double4)),
-               f_prf = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(float4)),
-               f_test = carve(pd.npair * 2 * sizeof(float4)),
-               f_kt = carve(tables ? nslots * KetTables::SLOT_BYTES : 0);
+               f_prf = carve((size_t)std::max(nprim_new, 1) * 3 * sizeof(float4));
   pd.buf.ensure(std::max<size_t>(o, 256));
   char* pb = pd.buf.as<char>();
   pd.info0 = reinterpret_cast<int4*>(pb + f_i0);
@@ -432,9 +417,15 @@ void System::build_pairs() {
   pd.geom = reinterpret_cast<double4*>(pb + f_g);
   pd.prim = reinterpret_cast<double4*>(pb + f_pr);
   pd.primf = reinterpret_cast<float4*>(pb + f_prf);
-  if (tables) pd.kt.carve(pb + f_kt, nslots);
-  else pd.kt = KetTables();
-  pd.test = reinterpret_cast<float4*>(pb + f_test);
+  tq[4] = clk::now();
+  build_tasks();
+  tq[5] = clk::now();
+  drop_split();
+  if (any_split) {
+    const long long mallocs = pool_mallocs();
+    any_split = alloc_split_records(pd, kt_buf, KET_TABLE_MAX);
+    leave_room(mallocs);
+  }
   if (pd.npair > 0) {
     PF_CUDA(cudaMemcpyAsync(d_perm, perm.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
     PF_CUDA(cudaMemcpyAsync(d_ps, new_ps.data(), pd.npair * sizeof(int), cudaMemcpyHostToDevice, stream));
@@ -442,14 +433,88 @@ void System::build_pairs() {
                         pd.info0, pd.info1, pd.info2, pd.geom, pd.prim, pd.primf, pd.test, pd.kt, stream);
   }
   PF_CUDA(cudaStreamSynchronize(stream));
-  tq[4] = clk::now();
-  build_tasks();
   if (opt.verbose) {
-    PF_CUDA(cudaStreamSynchronize(stream));
-    tq[5] = clk::now();
+    tq[6] = clk::now();
     auto ms = [](clk::time_point a, clk::time_point b) { return std::chrono::duration<double, std::milli>(b - a).count(); };
-    std::fprintf(stderr, "pyfacc pairs (ms): host lists %.3f  scratch %.3f  records+Q %.3f  sort+gather %.3f  tasks %.3f\n",
-                 ms(tq[0], tq[1]), ms(tq[1], tq[2]), ms(tq[2], tq[3]), ms(tq[3], tq[4]), ms(tq[4], tq[5]));
+    std::fprintf(stderr, "pyfacc pairs (ms): host lists %.3f  scratch %.3f  records+Q %.3f  sort %.3f  tasks %.3f  gather %.3f\n",
+                 ms(tq[0], tq[1]), ms(tq[1], tq[2]), ms(tq[2], tq[3]), ms(tq[3], tq[4]), ms(tq[4], tq[5]),
+                 ms(tq[5], tq[6]));
+  }
+}
+
+// The split kernels' records: the candidate tests and the transposed tables,
+// one row per primitive pair of the deepest contraction.  False, with pd and
+// buf without them, where they would take more than max_bytes (rows out of
+// proportion) or memory is short: the lists that the undivided kernels take
+// are always there.
+bool alloc_split_records(PairData& pd, DeviceBuf& buf, size_t max_bytes) {
+  size_t nslots = 0;
+  KetTables kt;
+  for (int c = 0; c < NCLASS; ++c) {
+    kt.slot[c] = (int)nslots;
+    kt.class_off[c] = pd.class_off[c];
+    kt.maxprim[c] = pd.class_maxprim[c];
+    nslots += (size_t)(pd.class_off[c + 1] - pd.class_off[c]) * (pd.class_maxprim[c] + 1);
+  }
+  kt.class_off[NCLASS] = pd.class_off[NCLASS];
+  nslots = (nslots + 64) / 64 * 64;
+  const size_t test_bytes = ((size_t)pd.npair * 2 * sizeof(float4) + 255) / 256 * 256;
+  bool fits = nslots * KetTables::SLOT_BYTES <= max_bytes;
+  if (fits) {
+    try {
+      buf.ensure(test_bytes + nslots * KetTables::SLOT_BYTES);
+    } catch (const Error&) {
+      (void)cudaGetLastError();
+      fits = false;
+    }
+  }
+  if (!fits) {
+    buf.release();
+    return false;
+  }
+  pd.test = buf.as<float4>();
+  kt.carve(buf.as<char>() + test_bytes, nslots);
+  pd.kt = kt;
+  return true;
+}
+
+// The records are not worth the memory that graphs, kernels' stacks and the
+// libraries ask the driver for later.
+// Asking costs half a millisecond and more: only after an allocation that the
+// pool did not serve.
+bool memory_left(long long mallocs) {
+  if (pool_mallocs() == mallocs) return true;
+  size_t left = 0, total = 0;
+  PF_CUDA(cudaMemGetInfo(&left, &total));
+  return left >= ((size_t)512 << 20);
+}
+
+// To the undivided kernels; the buffer stays for the next geometry.
+void System::drop_split() {
+  pd.kt = KetTables();
+  pd.test = nullptr;
+}
+
+void System::leave_room(long long mallocs) {
+  if (!pd.kt.xy || memory_left(mallocs)) return;
+  drop_split();
+  any_split = false;
+  kt_buf.release();
+  pool_trim(device);
+}
+
+// b.ensure(bytes); where memory is short, once more without the split
+// kernels' records.
+void System::ensure_matrices(DeviceBuf& b, size_t bytes) {
+  try {
+    b.ensure(bytes);
+  } catch (const Error&) {
+    if (!pd.kt.xy) throw;
+    (void)cudaGetLastError();
+    drop_split();
+    any_split = false;
+    kt_buf.release();
+    b.ensure(bytes);
   }
 }
 
@@ -528,7 +593,9 @@ void System::build_tasks() {
         }
         toff[nb] = ntask;
         if (prec == 0) quartets_total += quart;
-        const int chunk = bc >= NCLASS ? 0 : split_chunk(quart, far_share, pd.class_maxprim[bc] * pd.class_maxprim[kc], num_sms);
+        const int chunk = !split_class(pd, bc, kc)
+                              ? 0
+                              : split_chunk(quart, far_share, pd.class_maxprim[bc] * pd.class_maxprim[kc], num_sms);
         TaskList& tl = tasks[bc][kc][prec];
         tl.width = task_width;
         tl.nbra = nb;
@@ -627,7 +694,8 @@ void System::build_tasks() {
 void System::alloc_matrices() {
   const size_t n2 = (size_t)nbf * nbf;
   const int nmat = 31 + 4 * std::max(opt.diis_size, 1);
-  mats.ensure(nmat * n2 * sizeof(double) + 96 * sizeof(double) + ns * ns * sizeof(float) + 1024);
+  const long long mallocs = pool_mallocs();
+  ensure_matrices(mats, nmat * n2 * sizeof(double) + 96 * sizeof(double) + ns * ns * sizeof(float) + 1024);
   double* m = mats.as<double>();
   auto take = [&]() { double* r = m; m += n2; return r; };
   S = take(); T = take(); Vm = take(); H = take(); X = take();
@@ -647,9 +715,9 @@ void System::alloc_matrices() {
   pstate = m; m += 48;  // purification graph state (24 doubles used)
   dmax = reinterpret_cast<float*>(m);
   const size_t red_bytes = (size_t)RED_BLOCKS * (nd + 3) * sizeof(double);
-  small_buf.ensure(2 * nbf * sizeof(double) + 256 + sizeof(JkStats) + 256 + 64 * sizeof(double*) + 256 +
-                   3 * natoms * sizeof(double) + 256 + 256 + red_bytes + 256 + nbf * sizeof(double) + 256 + 256 +
-                   SPLIT_COUNTERS * sizeof(int) + 256);
+  ensure_matrices(small_buf, 2 * nbf * sizeof(double) + 256 + sizeof(JkStats) + 256 + 64 * sizeof(double*) + 256 +
+                                 3 * natoms * sizeof(double) + 256 + 256 + red_bytes + 256 + nbf * sizeof(double) +
+                                 256 + 256 + SPLIT_COUNTERS * sizeof(int) + 256);
   {
     char* b = small_buf.as<char>();
     size_t o = 0;
@@ -664,6 +732,7 @@ void System::alloc_matrices() {
     pmin_dev = reinterpret_cast<double*>(take(sizeof(double)));
     jk_next = reinterpret_cast<int*>(take(SPLIT_COUNTERS * sizeof(int)));
   }
+  leave_room(mallocs);
   {
     const std::vector<double> occ = atomic_occupations();
     PF_CUDA(cudaMemcpy(occ_dev, occ.data(), nbf * sizeof(double), cudaMemcpyHostToDevice));
@@ -671,7 +740,7 @@ void System::alloc_matrices() {
   int lwork = 0;
   PF_CUSOLVER(cusolverDnDsyevd_bufferSize(cusolver, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, nbf, W1, nbf,
                                           eps_dev, &lwork));
-  syev_work.ensure(std::max<size_t>((size_t)lwork * sizeof(double), 256));
+  ensure_matrices(syev_work, std::max<size_t>((size_t)lwork * sizeof(double), 256));
   syev_lwork = lwork;
 }
 

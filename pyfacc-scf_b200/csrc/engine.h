@@ -204,7 +204,7 @@ struct KetTables {
   }
 };
 
-constexpr size_t KET_TABLE_MAX = (size_t)16 << 30;  // bytes, one molecule (C100H202: 0.17 GB)
+constexpr size_t KET_TABLE_MAX = (size_t)16 << 30;  // bytes, one molecule (C100H202: 0.17 GB; nothing where no list is split)
 
 // Packed pair data of one molecule or of a batch (every pair stores the
 // offset and leading dimension of its molecule's matrices).
@@ -250,6 +250,8 @@ double digest_flops(int qclass, int nk);
 // ------------------------------------------------------------- launchers
 // Every kernel launch of this library is counted (pyfacc_launch_count).
 void count_launch();
+void count_split_launch(bool far);  // one of the split kernels, counted by half as well
+long long split_launch_count(bool far);
 void count_launches(long long n);  // kernels of a replayed CUDA graph
 long long launch_count();
 void ensure_boys_tables(int device);
@@ -316,7 +318,10 @@ constexpr double FAR_DISTANCE = 16.0;     // bohr: quartets of diffuse pairs tha
 constexpr int SPLIT_COUNTERS = 4 * NQCLASS;  // task counters of a build: two kernels per class and precision
 int split_run(long long nquartets, int prim_quartets, int num_sms);
 int split_chunk(long long nquartets, double far_share, int prim_quartets, int num_sms);
-bool jk_splits(const PairData& pd, const TaskList& tl, int bra_class, int ket_class);
+bool split_class(const PairData& pd, int bra_class, int ket_class);  // classes that they cover
+bool jk_splits(const PairData& pd, const TaskList& tl);
+bool alloc_split_records(PairData& pd, DeviceBuf& buf, size_t max_bytes);
+bool memory_left(long long mallocs);  // enough of the device's memory beside the engine's (mallocs: pool_mallocs before)
 void launch_jk_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32, int nk,
                      const JkArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
 // Bound on a quartet's density products, relative to the threshold, below

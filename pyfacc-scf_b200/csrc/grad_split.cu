@@ -314,7 +314,7 @@ void launch_one(int num_sms, cudaStream_t s, GradSplitArgs k) {
       1LL, std::min((k.l.ntasks + 3LL) / 4, (long long)num_sms * grad_min_blocks(LA + LB + LC + LD)));
   grad_split_kernel<R, LA, LB, LC, LD, FAR><<<blocks, 128, smem, s>>>(k);
   PF_CUDA(cudaGetLastError());
-  count_launch();
+  count_split_launch(FAR);
 }
 
 template <typename R, int LA, int LB, int LC, int LD>

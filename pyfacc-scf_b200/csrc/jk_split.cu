@@ -464,7 +464,7 @@ void launch_one(int blocks, cudaStream_t s, SplitArgs k) {
                std::max(STAGE_MAX_BYTES, 4 * 2 * Stage<R, (LA + LB > 0), FAR>::bytes(SPLIT_MAXPRIM)));
   jk_split_kernel<R, LA, LB, LC, LD, NK, FAR><<<blocks, 128, smem, s>>>(k);
   PF_CUDA(cudaGetLastError());
-  count_launch();
+  count_split_launch(FAR);
 }
 
 template <typename R, int LA, int LB, int LC, int LD>
@@ -513,11 +513,13 @@ int split_run(long long nquartets, int prim_quartets, int num_sms) {
   return c;
 }
 
-bool jk_splits(const PairData& pd, const TaskList& tl, int bc, int kc) {
-  // (pp|pp) keeps the undivided kernel: few quartets, and its time is the
-  // recursion's, not the Boys function's
-  return pd.kt.xy && tl.chunk > 0 && bc < NCLASS && !(bc == 2 && kc == 2) && pd.class_maxprim[bc] <= SPLIT_MAXPRIM;
+// (pp|pp) keeps the undivided kernel: few quartets, and its time is the
+// recursion's, not the Boys function's.
+bool split_class(const PairData& pd, int bc, int kc) {
+  return bc < NCLASS && !(bc == 2 && kc == 2) && pd.class_maxprim[bc] <= SPLIT_MAXPRIM;
 }
+
+bool jk_splits(const PairData& pd, const TaskList& tl) { return pd.kt.xy && tl.chunk > 0; }
 
 void launch_jk_split(const PairData& pd, const TaskList& tl, int bc, int kc, bool fp32, int nk, const JkArgs& a,
                      int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near) {

@@ -27,6 +27,12 @@ namespace pyfacc {
 
 static std::atomic<long long> g_launches{0};
 void count_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
+static std::atomic<long long> g_split_launches[2] = {};
+void count_split_launch(bool far) {
+  count_launch();
+  g_split_launches[far].fetch_add(1, std::memory_order_relaxed);
+}
+long long split_launch_count(bool far) { return g_split_launches[far].load(std::memory_order_relaxed); }
 void count_launches(long long n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
@@ -899,7 +905,7 @@ void launch_dyn_tasks(const PairData& pd, const float* dmax, int ns, double thre
         L.nket = pd.class_off[kc + 1] - pd.class_off[kc];
         L.same = bc == kc;
         L.part = part;
-        L.width = part == 1 && tl.far >= min_far && jk_splits(pd, tl, bc, kc) ? tl.chunk : tl.width;
+        L.width = part == 1 && tl.far >= min_far && jk_splits(pd, tl) ? tl.chunk : tl.width;
         L.task_off = tl.task_off;
         L.ket_lo = tl.ket_lo;
         L.ket_hi = tl.ket_hi;

@@ -24,6 +24,7 @@ std::map<int, std::vector<GpuContext>> g_free_ctx;
 std::map<std::string, std::shared_ptr<const std::vector<std::string>>> g_basis_text;
 constexpr size_t kMaxCachedBytesPerDevice = size_t(8) << 30;
 std::map<int, size_t> g_cached_bytes;
+thread_local long long t_mallocs = 0;
 }  // namespace
 
 void* pool_alloc(size_t bytes, size_t* got) {
@@ -42,6 +43,7 @@ void* pool_alloc(size_t bytes, size_t* got) {
       return p;
     }
   }
+  ++t_mallocs;
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e != cudaSuccess) {
@@ -53,6 +55,8 @@ void* pool_alloc(size_t bytes, size_t* got) {
   *got = bytes;
   return p;
 }
+
+long long pool_mallocs() { return t_mallocs; }
 
 void pool_free(void* p, size_t bytes) {
   if (!p) return;

@@ -15,6 +15,7 @@ namespace pyfacc {
 void* pool_alloc(size_t bytes, size_t* got);
 void pool_free(void* p, size_t bytes);
 void pool_trim(int device);
+long long pool_mallocs();  // cudaMallocs behind this thread's requests so far
 
 // One stream with its cuBLAS and cuSOLVER handles and two timing events.
 struct GpuContext {

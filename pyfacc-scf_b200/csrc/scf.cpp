@@ -98,7 +98,7 @@ void System::jk(const double* Dj, int nk, const double* const* Dk, double* Jo, d
       // long lists go to the split kernels, whose near half takes the stream
       // given here and whose far half the other one
       auto build = [&](const TaskList& tl, bool fp32, cudaStream_t s) {
-        if (jk_splits(pd, tl, bc, kc))
+        if (jk_splits(pd, tl))
           launch_jk_split(pd, tl, bc, kc, fp32, nk, a, num_sms, jk_next + 2 * (2 * qc + (fp32 ? 1 : 0)),
                           s == stream ? ctx.side : stream, s);
         else
@@ -872,7 +872,7 @@ void System::gradient(double* g_host) {
     for (int kc = bc; kc >= 0; --kc, ++nth) {
       const int qc = (bc == 0) ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
       auto derive = [&](const TaskList& tl, bool fp32, cudaStream_t s) {
-        if ((!fp32 || tl.far >= GRAD_SPLIT_FP32_FAR) && jk_splits(pd, tl, bc, kc))
+        if ((!fp32 || tl.far >= GRAD_SPLIT_FP32_FAR) && jk_splits(pd, tl))
           launch_grad_split(pd, tl, bc, kc, fp32, g2, num_sms, jk_next + 2 * (2 * qc + (fp32 ? 1 : 0)),
                             s == stream ? ctx.side : stream, s);
         else

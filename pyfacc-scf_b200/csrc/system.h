@@ -63,6 +63,7 @@ struct System {
   long long quartets_total = 0;
   DynTaskSet dyn;          // per-build task lists (mixed precision)
   DeviceBuf dyn_buf;
+  DeviceBuf kt_buf;  // the split kernels' records, where a list goes to them
 
   DeviceBuf mats;
   double *S = nullptr, *T = nullptr, *Vm = nullptr, *H = nullptr, *X = nullptr, *Xt = nullptr;
@@ -118,6 +119,9 @@ struct System {
   void nuclear_repulsion_gradient(double* g) const;
   void upload_shells();
   void build_pairs();
+  void drop_split();
+  void leave_room(long long mallocs);
+  void ensure_matrices(DeviceBuf& b, size_t bytes);
   void build_tasks();
   void alloc_matrices();
   void release_extra();
