@@ -33,7 +33,8 @@ template <typename R> __host__ __device__ constexpr float far_tmin(int L) {
 // in tau: the pair stores it at FAR_TAU0 and FAR_TAU1, and the chord bounds
 // it in between.  FAR_C2 is twice the 1/p of diffuse STO-nG pairs, where the
 // tangent is tight.  Written in rounding intrinsics so that the two kernels
-// that share a list decide alike; the margin covers the float coordinates.
+// that share a list decide alike; E covers the centres' rounding to float (of
+// molecules far from the origin), the margin that of the test itself.
 constexpr float FAR_C2 = 5.0f, FAR_TAU0 = 4.0f, FAR_TAU1 = 7.2f;
 
 template <typename R, int L> __device__ __forceinline__ float far_extent(float e0, float e1) {

@@ -394,11 +394,13 @@ __global__ void gather_pairs_kernel(int npair, const int* __restrict__ perm, con
     if (nk == 0) lo[0] = lo[1] = lo[2] = hi[0] = hi[1] = hi[2] = 0.0;
     const double rx = 0.5 * (hi[0] - lo[0]), ry = 0.5 * (hi[1] - lo[1]), rz = 0.5 * (hi[2] - lo[2]);
     const double cx = lo[0] + rx, cy = lo[1] + ry, cz = lo[2] + rz;
-    double e0 = 0.0, e1 = 0.0;
+    // the test takes the centre in float: what that moves it by belongs to r
+    const double rf = 6.1e-8 * (fabs(cx) + fabs(cy) + fabs(cz));
+    double e0 = rf, e1 = rf;
     for (int k = 0; k < nk; ++k) {
       const double4 r0 = opr[3 * (size_t)(a.z + k)], r1 = opr[3 * (size_t)(a.z + k) + 1];
       const double dx = r1.x - cx, dy = r1.y - cy, dz = r1.z - cz;
-      const double r = sqrt(dx * dx + dy * dy + dz * dz), w = r0.y / c2 + 0.25 * c2;  // s/(2c) + c/4, s = 2 r0.y
+      const double r = sqrt(dx * dx + dy * dy + dz * dz) + rf, w = r0.y / c2 + 0.25 * c2;  // s/(2c) + c/4, s = 2 r0.y
       e0 = fmax(e0, r + FAR_TAU0 * w);
       e1 = fmax(e1, r + FAR_TAU1 * w);
     }
