@@ -169,8 +169,9 @@ __global__ void __launch_bounds__(128, grad_min_blocks(LA + LB + LC + LD)) grad_
                   dad = __ldg(dmx + sa * ld + sd), dbc = __ldg(dmx + sb * ld + sc), dbd = __ldg(dmx + sb * ld + sd);
       const float dm = fmaxf(fmaxf(2.0f * fmaxf(dab, dcd), fmaxf(dac, dad)), fmaxf(dbc, dbd));
       const float gm = dab * dcd + dac * dbd + dad * dbc, qq = bt.y * kt.y;
-      if (!(qq * dm >= (float)A.thresh) || !(qq * gm >= (float)(GRAD_SPLIT_REL * A.thresh))) return -1;
-      if (A.prim_thresh > 0.0) cut = __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
+      const float thr = TEST_SLACK * (float)A.thresh;
+      if (!(qq * dm >= thr) || !(qq * gm >= (float)GRAD_SPLIT_REL * thr)) return -1;
+      if (A.prim_thresh > 0.0) cut = TEST_SLACK * __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
     }
     return 0;
   };

@@ -312,9 +312,10 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
       const float dk = dmax_exchange(dmx, A.ns_ld, sa, sb, sc, sd);
       const float dm = fmaxf(2.0f * fmaxf(__ldg(dmx + sa * A.ns_ld + sb), __ldg(dmx + sc * A.ns_ld + sd)), dk);
       const float qq = bt.y * kt.y;
-      if (!(qq * dm >= (float)A.thresh)) return -1;
-      if (FAR && !(qq * dk >= (float)A.thresh)) to = 0;
-      cut = __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
+      const float thr = TEST_SLACK * (float)A.thresh;
+      if (!(qq * dm >= thr)) return -1;
+      if (FAR && !(qq * dk >= thr)) to = 0;
+      cut = TEST_SLACK * __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
     }
     return to;
   };

@@ -60,6 +60,12 @@ inline SplitLists split_lists(const PairData& pd, const TaskList& tl, int bc, in
   return k;
 }
 
+// The tests are made in float from float bounds (five roundings of 2^-24 at
+// most and __fdividef's two units in the last place): thresholds and cuts are
+// lowered by this much, so that no quartet and no primitive goes that the same
+// test in double would keep.
+constexpr float TEST_SLACK = 0.999999f;
+
 constexpr int QUEUE = 64;  // a ring: up to 31 left over plus 32 new quartets
 constexpr int MAXSLOT = 8;
 
