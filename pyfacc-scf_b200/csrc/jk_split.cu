@@ -11,8 +11,8 @@
 // branches (the far half none of the Boys function's).  The far half keeps
 // quartets that only J needs apart from those that K needs too: the exchange
 // part of the digestion, four gathers and four atomics per quartet and
-// density, is paid only where Q_ab Q_cd max |D_ac, D_ad, D_bc, D_bd| reaches
-// the screening threshold.  One kernel with three rings did the candidate
+// density, is left out where Q_ab Q_cd max |D_ac, D_ad, D_bc, D_bd| stays below
+// EXCHANGE_REL of the screening threshold.  One kernel with three rings did the candidate
 // tests once, but needed the near half's registers throughout and was 5%
 // slower.
 //
@@ -36,6 +36,15 @@
 namespace pyfacc {
 
 namespace {
+
+// What a far quartet that J needs may still add to K without being digested,
+// relative to the screening threshold.  At 1 (the threshold of the quartets
+// themselves) K of an SCF density moved by 4e-13 to 9e-13 of its norm against
+// the kernels that digest everything, at 1e-3 by no more than the sums' own
+// rounding (1e-15 to 9e-15, the same as without this test: C40H82, C100H202,
+// gly30, C30H61).  FP64 build of C100H202: 11.08 ms at 1, 11.28 here, 11.54
+// without; FP32 7.04, 7.23, 7.76.
+constexpr float EXCHANGE_REL = 1e-3f;
 
 struct SplitArgs {
   SplitLists l;
@@ -314,7 +323,7 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
       const float qq = bt.y * kt.y;
       const float thr = TEST_SLACK * (float)A.thresh;
       if (!(qq * dm >= thr)) return -1;
-      if (FAR && !(qq * dk >= thr)) to = 0;
+      if (FAR && !(qq * dk >= EXCHANGE_REL * thr)) to = 0;
       cut = TEST_SLACK * __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
     }
     return to;
