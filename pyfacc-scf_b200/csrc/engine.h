@@ -324,9 +324,6 @@ bool alloc_split_records(PairData& pd, DeviceBuf& buf, size_t max_bytes);
 bool memory_left(long long mallocs);  // enough of the device's memory beside the engine's (mallocs: pool_mallocs before)
 void launch_jk_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32, int nk,
                      const JkArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
-// Bound on a quartet's density products, relative to the threshold, below
-// which the split gradient leaves it out.
-constexpr double GRAD_SPLIT_REL = 1e-2;
 // Far quartets of a list (estimate) from which its FP32 derivative quartets go
 // to the split kernels: C20H42, 4e5 to 5e5 a list, 1.19 ms undivided, 1.28
 // divided; C40H82, (ss|ss) and (ps|ss) 1.5e6, 4.1 -> 3.6 ms.

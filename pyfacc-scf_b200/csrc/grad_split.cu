@@ -1,13 +1,10 @@
 // Two-electron nuclear gradient of long quartet lists, far and near quartets
 // apart: the walk, the queues and the far limit of jk_split.cu, the derivatives
-// (grad_md.cuh) and the density products of grad2e_kernel (kernels.cu).  A quartet is left out when Q_ab Q_cd times the bound on its
-// density products, |D_ab D_cd| + |D_ac D_bd| + |D_ad D_bc|, stays below
-// GRAD_SPLIT_REL of the screening threshold: the undivided kernels test one
-// density factor, the largest, and evaluate quartets whose products are orders
-// of magnitude smaller, max |dg| 1e-11 Ha/bohr.  FP64 gradients of C40H82 10.2
-// -> 8.6 ms, C100H202 60 -> 52 ms, and with the Hermite derivatives 5.7 and 28.6;
-// FP32 lists (two bra primitives at a time in packed pairs) only with the
-// latter: mixed gradient of gly30 18.9 -> 15.2 ms, C100H202 29.0 -> 17.5.
+// (grad_md.cuh), the screening and the density products of grad2e_kernel
+// (kernels.cu).  FP64 gradients of C40H82 10.2 -> 8.7 ms, C100H202 60 -> 53 ms,
+// and with the Hermite derivatives 5.9 and 29.5; FP32 lists (two bra primitives
+// at a time in packed pairs) only with the latter: mixed gradient of gly30 18.9
+// -> 15.6 ms, C100H202 29.0 -> 18.2.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -163,14 +160,9 @@ __global__ void __launch_bounds__(128, grad_min_blocks(LA + LB + LC + LD)) grad_
       return -1;
     if (A.dmax) {
       const float* dmx = A.dmax + L.info2[bp].w;
-      const int ld = A.ns_ld, sa = __float_as_int(bt.z), sb = __float_as_int(bt.w), sc = __float_as_int(kt.z),
-                sd = __float_as_int(kt.w);
-      const float dab = __ldg(dmx + sa * ld + sb), dcd = __ldg(dmx + sc * ld + sd), dac = __ldg(dmx + sa * ld + sc),
-                  dad = __ldg(dmx + sa * ld + sd), dbc = __ldg(dmx + sb * ld + sc), dbd = __ldg(dmx + sb * ld + sd);
-      const float dm = fmaxf(fmaxf(2.0f * fmaxf(dab, dcd), fmaxf(dac, dad)), fmaxf(dbc, dbd));
-      const float gm = dab * dcd + dac * dbd + dad * dbc, qq = bt.y * kt.y;
-      const float thr = TEST_SLACK * (float)A.thresh;
-      if (!(qq * dm >= thr) || !(qq * gm >= (float)GRAD_SPLIT_REL * thr)) return -1;
+      const float dm = dmax_bound(dmx, A.ns_ld, __float_as_int(bt.z), __float_as_int(bt.w), __float_as_int(kt.z),
+                                  __float_as_int(kt.w));
+      if (!(bt.y * kt.y * dm >= TEST_SLACK * (float)A.thresh)) return -1;
       if (A.prim_thresh > 0.0) cut = TEST_SLACK * __fdividef((float)A.prim_thresh, fmaxf(dm, 1e-30f));
     }
     return 0;

@@ -827,8 +827,7 @@ void System::gradient(double* g_host) {
   g1.natoms_total = natoms;
   // one-electron terms once (shard 0); the two-electron term is sharded
   if (opt.shard_count <= 1 || opt.shard_rank == 0) launch_grad1e(shd, n1e, pairs1e, g1, num_sms, stream);
-  // the split kernels bound density products, spin by spin for an open shell
-  launch_dmax(ns, bf_off_dev, nfun_dev, nbf, Pt, uhf ? P[0] : nullptr, uhf ? P[1] : nullptr, dmax, stream);
+  launch_dmax(ns, bf_off_dev, nfun_dev, nbf, Pt, nullptr, nullptr, dmax, stream);
   GradArgs g2;
   g2.Pt = Pt;
   g2.Pa = uhf ? Ps[0] : Pt;
