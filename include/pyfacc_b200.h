@@ -246,6 +246,11 @@ long long pyfacc_split_launch_count(int far);
  * out_dev[i*(mmax+1)+m]).  mode: PYFACC_BOYS_*; fp32 != 0 uses the
  * single-precision path of mixed mode. */
 int pyfacc_boys_dev(int mode, int fp32, int mmax, int n, const double *x_dev, double *out_dev);
+/* The functions of the kernels for long quartet lists, L <= 4 (tests):
+ * out_dev[i*(L+1)+m] = what 0: F_m(x) from their table, 1: F_m(x) in the far
+ * limit (x beyond its bound, 36 + 3L in FP64 and 17 + 3L in FP32), and with
+ * L = 0: 2: 1/sqrt(x), 3: exp(-x) (FP64 only). */
+int pyfacc_split_values_dev(int what, int fp32, int L, int n, const double *x_dev, double *out_dev);
 
 /* Dense FP64 products on the tensor cores (the kernels of the SCF step),
  * row-major device matrices with leading dimensions m (A: m x k, or k x m

@@ -8,6 +8,7 @@
 
 #include "boys_rows.cuh"
 #include "engine.h"
+#include "split.cuh"
 
 namespace pyfacc {
 
@@ -62,7 +63,56 @@ void row_coefficients(int L, long double c, long double r, int n, long double* o
   for (int k = 0; k < n; ++k, s *= r) out[k] /= s;
 }
 
+// One function value per thread, for the tests: the table's F_0 .. F_L, the
+// far limit's (far_setup at |PQ|^2 = T with rho = 1), or far_rsqrt and br_expm.
+template <int L, bool FP32> __device__ void split_values(int what, double x, double* out) {
+  if (what == 0) {
+    if constexpr (FP32) {
+      F2 F[L + 1];
+      boys_rows<L>(g_br32[L], F2((float)x), F);
+      for (int m = 0; m <= L; ++m) out[m] = F[m].v.x;
+    } else {
+      boys_rows<L>(g_br64[L], x, out);
+    }
+  } else if (what == 1) {
+    using T = typename std::conditional<FP32, F2, double>::type;
+    PrimGeo<T> g;
+    const T PQ[3] = {T(typename Scalar<T>::R(sqrt(x))), T(0.0f), T(0.0f)};
+    far_setup<T, L>(PQ, T(typename Scalar<T>::R(0.88622692545275801365)), T(0.5f), T(0.5f), g);
+    for (int m = 0; m <= L; ++m) {
+      if constexpr (FP32) out[m] = g.I[m].v.x;
+      else out[m] = g.I[m];
+    }
+  } else if (what == 2) {
+    if constexpr (FP32) out[0] = far_rsqrt((float)x);
+    else out[0] = far_rsqrt(x);
+  } else {
+    out[0] = br_expm(x);
+  }
+}
+template <bool FP32>
+__global__ void split_values_kernel(int what, int L, int n, const double* __restrict__ x, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  double* o = out + (size_t)i * (L + 1);
+  switch (L) {
+    case 0: split_values<0, FP32>(what, x[i], o); break;
+    case 1: split_values<1, FP32>(what, x[i], o); break;
+    case 2: split_values<2, FP32>(what, x[i], o); break;
+    case 3: split_values<3, FP32>(what, x[i], o); break;
+    default: split_values<4, FP32>(what, x[i], o); break;
+  }
+}
+
 }  // namespace
+
+void launch_split_values(int what, bool fp32, int L, int n, const double* x, double* out, cudaStream_t s) {
+  if (n <= 0) return;
+  if (fp32) split_values_kernel<true><<<(n + 127) / 128, 128, 0, s>>>(what, L, n, x, out);
+  else split_values_kernel<false><<<(n + 127) / 128, 128, 0, s>>>(what, L, n, x, out);
+  PF_CUDA(cudaGetLastError());
+  count_launch();
+}
 
 // The tables of the current device (called once per device, under the lock of
 // ensure_boys_tables).

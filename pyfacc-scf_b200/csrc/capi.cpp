@@ -446,6 +446,19 @@ int pyfacc_boys_dev(int mode, int fp32, int mmax, int n, const double* x_dev, do
   });
 }
 
+int pyfacc_split_values_dev(int what, int fp32, int L, int n, const double* x_dev, double* out_dev) {
+  if (what < 0 || what > 3 || L < 0 || L > 4 || (what > 1 && L > 0) || (what == 3 && fp32) || n < 0 ||
+      (n > 0 && (!x_dev || !out_dev)))
+    return PYFACC_ERR_INVALID;
+  return guarded([&] {
+    int dev = 0;
+    PF_CUDA(cudaGetDevice(&dev));
+    pyfacc::ensure_boys_tables(dev);
+    pyfacc::launch_split_values(what, fp32 != 0, L, n, x_dev, out_dev, 0);
+    PF_CUDA(cudaDeviceSynchronize());
+  });
+}
+
 int pyfacc_dense_gemm_dev(int m, int n, int k, int ta, const double* A_dev, int tb, const double* B_dev,
                           double* C_dev, int sym, int asym_a) {
   if (m < 0 || n < 0 || k < 0 || (m * n > 0 && (!A_dev || !B_dev || !C_dev))) return PYFACC_ERR_INVALID;

@@ -332,6 +332,7 @@ void launch_grad_split(const PairData& pd, const TaskList& tl, int bra_class, in
                        const struct GradArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
 void upload_boys_rows(int device);  // their Boys tables, on the current device
 const void* boys_rows_table(bool fp32, int L);
+void launch_split_values(int what, bool fp32, int L, int n, const double* x, double* out, cudaStream_t s);
 
 // Task lists rebuilt on the GPU for one Fock build from the density bound
 // dmax (ns x ns): a bra pair i keeps the ket prefix with

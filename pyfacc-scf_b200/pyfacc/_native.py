@@ -111,6 +111,7 @@ SIGNATURES = {
     "pyfacc_launch_count": (ctypes.c_longlong, []),
     "pyfacc_split_launch_count": (ctypes.c_longlong, [c_int]),
     "pyfacc_boys_dev": (c_int, [c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "pyfacc_split_values_dev": (c_int, [c_int, c_int, c_int, c_int, c_void_p, c_void_p]),
     "pyfacc_partition": (c_int, [c_int, P_double, c_int, ctypes.POINTER(c_int)]),
     "pyfacc_dense_gemm_dev": (c_int, [c_int, c_int, c_int, c_int, c_void_p, c_int, c_void_p, c_void_p, c_int, c_int]),
     "pyfacc_purify_dev": (c_int, [c_int, c_int, c_void_p, c_void_p, ctypes.POINTER(c_int)]),
