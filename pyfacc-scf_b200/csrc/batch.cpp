@@ -684,7 +684,7 @@ void Batch::alloc() {
   for (size_t k = 0; k < nmat; ++k) om[k] = carve(m8);
   const size_t o_diis = carve(std::max<size_t>(2 * nd * m8, 8));
   const size_t o_dmax = carve((size_t)nmol * ns_max * ns_max * sizeof(float));
-  const size_t o_stats = carve(sizeof(JkStats) + 2 * NQCLASS * sizeof(unsigned long long));
+  const size_t o_stats = carve(sizeof(JkStats) + sizeof(GradStats));
   const size_t o_grad = carve(3 * (size_t)natoms_tot * sizeof(double));
   const size_t o_act = carve(sizeof(StepReport));
   const size_t o_ctl = carve(sizeof(BatchScfCtl));
@@ -1109,9 +1109,7 @@ void Batch::run(bool gradient) {
   for (int p = 0; p < 2; ++p)
     for (int q = 0; q < NQCLASS; ++q) {
       timing.quartets[p] += js.quartets[p][q];
-      const ClassFlops& cf = class_flops(q);
-      timing.flops_fock += (double)js.prims[p][q] * (cf.vrr + prim_overhead_flops(q, p == 1)) +
-                           (double)js.quartets[p][q] * (cf.hrr + digest_flops(q, 1));
+      timing.flops_fock += jk_flops(js, p, q, 1);
     }
   if (gradient) gradient_run();
   timing.ms_total = wall_ms() - t0;
@@ -1141,7 +1139,7 @@ void Batch::gradient_run() {
   launch_grad1e(shd, n1e, pairs1e, g1, num_sms, stream);
   PF_CUDA(cudaEventRecord(ev[2], stream));
   unsigned long long* gstats = stats_dev + sizeof(JkStats) / sizeof(unsigned long long);
-  PF_CUDA(cudaMemsetAsync(gstats, 0, 2 * NQCLASS * sizeof(unsigned long long), stream));
+  PF_CUDA(cudaMemsetAsync(gstats, 0, sizeof(GradStats), stream));
   GradArgs g2;
   g2.Pt = dargs.P;
   g2.Pa = dargs.P;
@@ -1193,8 +1191,8 @@ void Batch::gradient_run() {
   grad_host.assign(3 * (size_t)natoms_tot, 0.0);
   PF_CUDA(cudaMemcpyAsync(grad_host.data(), grad_dev, grad_host.size() * sizeof(double), cudaMemcpyDeviceToHost,
                           stream));
-  unsigned long long cnt[2 * NQCLASS];
-  PF_CUDA(cudaMemcpyAsync(cnt, gstats, sizeof(cnt), cudaMemcpyDeviceToHost, stream));
+  GradStats cnt;
+  PF_CUDA(cudaMemcpyAsync(&cnt, gstats, sizeof(cnt), cudaMemcpyDeviceToHost, stream));
   PF_CUDA(cudaStreamSynchronize(stream));
   if (opt.verbose) {
     float a = 0, b = 0, c = 0;
@@ -1204,10 +1202,7 @@ void Batch::gradient_run() {
     std::fprintf(stderr, "pyfacc batch gradient (ms): W + dmax %.3f  one-electron %.3f  two-electron %.3f\n", a, b, c);
   }
   for (auto& e : ev) cudaEventDestroy(e);
-  timing.flops_grad = 0.0;
-  for (int q = 0; q < NQCLASS; ++q)
-    timing.flops_grad += (double)cnt[NQCLASS + q] * (class_flops(q).grad + prim_overhead_flops(q, false)) +
-                       (double)cnt[q] * class_flops(q).gfin;
+  timing.flops_grad = grad_flops(cnt);
   // nuclear repulsion (molecule.f90:31-52 differentiated)
   for (const auto& M : mols)
     for (int i = 0; i < M.natoms; ++i)

@@ -230,22 +230,30 @@ struct PairData {
   DeviceBuf buf;
 };
 
+// Counters of the J/K kernels, [fp64, fp32][class].
 struct JkStats {
-  unsigned long long quartets[2][NQCLASS];  // [fp64, fp32][class]
+  unsigned long long quartets[2][NQCLASS];
   unsigned long long prims[2][NQCLASS];
+  unsigned long long far[2][NQCLASS];     // primitive quartets of the far kernels
+  unsigned long long j_only[2][NQCLASS];  // quartets of theirs that only J took
 };
+constexpr int JK_STATS_FAR = 4 * NQCLASS, JK_STATS_J_ONLY = 6 * NQCLASS;  // in words
+// Counters of the gradient kernels: quartets and primitive quartets per class,
+// in Hermite Gaussians, with contracted accumulators, and of the far kernels.
+struct GradStats {
+  struct Kind { unsigned long long quartets[NQCLASS], prims[NQCLASS]; } hermite, contracted, far;
+};
+constexpr int GRAD_STATS_CONTRACTED = 2 * NQCLASS, GRAD_STATS_FAR = 4 * NQCLASS;
 
-// Algorithmic flop counts of the generated class routines (eri_classes.cuh).
-// Generated operation counts of a class: J/K VRR per primitive quartet and
-// HRR per contracted quartet; gradient per primitive quartet (grad) and per
-// contracted quartet (gfin: the HRR after the primitive sum, 0 for the
-// classes that contract per primitive).
-struct ClassFlops { int L, nout, vrr, hrr, grad, gfin; };
+// Operation counts of a class: J/K VRR per primitive quartet and HRR per
+// contracted quartet (eri_classes.cuh); gradient per primitive quartet in
+// Hermite Gaussians (grad), or with contracted accumulators (gacc) and once
+// per contracted quartet (gfin).
+struct ClassFlops { int L, nout, vrr, hrr, grad, gacc, gfin; };
 const ClassFlops& class_flops(int qclass);
-// Flops charged per primitive quartet outside the VRR (prefactors + Boys)
-// and per contracted quartet for the J/K digestion.
-double prim_overhead_flops(int qclass, bool fp32);
-double digest_flops(int qclass, int nk);
+// Flops that the counted quartets took.
+double jk_flops(const JkStats& s, int prec, int qclass, int nk);
+double grad_flops(const GradStats& s);
 
 // ------------------------------------------------------------- launchers
 // Every kernel launch of this library is counted (pyfacc_launch_count).
@@ -300,7 +308,7 @@ struct JkArgs {
   const float* dmax;     // shell-block max |D|, ns x ns (or null)
   int ns_ld;             // leading dimension of dmax
   double thresh;         // density-weighted Schwarz threshold
-  unsigned long long* stats;  // JkStats layout (device) or null
+  unsigned long long* stats;  // JkStats (device) or null
   // primitive quartets with |K_ab K_cd| max|D| below this are skipped (the
   // primitive pairs of a shell pair are sorted by |K|); 0 = none
   double prim_thresh = 0.0;

@@ -305,12 +305,13 @@ __device__ __forceinline__ void md_gradient(const T* I, T scale, const T* PQ, co
 }
 
 // FP operations of md_gradient (an FMA counts as two), from the loops above.
-constexpr int md_flops(bool bb, int kl) {
-  const int L = 1 + (bb ? 1 : 0) + kl, nb = bb ? 3 : 1, ncd = kl == 2 ? 9 : (kl == 1 ? 3 : 1);
-  int n = ncd * ((bb ? 54 : 8) + (bb ? 10 : 4) * 4 * kl);  // Hermite densities
+constexpr int md_flops(int bl, int kl) {
+  const bool bb = bl == 2;
+  const int L = bl + kl, nb = bb ? 3 : 1, ncd = kl == 2 ? 9 : (kl == 1 ? 3 : 1);
+  int n = ncd * ((bb ? 54 : 8 * bl) + (bb ? 10 : 4) * 4 * kl);  // Hermite densities
   for (int m = 1; m <= L + 1; ++m) n += 2 * (herm_count(m) - 1);
   n += 8 * herm_count(L);
-  n += ncd * ((bb ? 4 : 1) * (kl == 2 ? 7 : 3 * kl) + (bb ? 57 : 7));
+  if (bl > 0) n += ncd * ((bb ? 4 : 1) * (kl == 2 ? 7 : 3 * kl) + (bb ? 57 : 7));
   if (kl > 0) n += 3 * nb * ((kl == 2 ? 4 : 1) * (bb ? 7 : 3) + (bb ? 4 : 0) + (kl == 2 ? 57 : 7));
   return n + 56;
 }

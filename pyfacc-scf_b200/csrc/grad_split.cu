@@ -279,8 +279,9 @@ __global__ void __launch_bounds__(128, grad_min_blocks(LA + LB + LC + LD)) grad_
       p += __shfl_xor_sync(0xffffffffu, p, o);
     }
     if (lane == 0 && nq) {
-      atomicAdd(A.stats + L.qclass, nq);
-      atomicAdd(A.stats + NQCLASS + L.qclass, p);
+      unsigned long long* out = A.stats + (FAR ? GRAD_STATS_FAR : 0) + L.qclass;
+      atomicAdd(out, nq);
+      atomicAdd(out + NQCLASS, p);
     }
   }
   if (nsm) {

@@ -288,6 +288,7 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
   extern __shared__ __align__(16) unsigned char split_smem[];
   __shared__ int2 queue[4][NRING][QUEUE];  // {ket * MAXSLOT + slot, primitive cut}
   __shared__ int2 slot_bra[4][MAXSLOT];    // {bra, staged primitive pairs}
+  __shared__ unsigned count[4][NRING];     // quartets evaluated
   __shared__ typename std::conditional<FAR, int, BoysRows<R>>::type tab_smem;
   const BoysRows<R>& tab = reinterpret_cast<const BoysRows<R>&>(tab_smem);  // near half only
   if constexpr (!FAR) {
@@ -301,7 +302,8 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
   const JkArgs& A = args.a;
   const size_t slot_bytes = S::bytes(L.maxp);
   unsigned char* st = split_smem + (size_t)wib * L.nslot * slot_bytes;
-  int nquart = 0;
+  if (lane < NRING) count[wib][lane] = 0;
+  __syncwarp();
   unsigned nprim = 0;
   auto stage = [&](int ib, int slot) {
     return stage_bra<(LA + LB > 0), FAR>(L, L.bra_off + ib, L.info0[L.bra_base + ib], (R)0, st + slot * slot_bytes,
@@ -332,6 +334,10 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
     const int bp = L.bra_base + q.bra.x, kp = L.ket_base + q.ket;
     const int4 bi0 = L.info0[bp], ki0 = L.info0[kp], bi2 = L.info2[bp];
     const int mo = bi2.x, ld = bi2.y, ma = bi0.x, mb = bi0.y, mc = ki0.x, md = ki0.y;
+    if (A.stats) {  // per warp and ring (a register per lane for it spilled)
+      const unsigned m = __ballot_sync(0xffffffffu, q.active);
+      if (lane == 0) count[wib][kind] += __popc(m);
+    }
     double jab[NA * NB];
 #pragma unroll
     for (int i = 0; i < NA * NB; ++i) jab[i] = 0.0;
@@ -339,7 +345,6 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
       R out[C::NOUT];
       nprim += quartet<R, LA, LB, LC, LD, FAR>(L, tab, st + q.slot * slot_bytes, q.bra.y, q.ket, ki0.w, L.geom[bp],
                                                L.geom[kp], q.cut, out);
-      ++nquart;
       double fac = 1.0;
       const float4 bt = L.test2[bp], kt = L.test2[kp];
       if (__float_as_int(bt.z) == __float_as_int(bt.w)) fac *= 0.5;
@@ -446,15 +451,17 @@ __global__ void __launch_bounds__(128, min_blocks(LA + LB + LC + LD)) jk_split_k
   };
   split_run<NRING>(L, queue[wib], slot_bra[wib], stage, test, eval);
   if (A.stats) {  // contracted and evaluated primitive quartets
-    unsigned long long nq = (unsigned)nquart, p = nprim;
+    unsigned long long p = nprim;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      nq += __shfl_xor_sync(0xffffffffu, nq, o);
-      p += __shfl_xor_sync(0xffffffffu, p, o);
-    }
+    for (int o = 16; o > 0; o >>= 1) p += __shfl_xor_sync(0xffffffffu, p, o);
+    const unsigned long long nj = count[wib][0], nq = NRING == 2 ? nj + count[wib][NRING - 1] : nj;
     if (lane == 0 && nq) {
       atomicAdd(A.stats + args.prec * NQCLASS + L.qclass, nq);
       atomicAdd(A.stats + (2 + args.prec) * NQCLASS + L.qclass, p);
+      if (FAR) {
+        atomicAdd(A.stats + JK_STATS_FAR + args.prec * NQCLASS + L.qclass, p);
+        atomicAdd(A.stats + JK_STATS_J_ONLY + args.prec * NQCLASS + L.qclass, nj);
+      }
     }
   }
 }

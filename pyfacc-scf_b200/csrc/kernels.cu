@@ -962,6 +962,8 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
   // and block at the end) when the gradient is small enough
   extern __shared__ double gsh[];
   constexpr bool kGamSmem = C::L >= 4;
+  // exponent-weighted accumulators over the primitives, or Hermite Gaussians
+  constexpr bool kContracted = C::L == 0 || (sizeof(R) == 4 && C::L < 3);
   const int nsm = args.smem_atoms * 3;
   for (int i = threadIdx.x; i < nsm; i += blockDim.x) gsh[i] = 0.0;
   if (nsm) __syncthreads();
@@ -1048,7 +1050,7 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
       const V* prim = grecords<R>(args);
       const R cut = (R)kcut;
       const R kab_max = fabs((R)brec[0].z);
-      if constexpr (C::L == 0 || (sizeof(R) == 4 && C::L < 3)) {
+      if constexpr (kContracted) {
         // exponent-weighted sums over the primitive quartets, then one HRR
         // and one contraction with Gamma per contracted quartet
         R acc[C::NGACC];
@@ -1125,8 +1127,9 @@ __global__ void __launch_bounds__(128) grad2e_kernel(const GradKernelArgs args) 
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
       if (lane == 0) {
-        if (slice == 0) atomicAdd(A.stats + args.qclass, (unsigned long long)__popc(amask));
-        atomicAdd(A.stats + NQCLASS + args.qclass, tot);
+        unsigned long long* st = A.stats + (kContracted ? GRAD_STATS_CONTRACTED : 0) + args.qclass;
+        if (slice == 0) atomicAdd(st, (unsigned long long)__popc(amask));
+        atomicAdd(st + NQCLASS, tot);
       }
     }
     // centre A and B are the bra's, uniform across a task's lanes
@@ -2291,8 +2294,7 @@ double probe_fp64(int device, double* fp32) {
 namespace pyfacc {
 
 // ---------------------------------------------------------------------------
-// Algorithmic flop counts (from the generated class routines; gradient: of
-// grad_md.cuh, also for the FP32 classes that keep contracted accumulators)
+// Flop counts (from the generated class routines and grad_md.cuh)
 // ---------------------------------------------------------------------------
 const ClassFlops& class_flops(int qc) {
   using C0 = EriClass<double, 0, 0, 0, 0>;
@@ -2302,25 +2304,40 @@ const ClassFlops& class_flops(int qc) {
   using C4 = EriClass<double, 1, 1, 1, 0>;
   using C5 = EriClass<double, 1, 1, 1, 1>;
   static const ClassFlops tab[NQCLASS] = {
-      {C0::L, C0::NOUT, C0::VRR_FLOPS, C0::HRR_FLOPS, C0::GACC_FLOPS, C0::GFIN_FLOPS},
-      {C1::L, C1::NOUT, C1::VRR_FLOPS, C1::HRR_FLOPS, md_flops(false, 0), 0},
-      {C2::L, C2::NOUT, C2::VRR_FLOPS, C2::HRR_FLOPS, md_flops(false, 1), 0},
-      {C3::L, C3::NOUT, C3::VRR_FLOPS, C3::HRR_FLOPS, md_flops(true, 0), 0},
-      {C4::L, C4::NOUT, C4::VRR_FLOPS, C4::HRR_FLOPS, md_flops(true, 1), 0},
-      {C5::L, C5::NOUT, C5::VRR_FLOPS, C5::HRR_FLOPS, md_flops(true, 2), 0},
+      {C0::L, C0::NOUT, C0::VRR_FLOPS, C0::HRR_FLOPS, md_flops(0, 0), C0::GACC_FLOPS, C0::GFIN_FLOPS},
+      {C1::L, C1::NOUT, C1::VRR_FLOPS, C1::HRR_FLOPS, md_flops(1, 0), C1::GACC_FLOPS, C1::GFIN_FLOPS},
+      {C2::L, C2::NOUT, C2::VRR_FLOPS, C2::HRR_FLOPS, md_flops(1, 1), C2::GACC_FLOPS, C2::GFIN_FLOPS},
+      {C3::L, C3::NOUT, C3::VRR_FLOPS, C3::HRR_FLOPS, md_flops(2, 0), C3::GACC_FLOPS, C3::GFIN_FLOPS},
+      {C4::L, C4::NOUT, C4::VRR_FLOPS, C4::HRR_FLOPS, md_flops(2, 1), 0, 0},
+      {C5::L, C5::NOUT, C5::VRR_FLOPS, C5::HRR_FLOPS, md_flops(2, 2), 0, 0},
   };
   return tab[qc];
 }
 
 // Per primitive quartet outside the VRR: P-Q (3), T (6), prefactor (2),
 // zeta/rho/W terms (12), Boys (Taylor 2*8 + downward recursion 4L), I_m (L+1).
-double prim_overhead_flops(int qc, bool) {
-  const int L = class_flops(qc).L;
-  return 3 + 6 + 2 + 12 + 16 + 4 * L + (L + 1);
+static double setup_flops(int L) { return 3 + 6 + 2 + 12 + 16 + 4 * L + (L + 1); }
+// In the far limit: P-Q (3), |PQ|^2 (5), k_ab k_cd and I_0 (2), and with L > 0
+// the step (2), I_m (2 L) and the W terms (10).
+static double far_setup_flops(int L) { return 3 + 5 + 2 + (L > 0 ? 2 + 2 * L + 10 : 0); }
+
+double jk_flops(const JkStats& s, int p, int q, int nk) {
+  const ClassFlops& cf = class_flops(q);
+  const double far = (double)s.far[p][q], near = (double)s.prims[p][q] - far;
+  // digestion: J 4 flops per integral, K 8 per integral and exchange density
+  return near * (cf.vrr + setup_flops(cf.L)) + far * (cf.vrr + far_setup_flops(cf.L)) +
+         (double)s.quartets[p][q] * (cf.hrr + cf.nout * (4.0 + 8.0 * nk)) - (double)s.j_only[p][q] * cf.nout * 8.0 * nk;
 }
 
-// Digestion per contracted quartet: J (4 flops per integral) and K (8 per
-// integral and exchange density).
-double digest_flops(int qc, int nk) { return (double)class_flops(qc).nout * (4.0 + 8.0 * nk); }
+double grad_flops(const GradStats& s) {
+  double f = 0.0;
+  for (int q = 0; q < NQCLASS; ++q) {
+    const ClassFlops& cf = class_flops(q);
+    f += (double)s.hermite.prims[q] * (cf.grad + setup_flops(cf.L + 1)) +
+         (double)s.contracted.prims[q] * (cf.gacc + setup_flops(cf.L + 1)) + (double)s.contracted.quartets[q] * cf.gfin +
+         (double)s.far.prims[q] * (cf.grad + far_setup_flops(cf.L + 1));
+  }
+  return f;
+}
 
 }  // namespace pyfacc

@@ -138,9 +138,7 @@ void System::jk_counters(int nk, double out[6], double* per_class) {
   for (int k = 0; k < 6; ++k) out[k] = 0.0;
   for (int p = 0; p < 2; ++p)
     for (int q = 0; q < NQCLASS; ++q) {
-      const ClassFlops& cf = class_flops(q);
-      out[p] += (double)js.prims[p][q] * (cf.vrr + prim_overhead_flops(q, p == 1)) +
-                (double)js.quartets[p][q] * (cf.hrr + digest_flops(q, nk));
+      out[p] += jk_flops(js, p, q, nk);
       out[2 + p] += (double)js.quartets[p][q];
       out[4 + p] += (double)js.prims[p][q];
       if (per_class) {
@@ -771,9 +769,7 @@ void System::run_scf() {
   for (int p = 0; p < 2; ++p)
     for (int q = 0; q < NQCLASS; ++q) {
       st.quartets[p] += js.quartets[p][q];
-      const ClassFlops& cf = class_flops(q);
-      st.flops_fock += (double)js.prims[p][q] * (cf.vrr + prim_overhead_flops(q, p == 1)) +
-                       (double)js.quartets[p][q] * (cf.hrr + digest_flops(q, nk));
+      st.flops_fock += jk_flops(js, p, q, nk);
     }
   st.done = true;
   cudaEventDestroy(t0);
@@ -845,7 +841,8 @@ void System::gradient(double* g_host) {
   g2.uhf = uhf ? 1 : 0;
   g2.grad = grad_dev;
   unsigned long long* gstats = stats_dev;  // reuse the J/K counters' space
-  PF_CUDA(cudaMemsetAsync(gstats, 0, 2 * NQCLASS * sizeof(unsigned long long), stream));
+  static_assert(sizeof(GradStats) <= sizeof(JkStats), "counters' space");
+  PF_CUDA(cudaMemsetAsync(gstats, 0, sizeof(GradStats), stream));
   g2.stats = gstats;
   // FP32 derivative integrals for the small quartets on request, or by
   // default in mixed mode (C20H42: 3.30 -> 3.18 ms, C100H202 80 -> 75 ms).  One
@@ -898,12 +895,9 @@ void System::gradient(double* g_host) {
   PF_CUDA(cudaMemcpyAsync(g.data(), grad_dev, 3 * natoms * sizeof(double), cudaMemcpyDeviceToHost, stream));
   PF_CUDA(cudaStreamSynchronize(stream));
   st.ms_grad = elapsed(a0, a1);
-  unsigned long long cnt[2 * NQCLASS];
-  PF_CUDA(cudaMemcpy(cnt, gstats, sizeof(cnt), cudaMemcpyDeviceToHost));
-  st.flops_grad = 0.0;
-  for (int q = 0; q < NQCLASS; ++q)
-    st.flops_grad += (double)cnt[NQCLASS + q] * (class_flops(q).grad + prim_overhead_flops(q, false)) +
-                       (double)cnt[q] * class_flops(q).gfin;
+  GradStats cnt;
+  PF_CUDA(cudaMemcpy(&cnt, gstats, sizeof(cnt), cudaMemcpyDeviceToHost));
+  st.flops_grad = grad_flops(cnt);
   nuclear_repulsion_gradient(g.data());
   grad_host = g;
   if (g_host) std::memcpy(g_host, g.data(), g.size() * sizeof(double));
