@@ -158,7 +158,9 @@ __global__ void __launch_bounds__(256) batch_pairs_kernel(const BatchPairArgs A)
       z += sum[2 * i] * sum[2 * i + 1];
     } else {
       k += cnt[2 * i + li] * (cnt[2 * i + li] + 1) / 2;
-      z += (sum[2 * i + li] * sum[2 * i + li] + sq[2 * i + li]) / 2;
+      // (twice the result may pass 2^31)
+      const unsigned s = sum[2 * i + li];
+      z += (int)((s * s + (unsigned)sq[2 * i + li]) / 2);
     }
     k += A.pair_off[c * A.nmol + m];
     z += A.prim_off[c * A.nmol + m];
