@@ -65,10 +65,10 @@ WORKLOADS = {
 # running the oracle's SCF on the same molecules
 ORACLE_SCF_ITERS = {"c20h42": 22, "c10h22": 21, "c40h82": 24}
 # DRAM bytes per launch of the dominant J/K class kernel from one ncu capture
-# (profiles/jk_kernel_fp64_c40h82.md): the working set is L2-resident
-JK_TRAFFIC_BYTES = 4.73e6
-JK_TRAFFIC_NOTE = ("dram read + write per launch of jk_kernel<double,1,0,0,0> (the largest class) in a full FP64 "
-                   "C40H82 build (ncu, profiles/jk_kernel_fp64_c40h82.md)")
+# (profiles/split_kernels_c40h82.md): the working set is L2-resident
+JK_TRAFFIC_BYTES = 3.39e6
+JK_TRAFFIC_NOTE = ("dram read + write per launch of jk_split_kernel<double,1,0,0,0> (near half, the largest launch) in a "
+                   "full FP64 C40H82 build (ncu, profiles/split_kernels_c40h82.md)")
 
 
 def metric_name(wl):
@@ -396,8 +396,8 @@ def run_ours(args):
     a64 = rates["fp64"]["tflops_fp64"]
     a32 = rates["fp32"]["tflops_fp32"]
     roof = {
-        "kernel": "J/K digestion (jk_kernel<double, class> x 6 classes), full FP64 Fock build on the converged "
-                  "density",
+        "kernel": "J/K digestion (jk_split_kernel<double, class>, near and far, for the long lists, "
+                  "jk_kernel<double, class> for the others), full FP64 Fock build on the converged density",
         "bound": "fp64",
         "achieved": a64,
         "peak": peak64 / 1e3 if peak64 else None,
@@ -409,7 +409,7 @@ def run_ours(args):
                        "MEASURED_PEAKS.json holds no FP64/FP32 CUDA-core figure",
         "algorithmic_flops_per_build": rates["fp64"]["flops_fp64"],
         "ms_per_build": rates["fp64"]["ms_per_build"],
-        "fp32": {"kernel": "jk_kernel<float, class> x 6, every quartet in FP32, converged density",
+        "fp32": {"kernel": "the same kernels in float, every quartet in FP32, converged density",
                  "bound": "fp32", "achieved": a32, "peak": peak32 / 1e3 if peak32 else None, "unit": "TFLOP/s",
                  "frac": (a32 / (peak32 / 1e3)) if peak32 else None,
                  "algorithmic_flops_per_build": rates["fp32"]["flops_fp32"],

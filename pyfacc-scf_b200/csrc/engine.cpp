@@ -542,6 +542,8 @@ void System::build_tasks() {
   std::vector<int> hostbuf;
   struct Pending { int bc, kc, prec; size_t off, off_c; int nbra; };
   std::vector<Pending> pend;
+  // runs of the device-built FP32 lists, from the whole lists
+  int dyn_chunk[NQCLASS] = {}, dyn_runs[NQCLASS] = {};
   const double thr = std::max(opt.schwarz_thresh, 0.0);
   const double t32 = opt.fp32_thresh;
   quartets_total = 0;
@@ -593,9 +595,22 @@ void System::build_tasks() {
         }
         toff[nb] = ntask;
         if (prec == 0) quartets_total += quart;
-        const int chunk = !split_class(pd, bc, kc)
-                              ? 0
-                              : split_chunk(quart, far_share, pd.class_maxprim[bc] * pd.class_maxprim[kc], num_sms);
+        auto runs = [&](int c) {
+          int nt = 0;
+          for (int i = 0; i < nb; ++i) nt += (hi[i] - lo[i] + c - 1) / c;
+          return nt;
+        };
+        auto chunk_of = [&](bool fp32) {
+          if (!split_class(pd, bc, kc)) return 0;
+          return split_chunk(quart, far_share, pd.class_maxprim[bc] * pd.class_maxprim[kc], fp32, num_sms);
+        };
+        const int chunk = chunk_of(prec == 2);
+        if (prec == 0 && chunk_of(true)) {
+          const int qc = (bc == 0) ? 0 : (bc == 1 ? 1 + kc : 3 + kc);
+          dyn_chunk[qc] = chunk_of(true);
+          dyn_runs[qc] = runs(dyn_chunk[qc]);
+          any_split = true;
+        }
         TaskList& tl = tasks[bc][kc][prec];
         tl.width = task_width;
         tl.nbra = nb;
@@ -640,10 +655,10 @@ void System::build_tasks() {
         tl.width = task_width;
         tl.nbra = nb;
         tl.ntasks = std::max(1, tasks[bc][kc][0].ntasks);
-        tl.chunk = part == 1 ? tasks[bc][kc][0].chunk : 0;
+        tl.chunk = part == 1 ? dyn_chunk[qc] : 0;
         tl.far = tasks[bc][kc][0].far;
         tl.nquartets = tasks[bc][kc][0].nquartets;  // a bound
-        tl.ntasks_c = std::max(1, tasks[bc][kc][0].ntasks_c);
+        tl.ntasks_c = std::max(1, dyn_runs[qc]);
         tl.task_off = tl.off_c = dd;
         tl.ket_lo = dd + nb + 1;
         tl.ket_hi = dd + 2 * nb + 1;

@@ -325,7 +325,8 @@ constexpr double SPLIT_MIN_FAR = 3.0e5;   // estimated far quartets of a list (s
 constexpr double FAR_DISTANCE = 16.0;     // bohr: quartets of diffuse pairs that far apart are far in FP64
 constexpr int SPLIT_COUNTERS = 4 * NQCLASS;  // task counters of a build: two kernels per class and precision
 int split_run(long long nquartets, int prim_quartets, int num_sms);
-int split_chunk(long long nquartets, double far_share, int prim_quartets, int num_sms);
+constexpr int SPLIT_DEEP = 400;           // primitive quartets (STO-4G: 256, STO-5G: 625)
+int split_chunk(long long nquartets, double far_share, int prim_quartets, bool fp32, int num_sms);
 bool split_class(const PairData& pd, int bra_class, int ket_class);  // classes that they cover
 bool jk_splits(const PairData& pd, const TaskList& tl);
 bool alloc_split_records(PairData& pd, DeviceBuf& buf, size_t max_bytes);
@@ -333,9 +334,10 @@ bool memory_left(long long mallocs);  // enough of the device's memory beside th
 void launch_jk_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32, int nk,
                      const JkArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
 // Far quartets of a list (estimate) from which its FP32 derivative quartets go
-// to the split kernels: C20H42, 4e5 to 5e5 a list, 1.19 ms undivided, 1.28
-// divided; C40H82, (ss|ss) and (ps|ss) 1.5e6, 4.1 -> 3.6 ms.
-constexpr double GRAD_SPLIT_FP32_FAR = 6.0e5;
+// to the split kernels, mixed gradient undivided and divided: C24H50 1.59 and
+// 1.68 ms, C28H58 2.01 and 2.06, C32H66 (1.4e6 a list) 2.61 and 2.58, C36H74
+// 3.21 and 3.11.
+constexpr double GRAD_SPLIT_FP32_FAR = 1.2e6;
 void launch_grad_split(const PairData& pd, const TaskList& tl, int bra_class, int ket_class, bool fp32,
                        const struct GradArgs& a, int num_sms, int* next, cudaStream_t s_far, cudaStream_t s_near);
 void upload_boys_rows(int device);  // their Boys tables, on the current device

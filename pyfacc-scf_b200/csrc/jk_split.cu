@@ -517,8 +517,13 @@ void dispatch(int qc, int nk, int blocks, cudaStream_t s_far, cudaStream_t s_nea
 // (pp|ps), 3e5 and 5e5, too), while a cluster of 16 waters, 5e5 quartets of
 // which next to none are far, loses (0.46 -> 0.63 ms).  far_share is the share
 // of atom pairs beyond FAR_DISTANCE.
-int split_chunk(long long nquartets, double far_share, int prim_quartets, int num_sms) {
-  return (double)nquartets * far_share < SPLIT_MIN_FAR ? 0 : split_run(nquartets, prim_quartets, num_sms);
+// FP64 lists of the deepest contractions need twice as many: their few runs
+// last too long to share evenly (STO-6G, FP64 build of C16H34 5.2 ms undivided,
+// 5.9 divided, C18H38 6.6 and 7.2, C20H42 8.2 and 8.0; in FP32 2.75 and 2.49,
+// 3.54 and 3.02, 4.36 and 3.41; STO-4G C18H38 FP64 1.74 and 1.67).
+int split_chunk(long long nquartets, double far_share, int prim_quartets, bool fp32, int num_sms) {
+  const double line = !fp32 && prim_quartets > SPLIT_DEEP ? 2.0 * SPLIT_MIN_FAR : SPLIT_MIN_FAR;
+  return (double)nquartets * far_share < line ? 0 : split_run(nquartets, prim_quartets, num_sms);
 }
 
 // Runs as long as leave SPLIT_RUNS_PER_SM per SM, more for deep contractions,

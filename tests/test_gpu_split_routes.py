@@ -109,3 +109,20 @@ def test_sharded_gradient_of_split_lists(engine):
     for rank in range(2):
         assert results[rank][0] == pytest.approx(ref.energy, abs=1e-9)
         assert np.abs(results[rank][1] - ref.gradient).max() < 1e-8
+
+
+def test_deep_contractions_split_fp64_lists_later(engine):
+    """STO-6G: between the lines of FP32 and FP64 lists, and above both."""
+    import torch
+    from pyfacc import geometry as G
+    for n, fp64 in ((17, False), (24, True)):
+        with engine.System(engine.Molecule(*G.alkane(n, seed=n), "sto-6g")) as s:
+            D = torch.eye(s.nbf, dtype=torch.float64, device="cuda")
+            (J, K), (near, _) = _split(lambda: s.jk(D))
+            assert (near > 0) == fp64
+            for precision in ("fp32", "mixed"):
+                (Jf, Kf), (near, far) = _split(lambda: s.jk(D, precision=precision))
+                assert precision == "mixed" or near == far > 0
+                # 36 roundings of 2^-24 of the largest element (1296 primitive quartets)
+                assert (Jf - J).abs().max().item() < 36 * 2.0 ** -24 * J.abs().max().item()
+                assert (Kf - K).abs().max().item() < 36 * 2.0 ** -24 * K.abs().max().item()
