@@ -1738,7 +1738,8 @@ constexpr size_t GRAD1E_SMEM_MAX = 96 * 1024;
 template <int LA, int LB>
 static void grad1e_launch(int blocks, size_t smem, int use_smem, int n, const int2* pairs, const ShellDev& sh,
                           const OneEGradArgs& a, cudaStream_t s) {
-  if (smem > 48 * 1024) allow_smem(grad1e_kernel<LA, LB>, GRAD1E_SMEM_MAX);
+  // (the default allowance of 48 KB holds the kernel's static arrays as well)
+  allow_smem(grad1e_kernel<LA, LB>, GRAD1E_SMEM_MAX);
   grad1e_kernel<LA, LB><<<blocks, 128, smem, s>>>(n, pairs, sh.cen, sh.desc, sh.nprim, sh.ex, sh.co, sh.mol, use_smem,
                                                   a);
 }
