@@ -462,7 +462,7 @@ void Batch::build_pairs() {
 }
 
 // Which (bra class, ket class) combinations go to the split kernels
-// (jk_split.cu, grad_split.cu), and the transposed records for them.  Their
+// (jk_split.cu), and the transposed records for them.  Their
 // near kernel alone is the faster one for a long list of near quartets: its
 // queues keep the lanes full across bras and molecules (a bra's kets end with
 // its molecule), its Boys table is read without bank conflicts.  256 clusters
@@ -470,11 +470,11 @@ void Batch::build_pairs() {
 // BATCH_SPLIT_MIN candidates it loses (12 clusters, lists from 1e6 on:
 // 28.4 -> 33 ms).  The far kernel's second pass over the candidates pays where
 // a good share of the atom pairs is far (24 alkanes of 18 to 21 carbons, FP64
-// SCF: undivided 304, near alone 215, both 173 ms).  The FP64 gradient takes
-// the near kernel for the longer lists (256 clusters 95 -> 77 ms, 64 24.2 ->
-// 21.5), not for lists with far halves (the alkanes: 56 -> 63 ms).  An
-// explicit task width is for the undivided kernels, and without memory for the
-// records they run as well.
+// SCF: undivided 304, near alone 215, both 173 ms).  The gradient keeps the
+// undivided kernels, whose time the Hermite derivatives take, not the Boys
+// function (256 clusters, FP64 65.3 ms and 63.9 with the near kernel, mixed 39.4
+// and 51.6; 64: 20.1 and 20.4, 12.8 and 16.7).  An explicit task width is for
+// the undivided kernels, and without memory for the records they run as well.
 void Batch::choose_split() {
   pd.kt = KetTables();
   pd.test = nullptr;
@@ -507,7 +507,6 @@ void Batch::choose_split() {
       if (nq < BATCH_SPLIT_MIN || !split_class(pd, bc, kc)) continue;
       split_len[bc][kc] = split_run((long long)(nq / BATCH_SPLIT_RUN_SHARE), pd.class_maxprim[bc] * pd.class_maxprim[kc], num_sms);
       split_halves[bc][kc] = nfar >= SPLIT_MIN_FAR && nfar >= BATCH_SPLIT_FAR_SHARE * nq;
-      grad_split[bc][kc] = !split_halves[bc][kc] && nq >= BATCH_SPLIT_GRAD_MIN;
       any_split = true;
     }
   if (!any_split) return;
@@ -1161,7 +1160,6 @@ void Batch::gradient_run() {
   const bool split = pd.primf != nullptr &&
                      (opt.gradient_precision == PYFACC_PRECISION_MIXED ||
                       (opt.gradient_precision < 0 && opt.precision == PYFACC_PRECISION_MIXED));
-  if (any_split) launch_zero(jk_next, SPLIT_COUNTERS * sizeof(int), stream);
   if (split) {  // the FP32 half on the side stream, overlapping the FP64 half
     PF_CUDA(cudaEventRecord(ctx.fork, stream));
     PF_CUDA(cudaStreamWaitEvent(ctx.side, ctx.fork, 0));
@@ -1169,18 +1167,11 @@ void Batch::gradient_run() {
   int nth = 0;
   for (int bc = NCLASS - 1; bc >= 0; --bc)
     for (int kc = bc; kc >= 0; --kc, ++nth) {
-      auto derive = [&](int part, bool fp32, cudaStream_t s) {
-        if (grad_split[bc][kc] && jk_splits(pd, split_tasks[bc][kc][part]))
-          launch_grad_split(pd, split_tasks[bc][kc][part], bc, kc, fp32, g2, num_sms,
-                            jk_next + 2 * (2 * qclass_index(bc, kc) + (fp32 ? 1 : 0)), s, s);
-        else
-          launch_grad2e(pd, tasks[bc][kc][part], bc, kc, fp32, g2, num_sms, s);
-      };
       if (split) {  // the two halves swap streams from class to class
-        derive(3, false, (nth & 1) ? ctx.side : stream);
-        derive(4, true, (nth & 1) ? stream : ctx.side);
+        launch_grad2e(pd, tasks[bc][kc][3], bc, kc, false, g2, num_sms, (nth & 1) ? ctx.side : stream);
+        launch_grad2e(pd, tasks[bc][kc][4], bc, kc, true, g2, num_sms, (nth & 1) ? stream : ctx.side);
       } else {
-        derive(0, false, stream);
+        launch_grad2e(pd, tasks[bc][kc][0], bc, kc, false, g2, num_sms, stream);
       }
     }
   if (split) {

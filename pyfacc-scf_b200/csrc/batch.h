@@ -33,7 +33,6 @@ constexpr int BATCH_THREADS = 512;
 constexpr int BATCH_NBF_MAX = 160;   // larger molecules run on their own
 // Lists for the split kernels (Batch::choose_split).
 constexpr double BATCH_SPLIT_MIN = 2.0e6;        // candidate quartets
-constexpr double BATCH_SPLIT_GRAD_MIN = 4.0e6;
 constexpr double BATCH_SPLIT_FAR_SHARE = 0.25;   // of them in far atom pairs
 // A run is as long as leaves every SM four times the runs that one molecule's
 // lists leave it: the molecules' ket lists are short and uneven (12 clusters,
@@ -238,7 +237,7 @@ class Batch {
   // the transposed records that those read
   TaskList split_tasks[NCLASS][NCLASS][BATCH_NPARTS];
   int split_len[NCLASS][NCLASS] = {};                 // kets per run, 0: undivided kernel
-  bool split_halves[NCLASS][NCLASS] = {}, grad_split[NCLASS][NCLASS] = {};
+  bool split_halves[NCLASS][NCLASS] = {};
   bool any_split = false;
   int* jk_next = nullptr;                             // their task counters
   DeviceBuf kt_buf;

@@ -12,8 +12,8 @@
 // primitive quartet for (pp|pp), here 3350, 4848 for (pp|ps), here 1000, or 66
 // and 69 accumulators a lane for (pp|ss) and (ps|ps), which filled the register
 // file.  The kernels are bound by the FP64 pipe and by the registers: FP64
-// gradient of C40H82 8.6 -> 5.7 ms, gly30 51 -> 25 ms, C30H61 (STO-6G, UHF) 55
-// -> 35 ms, FP32 (pp|pp) of gly30 5.3 -> 1.2 ms, (pp|ps) 4.9 -> 2.6 ms.  In the
+// gradient of C40H82 8.7 -> 5.9 ms, gly30 52 -> 26 ms, C30H61 (STO-6G, UHF) 55
+// -> 36 ms, FP32 (pp|pp) of gly30 5.3 -> 1.2 ms, (pp|ps) 4.9 -> 2.6 ms.  In the
 // undivided FP32 kernels (ps|ss), (ps|ps), (pp|ss) wait for loads either way
 // (C100H202: 10.5 / 4.2 / 1.8 ms, with this 10.5 / 4.1 / 1.6) and keep the
 // contracted accumulators.

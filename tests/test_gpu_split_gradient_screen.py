@@ -1,7 +1,7 @@
 """The split kernels' gradient takes the quartets that the undivided ones take:
-at a loose screening threshold, where a quartet more or less shows, the two
-gradients of a batch (its explicit task width is for the undivided kernels)
-agree far below the threshold."""
+at a loose screening threshold, where a quartet more or less shows, a chain's
+gradient from its own system (split) and from a batch of one (undivided) agree
+far below the threshold."""
 import numpy as np
 import pytest
 
@@ -11,15 +11,15 @@ pytestmark = pytest.mark.gpu
 def test_same_quartets_at_a_loose_threshold(engine):
     from pyfacc import _native as N
     from pyfacc import geometry as G
-    mols = [engine.Molecule(s, x) for s, x in G.water_clusters(40, 5, 6, 16)]
-    thresh = 1e-8
-    before = N.lib().pyfacc_split_launch_count(0)
-    a = engine.run_batch(mols, gradient=False, schwarz_thresh=thresh)
-    build = N.lib().pyfacc_split_launch_count(0) - before
-    a = engine.run_batch(mols, gradient=True, schwarz_thresh=thresh)
-    assert N.lib().pyfacc_split_launch_count(0) - before > 2 * build > 0, "the gradient was not split"
-    b = engine.run_batch(mols, gradient=True, schwarz_thresh=thresh, task_width=32)
-    # the densities agree to the builds' 1e-11; a quartet at the threshold adds
-    # up to 1e-8 times its density factors
-    for x, y in zip(a, b):
-        assert np.abs(x.gradient - y.gradient).max() < 1e-2 * thresh
+    mol = engine.Molecule(*G.alkane(22, seed=22))
+    opt = dict(schwarz_thresh=1e-8, eps_diis=1e-10)
+    with engine.System(mol, **opt) as s:
+        s.scf()
+        before = [N.lib().pyfacc_split_launch_count(h) for h in (0, 1)]
+        g = s.gradient()
+        assert all(N.lib().pyfacc_split_launch_count(h) > b for h, b in zip((0, 1), before))
+    ref = engine.run_batch([mol], gradient=True, task_width=32, **opt)[0].gradient
+    # left out on one side only, a quartet at the threshold moves an atom by up
+    # to 1e-8; the primitive cut is 1e-2 of it, and far pairs on one atom take
+    # all their primitives at once, cut or not: ten of those
+    assert np.abs(g - ref).max() < 1e-9
