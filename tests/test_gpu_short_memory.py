@@ -4,7 +4,7 @@ process of its own that first fills the GPU up to a given rest.  The molecule:
 a chain beside a helium atom of 24 primitives, whose pair makes the records
 (a row for each of its 576 primitive pairs, for every pair of the class) ten
 times as large as all the rest.  The batch: its records fit but leave little, or nothing
-for the matrices, or do not fit."""
+for the matrices, or do not fit, or would be larger than they may be."""
 import json
 import os
 import subprocess
@@ -53,15 +53,20 @@ def _run(kind, rest_mb, data="-"):
     return json.loads(p.stdout.strip().splitlines()[-1])
 
 
-def test_one_molecule(engine, tmp_path):
-    (tmp_path / "basis_set").mkdir()
+def _deep_helium(folder):
+    """STO-3G with a helium of 24 primitives, as the basis "deep" in folder."""
+    (folder / "basis_set").mkdir()
     a = np.geomspace(2000.0, 0.1, 24)
     c = np.exp(-0.5 * ((np.log(a) - 0.5) / 1.5) ** 2)
     text = open(basis_file("sto-3g")).read()
     lo = text.index("He     0")
     hi = text.index("****", lo)
     rows = "".join(f"  {x:.10E}  {y:.10E}\n" for x, y in zip(a, c / c.sum()))
-    (tmp_path / "basis_set" / "deep.txt").write_text(text[:lo] + "He     0\nS   24   1.00\n" + rows + text[hi:])
+    (folder / "basis_set" / "deep.txt").write_text(text[:lo] + "He     0\nS   24   1.00\n" + rows + text[hi:])
+
+
+def test_one_molecule(engine, tmp_path):
+    _deep_helium(tmp_path)
     plenty, split = _run("system", 0, str(tmp_path))
     short, none = _run("system", 320, str(tmp_path))
     assert split > 0 and none == 0
@@ -76,3 +81,22 @@ def test_batch(engine):
         out, undivided = _run("batch", rest)
         assert undivided == 0 and out is not None
         assert np.abs(np.array(out) - np.array(plenty)).max() < 1e-8
+
+
+def test_records_beyond_their_limit(engine, tmp_path):
+    """48 clusters with a helium of 24 primitives each: the batch's records
+    would take more than 4 GB, half of them less."""
+    from pyfacc import _native as N
+    from pyfacc import geometry as G
+    _deep_helium(tmp_path)
+    mols = [engine.Molecule(list(s) + ["He"], np.vstack([x, x.max(0) + 6.0]), "deep")
+            for s, x in G.water_clusters(48, 5, 16, 16)]
+
+    def run(ms):
+        before = N.lib().pyfacc_split_launch_count(0)
+        return [r.energy for r in engine.run_batch(ms, data_dir=str(tmp_path))], N.lib().pyfacc_split_launch_count(0) - before
+
+    whole, none = run(mols)
+    half, split = run(mols[:24])
+    assert split > 0 and none == 0
+    assert np.abs(np.array(whole[:24]) - np.array(half)).max() < 1e-8
