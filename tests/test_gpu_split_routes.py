@@ -125,3 +125,30 @@ def test_deep_contractions_split_fp64_lists_later(engine):
                 # 36 roundings of 2^-24 of the largest element (1296 primitive quartets)
                 assert (Jf - J).abs().max().item() < 36 * 2.0 ** -24 * J.abs().max().item()
                 assert (Kf - K).abs().max().item() < 36 * 2.0 ** -24 * K.abs().max().item()
+
+
+def test_lists_that_come_and_go_with_the_geometry(engine):
+    """One handle through a stretched chain, a coiled-up one without far
+    quartets and the first again: the records are made anew each time."""
+    import torch
+    from pyfacc import geometry as G
+    sp, xyz = G.alkane(26, seed=26)
+    # the same chain wound up: a helix of 4 bohr radius
+    c = xyz - xyz.mean(0)
+    t, u, v = (c @ np.linalg.svd(c)[2].T).T
+    coil = np.stack([(4.0 + u) * np.cos(t / 4.0), (4.0 + u) * np.sin(t / 4.0), t / 4.0 + v], 1)
+    mol = engine.Molecule(sp, xyz)
+    with engine.System(mol) as s:
+        d = np.random.default_rng(3).standard_normal((s.nbf, s.nbf))
+        D = torch.tensor(0.3 * (d + d.T), device="cuda")
+        first, far0 = _split(lambda: s.jk(D))
+        s.set_coords(coil)
+        wound, far1 = _split(lambda: s.jk(D))
+        s.set_coords(xyz)
+        again, far2 = _split(lambda: s.jk(D))
+    with engine.System(engine.Molecule(sp, coil)) as s:
+        ref = s.jk(D)
+    assert far0[1] > 0 and far1 == (0, 0) and far2 == far0
+    for x, y in ((first, again), (wound, ref)):
+        for m, n in zip(x, y):
+            assert (m - n).abs().max().item() < 1e-12 * n.abs().max().item()
